@@ -1361,6 +1361,14 @@ AdiArgs make_args(bph_ctx *c, const Schedule &sch, int step0, int nsteps_run, bo
 
 cudaError_t launch_adi(bph_ctx *c, const Schedule &sch, int step0, int nsteps_run, bool cold, double *P,
                        const double *R, int ninst, const int *d_inst_map, double *norms) {
+    if (modal_ready(c, sch) && !norms && step0 == 0 && nsteps_run == sch.nsteps)
+        return launch_modal(c, sch, cold, P ? P : c->d_P, R ? R : c->d_R, c->d_modY, 1, ninst, d_inst_map, nullptr, c->N,
+                            c->stream, c->pdl);
+    return launch_adi_plain(c, sch, step0, nsteps_run, cold, P, R, ninst, d_inst_map, norms);
+}
+
+cudaError_t launch_adi_plain(bph_ctx *c, const Schedule &sch, int step0, int nsteps_run, bool cold, double *P,
+                             const double *R, int ninst, const int *d_inst_map, double *norms) {
     AdiArgs a = make_args(c, sch, step0, nsteps_run, cold);
     if (P) a.P = P;
     if (R) a.R = R;
@@ -1398,7 +1406,10 @@ cudaError_t launch_adi(bph_ctx *c, const Schedule &sch, int step0, int nsteps_ru
 
 cudaError_t launch_adi_slots(bph_ctx *c, const Schedule &sch, bool cold, const int *d_slots, int nslots,
                              cudaStream_t st, bool pdl) {
-    if (!c->adi_seg || nslots < 1) return cudaErrorNotSupported;
+    if (nslots < 1) return cudaErrorNotSupported;
+    if (modal_ready(c, sch))
+        return launch_modal(c, sch, cold, c->d_P, c->d_R, c->d_modY, 1, 1, nullptr, d_slots, nslots, st, pdl);
+    if (!c->adi_seg) return cudaErrorNotSupported;
     if (c->adi_warp)
         return launch_adi_warp(c, sch, 0, sch.nsteps, cold, c->d_P, c->d_R, 1, nullptr, d_slots, nslots, nullptr, st,
                                pdl);

@@ -152,6 +152,7 @@ void free_schedule(bph_ctx *c, Schedule &s) {
     dev_free(s.d_warp_ver);
     dev_free(s.d_warp_rad32);
     dev_free(s.d_warp_ver32);
+    dev_free(s.d_mod_rad);
     free(s.h_dt);
     s = Schedule();
     (void)c;
@@ -201,6 +202,7 @@ int get_schedule(bph_ctx *c, int nsteps, Schedule **out) {
         }
         BPH_CUDA(launch_pack_warp(c, s));
     }
+    BPH_CUDA(modal_pack(c, s));
     BPH_CUDA(cudaStreamSynchronize(c->stream));
     *out = &s;
     return BPH_OK;
@@ -301,9 +303,9 @@ int autotune_setup(bph_ctx *c) {
         if (rc) return rc;
         const int shape = c->adi_warp;
         c->adi_warp = 0;
-        timed([&] { return launch_adi(c, *s, 0, 5, false); }, &c->tuned_adi_us[0]);
+        timed([&] { return launch_adi_plain(c, *s, 0, 5, false); }, &c->tuned_adi_us[0]);
         c->adi_warp = shape;
-        timed([&] { return launch_adi(c, *s, 0, 5, false); }, &c->tuned_adi_us[1]);
+        timed([&] { return launch_adi_plain(c, *s, 0, 5, false); }, &c->tuned_adi_us[1]);
         if (c->tuned_adi_us[0] < c->tuned_adi_us[1]) c->adi_warp = 0;
     }
     if (e0) cudaEventDestroy(e0);
@@ -491,6 +493,7 @@ int setup_impl(bph_ctx *c) {
     if ((rc = adi_configure(c))) return rc;
     if ((rc = warp_configure(c))) return rc;
     if ((rc = direct_configure(c))) return rc;
+    if ((rc = modal_configure(c))) return rc;
     if ((rc = contract_configure(c))) return rc;
     if ((rc = noalloc_setup(c))) return rc;
     {
@@ -557,8 +560,8 @@ int solve_device(bph_ctx *c, const double *d_rho, double *d_pot, const Schedule 
     BPH_CUDA(launch_fft_fwd_rho(c, d_rho));
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (c->green) BPH_CUDA(cudaStreamIsCapturing(c->stream, &cap));
-    if (c->green && cap == cudaStreamCaptureStatusNone && c->overlap && c->adi_seg && c->nfree > 0 &&
-        c->nfree < c->N) {
+    const bool split = c->overlap && (c->adi_seg || modal_ready(c, s)) && c->nfree > 0 && c->nfree < c->N;
+    if (c->green && cap == cudaStreamCaptureStatusNone && split) {
         // contraction on partition 0, free-slot ADI on partition 1, both from the forward FFT
         BPH_CUDA(cudaEventRecord(c->ev_fft, c->stream));
         {
@@ -576,7 +579,7 @@ int solve_device(bph_ctx *c, const double *d_rho, double *d_pot, const Schedule 
         BPH_CUDA(cudaStreamWaitEvent(c->stream, c->ev_free, 0));
         PdlOff off(c);
         BPH_CUDA(launch_fft_inv(c, d_pot, d_phieff, omega));
-    } else if (c->overlap && c->adi_seg && c->nfree > 0 && c->nfree < c->N) {
+    } else if (split) {
         BPH_CUDA(cudaEventRecord(c->ev_fft, c->stream));
         BPH_CUDA(cudaStreamWaitEvent(c->side_stream, c->ev_fft, 0));
         BPH_CUDA(launch_adi_slots(c, s, cold, c->d_slot_map, c->nfree, c->side_stream, false));
@@ -665,7 +668,9 @@ static void ctx_free(bph_ctx *c) {
     dev_free(c->d_kpart);
     dev_free(c->d_kcnt);
     conv_graphs_free(c);
+    modal_free(c);
     dev_free(c->d_work32);
+    dev_free(c->d_modpre);
     dev_free(c->d_warp_coef);
     dev_free(c->d_warp_coef32);
     dev_free(c->d_r32);
@@ -883,8 +888,8 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
     BPH_DEVICE_SCOPE(c);
     Schedule *s;
     if ((rc = get_schedule(c, nsteps, &s))) return rc;
-    if (mixed && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && (rc = ensure_mixed_work(c))) return rc;
-    if (!mixed && !c->d_prev && (rc = dev_alloc(c, &c->d_prev, (size_t)c->N * c->nplane))) return rc;
+    const bool want_modal = modal_converged(c, *s, mixed);
+    if ((!mixed || want_modal) && !c->d_prev && (rc = dev_alloc(c, &c->d_prev, (size_t)c->N * c->nplane))) return rc;
     const size_t bytes = sizeof(double) * (size_t)c->ntot;
     const double *d_rho = rho;
     double *d_pot = pot;
@@ -895,9 +900,15 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
         d_pot = c->d_pot_stage;
     }
     if (cold) BPH_CUDA(cudaMemsetAsync(c->d_P, 0, sizeof(double) * (size_t)c->N * c->nplane, c->stream));
+    if (want_modal && !mixed && !c->d_modpre) (void)dev_alloc(c, &c->d_modpre, modal_size(c));
+    const bool modal = want_modal && (mixed || c->d_modpre);  // no room: the half-step form
+    if (mixed && !modal && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && (rc = ensure_mixed_work(c))) return rc;
     BPH_CUDA(launch_fft_fwd_rho(c, d_rho));
     BPH_CUDA(launch_green_contract(c));  // also writes the Dirichlet slots
-    std::vector<double> h(2 * (size_t)c->N);
+    const int pairs = modal ? c->N * modal_groups(c) : c->N;  // norm pairs of a cycle
+    double *red = modal ? c->d_modnorm : c->d_red;
+    if (modal) BPH_CUDA(launch_modal_begin(c, cold != 0, c->d_P, c->d_R, c->d_modY, c->d_prev, 1, nullptr));
+    std::vector<double> h(2 * (size_t)pairs);
     int cyc = 0;
     double upd = 0.0;
     bool device_loop = c->conv_graph && conv_loop_device(c, *s, mixed, tol, max_cycles) == BPH_OK;
@@ -905,7 +916,9 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
         c->conv_graph = false;  // graphs unavailable: host loop from now on
         double prev_upd = INFINITY;
         for (;;) {
-            if (mixed) {
+            if (modal) {
+                BPH_CUDA(launch_modal_cycle(c, *s, c->d_modY, c->d_prev, mixed ? nullptr : c->d_modpre, 1, red));
+            } else if (mixed) {
                 BPH_CUDA(launch_adi_defect(c, *s));
             } else if (c->adi_seg) {  // update norms from the sweep's write-back
                 BPH_CUDA(launch_adi(c, *s, 0, s->nsteps, false, nullptr, nullptr, 1, nullptr, c->d_red));
@@ -915,15 +928,18 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
                 BPH_CUDA(launch_update_norm(c, c->d_red));
             }
             ++cyc;
-            BPH_CUDA(cudaMemcpyAsync(h.data(), c->d_red, sizeof(double) * h.size(), cudaMemcpyDeviceToHost,
-                                     c->stream));
+            BPH_CUDA(cudaMemcpyAsync(h.data(), red, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
             BPH_CUDA(cudaStreamSynchronize(c->stream));
-            upd = host_ratio(h, c->N);
+            upd = host_ratio(h, pairs);
             bool stop = upd <= tol || cyc >= max_cycles;
             if (mixed) stop = stop || !(upd == upd) || upd > 0.5 * prev_upd;
             if (stop) break;
             prev_upd = upd;
         }
+    }
+    if (modal) {
+        BPH_CUDA(launch_modal_end(c, c->d_P, mixed ? c->d_prev : c->d_modpre, 1, nullptr));
+        if (!mixed) BPH_CUDA(launch_adi_plain(c, *s, s->nsteps - 1, 1, false));
     }
     if (resid_out) BPH_CUDA(launch_residual_norm(c, c->d_red));
     BPH_CUDA(launch_fft_inv(c, d_pot));
@@ -933,7 +949,7 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
     if (device_loop)
         BPH_CUDA(cudaMemcpyAsync(&st, c->d_conv, sizeof(ConvState), cudaMemcpyDeviceToHost, c->stream));
     if (resid_out)
-        BPH_CUDA(cudaMemcpyAsync(h.data(), c->d_red, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
+        BPH_CUDA(cudaMemcpyAsync(h.data(), c->d_red, sizeof(double) * 2 * c->N, cudaMemcpyDeviceToHost, c->stream));
     if ((rc = read_status(c))) return rc;  // synchronises
     if (device_loop) {
         cyc = st.cycles;

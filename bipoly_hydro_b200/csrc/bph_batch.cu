@@ -44,7 +44,13 @@ struct bph_batch {
     int *h_stat = nullptr;     // [cap] pinned host copy
     int stage_cap = 0;         // positions of the host-array staging buffers
     double *d_LW = nullptr, *d_LQ = nullptr;  // grid-wide ADI scratch [cap][N][np] (large slots)
-    double *d_prev = nullptr;         // converged FP64 solves: slot arrays of the previous cycle (on first use)
+    double *d_prev = nullptr;         // converged FP64 solves: slot arrays of the previous cycle (on first use);
+                                      // modal form: the modal potential
+    double *d_mod = nullptr;          // modal form: the modal residual (cap times modal_size)
+    double *d_mody = nullptr;         // modal work array of modal_chunk instances (nullptr: half-step form)
+    double *d_modpre = nullptr;       // the modal potential before a cycle's last step,
+    double *d_mnorm = nullptr;        // and partial norms [cap][N][modal_groups][2], h_mnorm on the host
+    double *h_mnorm = nullptr;
     double *d_work32 = nullptr;       // FP32 work arrays of the mixed converged forms (kind-dependent size)
     size_t work32_doubles = 0;        // its size in doubles
     double *d_cnorm = nullptr;        // converged solves: per (instance, slot) norm pairs [cap][N][2]
@@ -537,6 +543,7 @@ int bph_batch_create(bph_ctx_t *c, int capacity, bph_batch_t **out) {
     int rc = BPH_OK;
     if (!rc) rc = batch_alloc(b, &b->d_P, (size_t)capacity * c->N * c->nplane);
     if (!rc) rc = batch_alloc(b, &b->d_R, (size_t)capacity * c->N * c->np);
+    if (!rc && c->modal) (void)batch_alloc(b, &b->d_mody, (size_t)modal_chunk(c, capacity) * modal_size(c));
     if (!rc) rc = batch_alloc(b, &b->d_mom, (size_t)c->g.mmax * capacity * 2 * c->np);
     if (!rc) rc = batch_alloc(b, &b->d_C, (size_t)c->g.mmax * 2 * capacity * c->nb);
     if (!rc && large) rc = batch_alloc(b, &b->d_LW, (size_t)capacity * c->N * c->np);
@@ -598,7 +605,7 @@ int bph_batch_destroy(bph_batch_t *b) {
     ::bph::DeviceScope scope_(b->c ? b->c->device : 0);
     if (b->c && b->c->stream) cudaStreamSynchronize(b->c->stream);
     double *bufs[] = {b->d_P,     b->d_R,     b->d_mom, b->d_C,    b->d_rho_stage, b->d_pot_stage,
-                      b->d_cpart, b->d_LW,    b->d_LQ,  b->d_prev, b->d_cnorm, b->d_work32};
+                      b->d_cpart, b->d_LW,    b->d_LQ,  b->d_prev, b->d_cnorm, b->d_work32, b->d_mod, b->d_modpre, b->d_mnorm, b->d_mody};
     for (double *p : bufs)
         if (p) cudaFree(p);
     if (b->d_ccnt) cudaFree(b->d_ccnt);
@@ -610,6 +617,7 @@ int bph_batch_destroy(bph_batch_t *b) {
     if (b->d_stat) cudaFree(b->d_stat);
     if (b->h_stat) cudaFreeHost(b->h_stat);
     if (b->h_cnorm) cudaFreeHost(b->h_cnorm);
+    if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
     if (b->c) ctx_release(b->c);
     delete b;
     return BPH_OK;
@@ -815,8 +823,11 @@ int batch_enqueue(bph_batch *b, int n, const double *const *d_in, double *const 
     Schedule *s = &sch;
     int rc = batch_prologue(b, n, d_in, d_map, per_pos);
     if (rc) return rc;
-    if (c->adi_seg)
-        BPH_CUDA(launch_adi(c, *s, 0, s->nsteps, !warm, b->d_P, b->d_R, n, d_map));
+    if (modal_ready(c, *s) && b->d_mody)
+        BPH_CUDA(launch_modal(c, *s, !warm, b->d_P, b->d_R, b->d_mody, modal_chunk(c, b->cap), n, d_map, nullptr, c->N,
+                              c->stream, c->pdl));
+    else if (c->adi_seg)
+        BPH_CUDA(launch_adi_plain(c, *s, 0, s->nsteps, !warm, b->d_P, b->d_R, n, d_map));
     else
         BPH_CUDA(launch_adi_large(c, *s, 0, s->nsteps, !warm, b->d_P, b->d_R, n, d_map, b->d_LW, b->d_LQ));
     BPH_CUDA(launch_fft_inv_batch(c, n, d_out, d_map, b->d_P, (long long)c->N * c->nplane));
@@ -828,6 +839,22 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
     int rc;
     if (!b->d_cnorm && (rc = batch_alloc(b, &b->d_cnorm, 2ull * b->cap * c->N))) return rc;
     if (!b->h_cnorm) BPH_CUDA(cudaMallocHost((void **)&b->h_cnorm, sizeof(double) * 2 * (size_t)b->cap * c->N));
+    // modal form: modal potential, residual and partial norms; without room for them the other
+    // forms run
+    const bool want_modal = c->modal && (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
+    if (want_modal && !b->d_mnorm) {
+        const size_t norms = 2ull * b->cap * c->N * modal_groups(c);
+        if ((b->d_prev || !batch_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)) &&
+            (b->d_mod || !batch_alloc(b, &b->d_mod, (size_t)b->cap * modal_size(c))) &&
+            (b->d_modpre || !batch_alloc(b, &b->d_modpre, (size_t)b->cap * modal_size(c))) &&
+            cudaMallocHost((void **)&b->h_mnorm, sizeof(double) * norms) == cudaSuccess)
+            (void)batch_alloc(b, &b->d_mnorm, norms);
+        if (!b->d_mnorm) {
+            cudaGetLastError();
+            if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
+            b->h_mnorm = nullptr;
+        }
+    }
     // FP64 on the grid-wide kernels: the previous cycle's slot arrays (the segmented kernel
     // forms the update while writing back)
     if (!mixed && !c->adi_seg && !b->d_prev &&
@@ -836,7 +863,7 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
     // FP32 work arrays of the refinement: the grid-wide cycle keeps r, delta and two right-hand
     // sides per position; the warp-cooperative one the rounded residual per position
     size_t need = 0;
-    if (mixed && c->mixed_kind == BPH_MIXED_ADI_GLOBAL) need = 2ull * b->cap * c->N * c->np;
+    if (mixed && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && !(b->d_mnorm && !c->adi_warp)) need = 2ull * b->cap * c->N * c->np;
     if (mixed && c->mixed_kind == BPH_MIXED_ADI_WARP)
         need = ((size_t)b->cap * c->N * c->np + 1) / 2;
     if (need > b->work32_doubles) {
@@ -854,7 +881,7 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
 }
 
 // Sums the per-slot norm pairs of instance i: sqrt(sum |a|^2 / sum |b|^2).
-static double instance_ratio(const double *h, int N, int i) {
+static double instance_ratio(const double *h, int N, int i) {  // N: pairs per instance
     double num = 0.0, den = 0.0;
     for (int sl = 0; sl < N; ++sl) {
         num += h[2 * ((size_t)i * N + sl)];
@@ -885,13 +912,18 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
         for (int i = 0; i < n; ++i)
             BPH_CUDA(cudaMemsetAsync(b->d_P + (size_t)inst[i] * c->N * c->nplane, 0, ibytes, c->stream));
     if ((rc = batch_prologue(b, n, d_in, d_map, per_pos))) return rc;
+    const bool modal = modal_converged(c, *s, cv.mixed) && b->d_mnorm;
+    const int mpairs = modal ? c->N * modal_groups(c) : 0;  // norm pairs per position
+    if (modal) BPH_CUDA(launch_modal_begin(c, cv.cold, b->d_P, b->d_R, b->d_mod, b->d_prev, n, d_map));
     std::vector<double> prev_upd((size_t)n, INFINITY);
     std::vector<char> done((size_t)n, 0);
     const size_t hbytes = sizeof(double) * 2 * (size_t)top * c->N;
     int cyc = 0;
     bool diverged = false;
     for (;;) {
-        if (cv.mixed) {
+        if (modal) {
+            BPH_CUDA(launch_modal_cycle(c, *s, b->d_mod, b->d_prev, cv.mixed ? nullptr : b->d_modpre, n, b->d_mnorm));
+        } else if (cv.mixed) {
             if (c->mixed_kind == BPH_MIXED_ADI_GLOBAL)
                 BPH_CUDA(launch_adi_defect_large_batch(c, *s, b->d_P, b->d_R, n, d_map,
                                                        reinterpret_cast<float *>(b->d_work32), b->d_cnorm));
@@ -918,12 +950,17 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
             BPH_CUDA(launch_norms_batch(c, false, b->d_P, b->d_prev, nullptr, n, d_map, b->d_cnorm));
         }
         ++cyc;
-        BPH_CUDA(cudaMemcpyAsync(b->h_cnorm, b->d_cnorm, hbytes, cudaMemcpyDeviceToHost, c->stream));
+        if (modal)
+            BPH_CUDA(cudaMemcpyAsync(b->h_mnorm, b->d_mnorm, sizeof(double) * 2 * (size_t)n * mpairs,
+                                     cudaMemcpyDeviceToHost, c->stream));
+        else
+            BPH_CUDA(cudaMemcpyAsync(b->h_cnorm, b->d_cnorm, hbytes, cudaMemcpyDeviceToHost, c->stream));
         BPH_CUDA(cudaStreamSynchronize(c->stream));
         bool all = true;
         for (int i = 0; i < n; ++i) {
             if (done[(size_t)i]) continue;  // converged instances keep cycling with the rest (harmless)
-            const double upd = instance_ratio(b->h_cnorm, c->N, inst[i]);
+            const double upd = modal ? instance_ratio(b->h_mnorm, mpairs, i)  // modal norms go by position
+                                     : instance_ratio(b->h_cnorm, c->N, inst[i]);
             // a non-finite update ends the instance (a non-finite density is
             // also flagged per position by the forward transform)
             bool stop = upd <= cv.tol || !(upd == upd);
@@ -936,6 +973,15 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
         if (all || diverged || cyc >= cv.max_cycles) break;
     }
     cv.cycles = cyc;
+    if (modal) {
+        BPH_CUDA(launch_modal_end(c, b->d_P, cv.mixed ? b->d_prev : b->d_modpre, n, d_map));
+        if (cv.mixed)
+            ;  // the modal potential is the result
+        else if (c->adi_seg)
+            BPH_CUDA(launch_adi_plain(c, *s, s->nsteps - 1, 1, false, b->d_P, b->d_R, n, d_map));
+        else
+            BPH_CUDA(launch_adi_large(c, *s, s->nsteps - 1, 1, false, b->d_P, b->d_R, n, d_map, b->d_LW, b->d_LQ));
+    }
     if (cv.want_resid) {
         BPH_CUDA(launch_norms_batch(c, true, b->d_P, nullptr, b->d_R, n, d_map, b->d_cnorm));
         BPH_CUDA(cudaMemcpyAsync(b->h_cnorm, b->d_cnorm, hbytes, cudaMemcpyDeviceToHost, c->stream));

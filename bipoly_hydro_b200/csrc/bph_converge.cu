@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kCheckThreads) k_conv_check(const double *__re
 // arrays and schedule s (the cycle body captured from the launchers).
 static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t *out) {
     *out = nullptr;
+    const bool modal = modal_converged(c, s, mixed) && (mixed || c->d_modpre);
     cudaGraph_t g = nullptr;
     cudaStream_t cs = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -95,7 +96,9 @@ static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t
         c->stream = cs;
         c->pdl = false;  // plain serial edges inside the loop body
         cudaError_t ce = cudaSuccess;
-        if (mixed) {
+        if (modal) {
+            ce = launch_modal_cycle(c, s, c->d_modY, c->d_prev, mixed ? nullptr : c->d_modpre, 1, c->d_modnorm);
+        } else if (mixed) {
             ce = launch_adi_defect(c, s);
         } else if (c->adi_seg) {  // the update norms come from the sweep's write-back
             ce = launch_adi(c, s, 0, s.nsteps, false, nullptr, nullptr, 1, nullptr, c->d_red);
@@ -106,7 +109,8 @@ static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t
             if (ce == cudaSuccess) ce = launch_update_norm(c, c->d_red);
         }
         if (ce == cudaSuccess) {
-            k_conv_check<<<1, kCheckThreads, 0, cs>>>(c->d_red, c->N, c->d_conv, cond);
+            k_conv_check<<<1, kCheckThreads, 0, cs>>>(modal ? c->d_modnorm : c->d_red,
+                                                      modal ? c->N * modal_groups(c) : c->N, c->d_conv, cond);
             ce = cudaGetLastError();
         }
         ++c->launches;
@@ -139,7 +143,8 @@ int conv_loop_device(bph_ctx *c, Schedule &s, bool mixed, double tol, int max_cy
         c->bytes += sizeof(ConvState);
     }
     ConvGraph &cg = c->conv[mixed ? 1 : 0];
-    const int kind = mixed ? (c->mixed_kind * 2 + (c->mixed_pf ? 1 : 0)) : 0;
+    const bool modal = modal_converged(c, s, mixed) && (mixed || c->d_modpre);
+    const int kind = modal ? -2 : mixed ? (c->mixed_kind * 2 + (c->mixed_pf ? 1 : 0)) : 0;
     if (!cg.exec || cg.build_id != s.build_id || cg.kind != kind) {
         if (cg.exec) cudaGraphExecDestroy(cg.exec);
         cg.exec = nullptr;

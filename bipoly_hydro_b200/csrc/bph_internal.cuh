@@ -84,6 +84,10 @@ struct Schedule {
     double *d_warp_ver = nullptr;
     float *d_warp_rad32 = nullptr;  // the same blocks in float (warp-cooperative refinement kernel)
     float *d_warp_ver32 = nullptr;
+    // modal ADI (bph_modal.cu): radial factor blocks [nsteps][N][block] and step
+    // coefficients [nsteps][nz] (nullptr: the schedule runs the half-step form)
+    double *d_mod_rad = nullptr;
+    double2 *d_mod_cs = nullptr;
 };
 
 // Converged-loop state on the device (bph_converge.cu).
@@ -199,6 +203,14 @@ struct bph_ctx {
     int mixed_warp = 0;                // FP32 warp-cooperative refinement kernel available
     float *d_warp_coef32 = nullptr;    // its coefficient blocks
     float *d_r32 = nullptr;            // rounded residual of one solve [N][np] (FP32 warp refinement)
+    // ADI in the vertical eigenbasis (bph_modal.cu)
+    int modal = 0;                     // 1: the FP64 ADI runs there
+    int modal_seg = 0;                 // radii per segment of a radial line
+    double *d_modE = nullptr;          // packed fragments of E, then of E^T (one allocation with the next three)
+    double *d_modlam = nullptr;        // [nz] gamma lambda_q
+    double *d_modY = nullptr;          // [N][nr][nz, even] modal residual / update
+    double *d_modpre = nullptr;        // converged form: potential before a cycle's last step (on first use)
+    double *d_modnorm = nullptr;       // [N][modal_groups][2] partial update norms of a cycle
     double *d_scf = nullptr;           // SCF-step mass partials and scale (bph_scf.cu)
     void *noalloc_scratch = nullptr;   // device address of the allocation-free contraction's scratch array
     long long launches = 0;
@@ -278,6 +290,10 @@ cudaError_t launch_boundary_slots(bph_ctx *c);
 cudaError_t launch_adi(bph_ctx *c, const Schedule &s, int step0, int nsteps_run, bool cold, double *P = nullptr,
                        const double *R = nullptr, int ninst = 1, const int *d_inst_map = nullptr,
                        double *norms = nullptr);
+// The half-step form of launch_adi whatever form the context runs.
+cudaError_t launch_adi_plain(bph_ctx *c, const Schedule &s, int step0, int nsteps_run, bool cold, double *P = nullptr,
+                             const double *R = nullptr, int ninst = 1, const int *d_inst_map = nullptr,
+                             double *norms = nullptr);
 // The slots d_slots[0..nslots) of the context's own arrays, on stream st
 // (pdl: with programmatic dependent launch on that stream).
 cudaError_t launch_adi_slots(bph_ctx *c, const Schedule &s, bool cold, const int *d_slots, int nslots,
@@ -390,6 +406,29 @@ cudaError_t launch_adi_warp(bph_ctx *c, const Schedule &s, int step0, int nsteps
 // array for a context being set up (bph_noalloc.cu).
 int noalloc_setup(bph_ctx *c);
 int fft_configure(bph_ctx *c);
+// ADI in the vertical eigenbasis (bph_modal.cu).  launch_modal: a whole
+// schedule on ninst instances (row r: instance inst_map[r], slots
+// slot_map[0..nslots) of each), chunk instances per pass in Y.  Converged form: begin (modal residual in Y,
+// modal potential in phi, ninst times modal_size each), cycles (partial norms
+// [ninst][N][modal_groups][2]), end (a potential back into P: pre, the
+// caller running that step with launch_adi_plain, or phi).
+int modal_configure(bph_ctx *c);
+void modal_free(bph_ctx *c);
+int modal_groups(const bph_ctx *c);
+size_t modal_size(const bph_ctx *c);  // doubles of one instance's modal array
+int modal_chunk(const bph_ctx *c, int capacity);  // instances per pass of a batch's launch_modal
+cudaError_t modal_pack(bph_ctx *c, Schedule &s);
+bool modal_ready(const bph_ctx *c, const Schedule &s);
+// Whether converged cycles of schedule s run there (mixed: in place of the
+// grid-wide FP32 refinement).
+bool modal_converged(const bph_ctx *c, const Schedule &s, bool mixed);
+cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, const double *R, double *Y, int chunk,
+                         int ninst, const int *inst_map, const int *slot_map, int nslots, cudaStream_t st, bool pdl);
+cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R, double *Y, double *phi, int ninst,
+                               const int *inst_map);
+cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double *phi, double *pre, int ninst,
+                               double *norms);
+cudaError_t launch_modal_end(bph_ctx *c, double *P, double *pre, int ninst, const int *inst_map);
 // Context references (bph_api.cu): a batch takes one at creation and gives
 // it back at its destruction; the last release frees the device state.
 void ctx_retain(bph_ctx *c);

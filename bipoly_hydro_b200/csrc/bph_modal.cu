@@ -1,0 +1,697 @@
+// bph_modal.cu -- the FP64 ADI of every Fourier slot in the vertical
+// eigenbasis.
+//
+// A slot's operator is A = A_r (x) I + I (x) A_z with A_z = gamma T the same
+// for every slot, and T has closed-form eigenvectors (bph_direct.h).  The
+// Peaceman-Rachford half-steps of helmadi.F90:195-355 are rational functions
+// of A_r and A_z, which commute, so on vertical mode q (eigenvalue lambda_q)
+// one whole step of the iteration is
+//   delta = (A_r + dt)^-1 r,
+//   phi  += 2 dt / (dt + lambda_q) delta,
+//   r     = (dt - lambda_q) / (dt + lambda_q) (2 dt delta - r),
+// with r the residual of the current potential (r = R - A phi at the start,
+// Dirichlet terms included): a radial solve whose matrix is the radial
+// half-step's own and the same for every q, and two elementwise updates.
+// The vertical half-steps, the right-hand sides and the exchange of the slot
+// between row and column order after every half-step are gone, and the cost
+// of a step no longer depends on where the slot fits.  A solve is
+//   k_modal_fwd     r = R - A phi in physical space, transformed: Y = E r
+//   k_modal_radial  every step of one line (slot, mode) in registers
+//   k_modal_inv     phi += E^T Y
+// Rounding differs from the half-step form (no 1/(dt + lambda) amplification
+// of the radially stiff components); the iteration is the same one.
+//
+// The transforms are the matrix products of the path (2 nz FMA per zone each)
+// and run on the FP64 tensor cores, mma.sync m16n8k8.f64: 37 TFLOP/s
+// measured for the instruction alone against 33 for FMA.
+#include <cmath>
+#include <cstdlib>
+#include <vector>
+
+#include "bph_internal.cuh"
+
+namespace bph {
+
+static int modal_ldq(const bph_ctx *c);
+
+namespace {
+
+constexpr int kLines = 32;      // radial lines per block: one per lane
+constexpr int kMaxSegs = 16;    // warps of a radial block
+
+struct ModalArgs {
+    const double *E;         // packed A fragments of E (forward) or E^T (inverse)
+    double *P;               // slot arrays [inst][N][nplane]
+    const double *R;         // [inst][N][np]
+    double *Y;               // modal arrays [row][N][nr][ldq], column q = mode
+    double *phi;             // converged form: modal potential, the same layout
+    double *pre;             // converged form: the potential before the cycle's last step
+    const double *brb;       // [N][numr]
+    const double *alphar;    // [numr]
+    const double *betar;     // [numr]
+    const int *inst_map;     // instance of each row (nullptr: inst0 + row)
+    const int *slot_map;     // slot of each block within a row (nullptr: block = slot)
+    const double *rad;       // [nsteps][N][block] radial factors
+    const double2 *cs;       // [nsteps][nz] (2 dt / (dt + lambda), (dt - lambda) / (dt + lambda))
+    const double *dt;        // [nsteps]
+    double *norms;           // converged form: [row][N][groups][2]
+    int inst0, nslots, ntile, groups;
+    int numr, numz, nr, nz, ldq, N, isym, mtiles, ksteps;
+    int nsteps, source, add;
+    double gamma;
+};
+
+// What k_modal_fwd transforms.
+enum { kResidual = 0, kColdResidual = 1, kPotential = 2 };
+
+__device__ __forceinline__ void dmma(double *c, const double2 &a01, const double2 &a23, double b0, double b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a01.x), "d"(a01.y), "d"(a23.x), "d"(a23.y), "d"(b0), "d"(b1));
+}
+
+// Rows of 8 NT columns, padded to 4 modulo the 16 eight-byte banks: the four
+// rows of a B fragment then fall into different banks.
+template <int NT>
+struct TileShape {
+    static constexpr int cols = 8 * NT;
+    static constexpr int ld = cols + 4;
+};
+
+struct TileIndex {
+    int tile, slot, row;
+    long long inst;
+};
+__device__ __forceinline__ TileIndex tile_index(const ModalArgs &a, int per_slot) {
+    TileIndex t;
+    t.tile = blockIdx.x % per_slot;
+    const int b = blockIdx.x / per_slot;
+    const int local = b % a.nslots;
+    t.row = b / a.nslots;
+    t.slot = a.slot_map ? a.slot_map[local] : local;
+    t.inst = a.inst_map ? a.inst_map[t.row] : a.inst0 + t.row;
+    return t;
+}
+
+// acc = A(mt) X for the 16 rows of tile mt and every column of the tile in
+// shared memory.  The A fragments come from L1/L2 (E is shared by every
+// block), one k-step ahead; a 16 x 8 x 8 product holds the tensor pipe for 64
+// cycles, so neither operand's path limits it.
+// B (k, n) sits at sx[k * kstr + n * nstr].
+template <int NT>
+__device__ __forceinline__ void tile_product(const ModalArgs &a, const double *sx, int kstr, int nstr, int mt, int lane,
+                                             double (*acc)[4]) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[n][v] = 0.0;
+    const double2 *ap = reinterpret_cast<const double2 *>(a.E + (long long)mt * a.ksteps * 128) + 2 * lane;
+    double2 a01 = __ldg(ap), a23 = __ldg(ap + 1);
+    const double *bp = sx + t * kstr + g * nstr;
+    for (int ks = 0; ks < a.ksteps; ++ks) {
+        double2 n01 = a01, n23 = a23;
+        if (ks + 1 < a.ksteps) {
+            n01 = __ldg(ap + 64 * (ks + 1));
+            n23 = __ldg(ap + 64 * (ks + 1) + 1);
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) dmma(acc[n], a01, a23, bp[8 * n * nstr], bp[4 * kstr + 8 * n * nstr]);
+        bp += 8 * kstr;
+        a01 = n01;
+        a23 = n23;
+    }
+}
+
+// Block: 8 NT columns of a slot, all rows.  The residual is formed once per
+// column tile, a warp per band of rows with the rows below and at hand kept
+// in registers, and stays in shared memory as the B operand.
+template <int NT>
+__global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
+    extern __shared__ double sx[];
+    constexpr int ld = TileShape<NT>::ld;
+    const TileIndex ti = tile_index(a, a.ntile);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int nr = a.nr, nz = a.nz, numr = a.numr, j0 = ti.tile * TileShape<NT>::cols;
+    const long long np = (long long)nr * nz, nplane = (long long)numr * a.numz;
+    const double *__restrict__ Pg = a.P + (ti.inst * a.N + ti.slot) * nplane;
+    const double *__restrict__ Rs = a.R + (ti.inst * a.N + ti.slot) * np;
+    const bool dirichlet = a.isym == 1;
+    const int per = (nz + nwarps - 1) / nwarps, k0 = warp * per, k1 = min(nz, k0 + per);
+    for (int e = threadIdx.x; e < (8 * a.ksteps - nz) * ld; e += blockDim.x) sx[nz * ld + e] = 0.0;
+    pdl_wait();
+    for (int cc = lane; cc < TileShape<NT>::cols; cc += 32) {
+        const int j = j0 + cc;
+        if (j >= nr) {
+            for (int k = k0; k < k1; ++k) sx[k * ld + cc] = 0.0;
+            continue;
+        }
+        const double al = a.alphar[j + 1], be = a.betar[j + 1], bd = a.brb[(long long)ti.slot * numr + j + 1];
+        const double *p = Pg + (j + 1);
+        if (a.source == kResidual) {
+            double dn = 0.0, cur = 0.0;
+            if (k0 < k1) {
+                dn = (k0 > 0 || dirichlet) ? p[(long long)k0 * numr] : 0.0;
+                cur = p[(long long)(k0 + 1) * numr];
+            }
+#pragma unroll 8
+            for (int k = k0; k < k1; ++k) {
+                const double *pk = p + (long long)(k + 1) * numr;
+                const double up = pk[numr], east = pk[1], west = (j > 0) ? pk[-1] : 0.0;
+                const double diag = (k == 0 && !dirichlet) ? cur : 2.0 * cur;
+                const double ar = bd * cur + al * east + be * west;
+                sx[k * ld + cc] = (Rs[(long long)k * nr + j] - ar) - a.gamma * (diag - up - dn);
+                dn = cur;
+                cur = up;
+            }
+        } else if (a.source == kColdResidual) {
+#pragma unroll 4
+            for (int k = k0; k < k1; ++k) {
+                double v = Rs[(long long)k * nr + j];
+                if (k == nz - 1) v += a.gamma * p[(long long)(nz + 1) * numr];
+                if (k == 0 && dirichlet) v += a.gamma * p[0];
+                if (j == nr - 1) v -= al * p[(long long)(k + 1) * numr + 1];
+                sx[k * ld + cc] = v;
+            }
+        } else {
+#pragma unroll 4
+            for (int k = k0; k < k1; ++k) sx[k * ld + cc] = p[(long long)(k + 1) * numr];
+        }
+    }
+    __syncthreads();
+    double *Yb = a.Y + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
+    const int g = lane >> 2, t = lane & 3;
+    for (int mt = warp; mt < a.mtiles; mt += nwarps) {
+        double acc[NT][4];
+        tile_product<NT>(a, sx, ld, 1, mt, lane, acc);
+        if (mt + nwarps >= a.mtiles) pdl_trigger();
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int j = j0 + 8 * n + 2 * t + (v & 1), q = 16 * mt + g + 8 * (v >> 1);
+                if (q < nz && j < nr) Yb[(long long)j * a.ldq + q] = acc[n][v];
+            }
+    }
+}
+
+// Block: 8 NT columns of a slot: P (+)= E^T Y.  The tile keeps the modal
+// array's order [column][mode] in shared memory (16-byte copies), rows 4
+// modulo 16 words apart.
+__host__ __device__ inline int inv_ld(int ksteps) { return (8 * ksteps + 15) / 16 * 16 + 4; }
+
+template <int NT>
+__global__ void __launch_bounds__(256) k_modal_inv(ModalArgs a) {
+    extern __shared__ __align__(16) double sx[];
+    const int ld = inv_ld(a.ksteps);
+    const TileIndex ti = tile_index(a, a.ntile);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int nr = a.nr, nz = a.nz, numr = a.numr, j0 = ti.tile * TileShape<NT>::cols;
+    const long long nplane = (long long)numr * a.numz;
+    const double *Yb = a.Y + (((long long)ti.row * a.N + ti.slot) * nr + j0) * a.ldq;
+    double *Pg = a.P + (ti.inst * a.N + ti.slot) * nplane;
+    pdl_wait();
+    for (int cc = warp; cc < TileShape<NT>::cols; cc += nwarps) {
+        double *row = sx + cc * ld;
+        if (j0 + cc < nr) {
+            for (int q = 2 * lane; q < a.ldq; q += 64) {
+                const unsigned d = (unsigned)__cvta_generic_to_shared(row + q);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(Yb + (long long)cc * a.ldq + q));
+            }
+        }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int cc = warp; cc < TileShape<NT>::cols; cc += nwarps) {  // modes and columns past the slot
+        const int from = (j0 + cc < nr) ? nz : 0;
+        for (int q = from + lane; q < 8 * a.ksteps; q += 32) sx[cc * ld + q] = 0.0;
+    }
+    __syncthreads();
+    const int g = lane >> 2, t = lane & 3;
+    for (int mt = warp; mt < a.mtiles; mt += nwarps) {
+        double acc[NT][4];
+        tile_product<NT>(a, sx, 1, ld, mt, lane, acc);
+        if (mt + nwarps >= a.mtiles) pdl_trigger();
+        double *p = Pg + (long long)(16 * mt + g + 1) * numr + j0 + 2 * t + 1;
+        const bool k0 = 16 * mt + g < nz, k1 = 16 * mt + g + 8 < nz;
+        if (a.add) {  // every load before the first store: they may not pass it
+            double old[NT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    old[n][v] = ((v < 2 ? k0 : k1) && j0 + 8 * n + 2 * t + (v & 1) < nr)
+                                    ? p[(v >> 1) * 8 * numr + 8 * n + (v & 1)]
+                                    : 0.0;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) acc[n][v] += old[n][v];
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                if ((v < 2 ? k0 : k1) && j0 + 8 * n + 2 * t + (v & 1) < nr)
+                    p[(v >> 1) * 8 * numr + 8 * n + (v & 1)] = acc[n][v];
+    }
+}
+
+// Radial factor block of one (step, slot): per radius the pairs (1/bet,
+// a/bet), then the pairs (G, K) of the forward and backward segment carries,
+// then gam_{j+1}; radii padded to whole segments with zeros.
+__host__ __device__ inline int radial_block(int nseg, int seg) { return 5 * nseg * seg; }
+
+__global__ void k_pack_modal(const double *__restrict__ rad, double *__restrict__ out, int nr, int nseg, int seg) {
+    // one block per (step, slot), one thread per segment
+    const double *src = rad + (long long)blockIdx.x * kAdiFactors * nr;
+    double *dst = out + (long long)blockIdx.x * radial_block(nseg, seg);
+    double *carry = dst + 2 * nseg * seg, *gam = dst + 4 * nseg * seg;
+    const int s = threadIdx.x;
+    double G = 1.0, K = 1.0;
+    for (int e = 0; e < seg; ++e) {
+        const int j = s * seg + e;
+        const bool in = j < nr;
+        const double dd = in ? src[nr + j] : 0.0;
+        G = in ? G * -dd : 0.0;
+        dst[2 * j] = in ? src[j] : 0.0;
+        dst[2 * j + 1] = dd;
+        carry[2 * j] = G;
+        gam[j] = (j + 1 < nr) ? src[2 * nr + j + 1] : 0.0;
+    }
+    for (int e = seg - 1; e >= 0; --e) {
+        const int j = s * seg + e;
+        K = (j + 1 < nr) ? K * -src[2 * nr + j + 1] : 0.0;
+        carry[2 * j + 1] = K;
+    }
+}
+
+__global__ void k_modal_coef(const double *__restrict__ dt, const double *__restrict__ lam, double2 *__restrict__ cs,
+                             int nz) {
+    const double d = dt[blockIdx.x];
+    for (int q = threadIdx.x; q < nz; q += blockDim.x) {
+        const double den = d + lam[q];
+        cs[(long long)blockIdx.x * nz + q] = make_double2(2.0 * d / den, (d - lam[q]) / den);
+    }
+}
+
+// All steps of a group of lines (one slot, 32 modes) in registers: a lane per
+// line, a warp per segment of SEG consecutive radii.  A solve is the Thomas
+// recurrence per segment with zero carry-in, the segment ends exchanged
+// through shared memory, and the carry added on the way back (the
+// partitioned form of tridagr).  With the modes in the lanes, the factors of
+// a radius are one broadcast word for the warp and the modal array is read
+// and written in whole rows; eight lanes per line with shuffle scans instead
+// spent 250 shared-memory cycles per 512 zones and step (66 us for five steps
+// at 130 x 98 x 256).  A step's factors arrive one step ahead by cp.async.
+// kCycle (converged form): Y keeps the residual for the next cycle, the
+// potential's modal coefficients advance in phi, pre takes those before the
+// cycle's last step (the solve ends with that step in half-step form), and the
+// block's partial |update|^2 and |phi|^2 go to norms.
+template <int SEG, bool kCycle>
+__global__ void __launch_bounds__(kLines *kMaxSegs) k_modal_radial(ModalArgs a) {
+    extern __shared__ __align__(16) double sm[];
+    const int nseg = blockDim.x >> 5, rows = nseg * SEG, block = radial_block(nseg, SEG);
+    double *ends = sm + 2 * block;             // [nseg][32] forward ends
+    double *starts = ends + nseg * kLines;     // [nseg][32] backward starts
+    const TileIndex ti = tile_index(a, a.groups);
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int nr = a.nr, nz = a.nz;
+    const double *frad = a.rad + (long long)ti.slot * block;
+    const long long fstep = (long long)a.N * block;
+    auto fetch = [&](int step) {
+        const double *src = frad + step * fstep;
+        double *dst = sm + (step & 1) * block;
+        for (int i = 2 * tid; i < block; i += 2 * blockDim.x) {
+            const unsigned d = (unsigned)__cvta_generic_to_shared(dst + i);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + i));
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+    fetch(0);
+    pdl_wait();
+    const int q = min(ti.tile * kLines + lane, nz - 1);
+    const bool mine = ti.tile * kLines + lane < nz;
+    const long long base = ((long long)ti.row * a.N + ti.slot) * nr * a.ldq + (long long)w * SEG * a.ldq + q;
+    double *Yq = a.Y + base;
+    const int count = min(SEG, nr - w * SEG);  // radii of this segment
+    double r[SEG], x[SEG], acc[SEG];
+#pragma unroll
+    for (int e = 0; e < SEG; ++e) {
+        r[e] = (e < count && mine) ? Yq[(long long)e * a.ldq] : 0.0;
+        acc[e] = 0.0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int step = 0; step < a.nsteps; ++step) {
+        const double *fac = sm + (step & 1) * block;
+        const double2 *pair = reinterpret_cast<const double2 *>(fac) + w * SEG;
+        const double2 *carry = reinterpret_cast<const double2 *>(fac) + rows;
+        const double *gam = fac + 4 * rows + w * SEG;
+        const double2 cs = a.cs[(long long)step * nz + q];
+        const double dt2 = 2.0 * a.dt[step];
+        double y = 0.0;
+#pragma unroll
+        for (int e = 0; e < SEG; ++e) {
+            const double2 f = pair[e];
+            y = fma(-f.y, y, r[e] * f.x);
+            x[e] = y;
+        }
+        ends[w * kLines + lane] = y;
+        __syncthreads();  // every warp is past the previous step: its factor buffer is free
+        if (step + 1 < a.nsteps) fetch(step + 1);
+        double in = 0.0;
+        for (int s = 0; s < w; ++s) in = fma(carry[s * SEG + SEG - 1].x, in, ends[s * kLines + lane]);
+        double m = 0.0;
+#pragma unroll
+        for (int e = SEG - 1; e >= 0; --e) {
+            m = fma(-gam[e], m, fma(carry[w * SEG + e].x, in, x[e]));
+            x[e] = m;
+        }
+        starts[w * kLines + lane] = m;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        in = 0.0;
+        for (int s = nseg - 1; s > w; --s) in = fma(carry[s * SEG].y, in, starts[s * kLines + lane]);
+#pragma unroll
+        for (int e = 0; e < SEG; ++e) {
+            const double v = fma(carry[w * SEG + e].y, in, x[e]);
+            acc[e] = fma(cs.x, v, acc[e]);
+            r[e] = cs.y * fma(dt2, v, -r[e]);
+            x[e] = cs.x * v;
+        }
+    }
+    pdl_trigger();
+    if (!kCycle) {
+#pragma unroll
+        for (int e = 0; e < SEG; ++e)
+            if (e < count && mine) Yq[(long long)e * a.ldq] = acc[e];
+        return;
+    }
+    double *Fq = a.phi + base, *Bq = a.pre ? a.pre + base : nullptr;
+    double num = 0.0, den = 0.0;
+#pragma unroll
+    for (int e = 0; e < SEG; ++e)
+        if (e < count && mine) Yq[(long long)e * a.ldq] = r[e];
+#pragma unroll
+    for (int e = 0; e < SEG; ++e)
+        r[e] = (e < count && mine) ? Fq[(long long)e * a.ldq] : 0.0;
+#pragma unroll
+    for (int e = 0; e < SEG; ++e)
+        if (e < count && mine) {
+            const double v = r[e] + acc[e];
+            Fq[(long long)e * a.ldq] = v;
+            if (Bq) Bq[(long long)e * a.ldq] = v - x[e];
+            num = fma(acc[e], acc[e], num);
+            den = fma(v, v, den);
+        }
+    // the block's sums in a fixed order, with the slot's Parseval weight
+    for (int d = 16; d > 0; d >>= 1) {
+        num += __shfl_down_sync(0xffffffffu, num, d);
+        den += __shfl_down_sync(0xffffffffu, den, d);
+    }
+    __syncthreads();
+    if (lane == 0) {
+        sm[2 * w] = num;
+        sm[2 * w + 1] = den;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        num = den = 0.0;
+        for (int s = 0; s < nseg; ++s) {
+            num += sm[2 * s];
+            den += sm[2 * s + 1];
+        }
+        const double wt = (ti.slot == 0 || ti.slot == a.N / 2) ? 1.0 : 2.0;
+        double *out = a.norms + 2 * (((long long)ti.row * a.N + ti.slot) * a.groups + ti.tile);
+        out[0] = wt * num;
+        out[1] = wt * den;
+    }
+}
+
+// Radii per segment: 16 hold a line's residual, solution and update in 96
+// registers; up to 64 radii take 8, which halves the serial chains (the
+// smallest grids do not fill the chip).
+int radial_seg(int nr) { return nr <= 64 ? 8 : 16; }
+int radial_nseg(const bph_ctx *c) { return (c->nr + c->modal_seg - 1) / c->modal_seg; }
+
+template <bool kCycle>
+const void *radial_kernel(const bph_ctx *c) {
+    return c->modal_seg == 8 ? (const void *)k_modal_radial<8, kCycle> : (const void *)k_modal_radial<16, kCycle>;
+}
+
+size_t radial_smem(const bph_ctx *c) {
+    const int n = radial_nseg(c);
+    return sizeof(double) * (2 * (size_t)radial_block(n, c->modal_seg) + 2 * (size_t)n * kLines);
+}
+constexpr int kNT = 4;  // 32 columns per transform tile (64: 161 against 129 us per solve at 130 x 98 x 256)
+size_t fwd_smem(const bph_ctx *c) { return sizeof(double) * (size_t)((c->nz + 7) / 8 * 8) * TileShape<kNT>::ld; }
+size_t inv_smem(const bph_ctx *c) { return sizeof(double) * (size_t)TileShape<kNT>::cols * inv_ld((c->nz + 7) / 8); }
+int tile_threads(const bph_ctx *c) {
+    const int mt = (c->nz + 15) / 16;
+    const int rounds = (mt + 7) / 8;
+    const int w = (mt + rounds - 1) / rounds;
+    return 32 * (w < 4 ? 4 : w);
+}
+
+ModalArgs base_args(const bph_ctx *c) {
+    ModalArgs a = {};
+    a.brb = c->d_brb;
+    a.alphar = c->d_alphar;
+    a.betar = c->d_betar;
+    a.nslots = c->N;
+    a.ntile = (c->nr + 8 * kNT - 1) / (8 * kNT);
+    a.groups = modal_groups(c);
+    a.numr = c->g.numr;
+    a.numz = c->g.numz;
+    a.nr = c->nr;
+    a.nz = c->nz;
+    a.ldq = modal_ldq(c);
+    a.N = c->N;
+    a.isym = c->g.isym;
+    a.mtiles = (c->nz + 15) / 16;
+    a.ksteps = (c->nz + 7) / 8;
+    a.gamma = c->gamma;
+    return a;
+}
+
+cudaError_t launch(bph_ctx *c, const void *fn, long long blocks, int threads, size_t smem, ModalArgs &a,
+                   cudaStream_t st, bool pdl) {
+    ++c->launches;
+    void *args[] = {&a};
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = launch_config(c, dim3((unsigned)blocks), dim3(threads), smem, attr);
+    cfg.stream = st;
+    if (!pdl) cfg.numAttrs = 0;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+}  // namespace
+
+int modal_groups(const bph_ctx *c) { return (c->nz + kLines - 1) / kLines; }
+static int modal_ldq(const bph_ctx *c) { return (c->nz + 1) / 2 * 2; }  // 16-byte rows
+size_t modal_size(const bph_ctx *c) { return (size_t)c->N * c->nr * modal_ldq(c); }
+
+// A batch works through its instances in passes whose modal array stays well
+// inside the 126 MB L2 (the three kernels hand it to each other).
+int modal_chunk(const bph_ctx *c, int capacity) {
+    const size_t fit = (48ull << 20) / (sizeof(double) * modal_size(c));
+    const int most = fit < 1 ? 1 : fit > 64 ? 64 : (int)fit;
+    return capacity < most ? capacity : most;
+}
+
+// Decides whether the grid runs the modal form and prepares it.  Lines of up
+// to 256 radii fit a block; the transforms cost 4 nz FMA per zone and solve,
+// and their column tile has to fit in shared memory (nz <= 640), where five
+// half-step pairs cost a fixed ~70.  BPH_ADI_WARP in the environment asks for
+// a half-step kernel by name, BPH_ADI_MODAL=0 for the half-step form.
+int modal_configure(bph_ctx *c) {
+    c->modal = 0;
+    const char *want = std::getenv("BPH_ADI_MODAL");
+    if ((want && want[0] == '0') || std::getenv("BPH_ADI_WARP")) return BPH_OK;
+    if (c->nr > 16 * kMaxSegs || c->nz > 640) return BPH_OK;
+    c->modal_seg = radial_seg(c->nr);
+    const int nz = c->nz, ks = (nz + 7) / 8, mt = (nz + 15) / 16;
+    // E[q][k] from a table of one period: its argument is (2k+1)(2q+1) pi / (2 (2 nz + 1))
+    // (reflecting bottom) or (k+1)(q+1) pi / (nz + 1) (Dirichlet)
+    const bool dirichlet = c->g.isym == 1;
+    const long long period = dirichlet ? 2LL * (nz + 1) : 4LL * (2 * nz + 1);
+    std::vector<double> wave((size_t)period), lam((size_t)nz);
+    const long double pi = std::acos(-1.0L);
+    const long double scale = dirichlet ? std::sqrt(2.0L / (nz + 1.0L)) : 2.0L / std::sqrt(2.0L * nz + 1.0L);
+    for (long long i = 0; i < period; ++i) {
+        const long double x = 2.0L * pi * (long double)i / (long double)period;
+        wave[(size_t)i] = (double)(scale * (dirichlet ? std::sin(x) : std::cos(x)));
+    }
+    for (int q = 0; q < nz; ++q) {
+        const long double half =
+            dirichlet ? 0.5L * (q + 1.0L) * pi / (nz + 1.0L) : 0.5L * (q + 0.5L) * pi / (nz + 0.5L);
+        const long double sn = std::sin(half);
+        lam[(size_t)q] = (double)((long double)c->gamma * 4.0L * sn * sn);
+    }
+    auto entry = [&](int q, int k) -> double {
+        if (q >= nz || k >= nz) return 0.0;
+        const long long i = dirichlet ? (long long)(q + 1) * (k + 1) : (2LL * q + 1) * (2LL * k + 1);
+        return wave[(size_t)(i % period)];
+    };
+    const size_t frag = (size_t)mt * ks * 128;
+    std::vector<double> pack(2 * frag);
+    for (int m = 0; m < mt; ++m)
+        for (int k = 0; k < ks; ++k)
+            for (int l = 0; l < 32; ++l) {
+                const int g = l / 4, t = l % 4;
+                for (int v = 0; v < 4; ++v) {
+                    const int row = 16 * m + g + 8 * (v & 1), col = 8 * k + t + 4 * (v >> 1);
+                    const size_t at = ((size_t)m * ks + k) * 128 + 4 * l + v;
+                    pack[at] = entry(row, col);         // E: row = mode
+                    pack[frag + at] = entry(col, row);  // E^T: row = height
+                }
+            }
+    // one allocation: both fragment arrays, the eigenvalues, the norm partials, one instance's modal array
+    const size_t norms = 2 * (size_t)c->N * modal_groups(c), lams = ((size_t)nz + 1) / 2 * 2;
+    const size_t all = pack.size() + lams + norms + modal_size(c);
+    if (cudaMalloc((void **)&c->d_modE, sizeof(double) * all) != cudaSuccess) {
+        cudaGetLastError();  // no room: the half-step kernels need none of it
+        c->d_modE = nullptr;
+        return BPH_OK;
+    }
+    c->d_modlam = c->d_modE + pack.size();
+    c->d_modnorm = c->d_modlam + lams;
+    c->d_modY = c->d_modnorm + norms;
+    c->bytes += sizeof(double) * all;
+    pack.insert(pack.end(), lam.begin(), lam.end());
+    BPH_CUDA(cudaMemcpyAsync(c->d_modE, pack.data(), sizeof(double) * pack.size(), cudaMemcpyHostToDevice, c->stream));
+    BPH_CUDA(cudaStreamSynchronize(c->stream));  // pack is this call's own
+    BPH_CUDA(raise_smem_limit((const void *)k_modal_fwd<kNT>, (int)fwd_smem(c)));
+    BPH_CUDA(raise_smem_limit((const void *)k_modal_inv<kNT>, (int)inv_smem(c)));
+    BPH_CUDA(raise_smem_limit(radial_kernel<false>(c), (int)radial_smem(c)));
+    BPH_CUDA(raise_smem_limit(radial_kernel<true>(c), (int)radial_smem(c)));
+    c->modal = 1;
+    return BPH_OK;
+}
+
+void modal_free(bph_ctx *c) {
+    if (c->d_modE) cudaFree(c->d_modE);
+    c->d_modE = c->d_modlam = c->d_modnorm = c->d_modY = nullptr;
+    c->modal = 0;
+}
+
+// A schedule's radial blocks and step coefficients (after launch_adi_factors);
+// without room for them the schedule runs the half-step form.
+cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
+    if (!c->modal) return cudaSuccess;
+    const size_t rad = (size_t)s.nsteps * c->N * radial_block(radial_nseg(c), c->modal_seg);
+    const size_t cs = (size_t)s.nsteps * c->nz;
+    if (cudaMalloc((void **)&s.d_mod_rad, sizeof(double) * rad + sizeof(double2) * cs) != cudaSuccess) {
+        cudaGetLastError();
+        s.d_mod_rad = nullptr;
+        return cudaSuccess;
+    }
+    s.d_mod_cs = reinterpret_cast<double2 *>(s.d_mod_rad + rad);  // rad is even
+    c->bytes += sizeof(double) * rad + sizeof(double2) * cs;
+    c->launches += 2;
+    const int nseg = radial_nseg(c);
+    k_pack_modal<<<(unsigned)(s.nsteps * c->N), nseg, 0, c->stream>>>(s.d_rad, s.d_mod_rad, c->nr, nseg, c->modal_seg);
+    k_modal_coef<<<(unsigned)s.nsteps, 128, 0, c->stream>>>(s.d_dt, c->d_modlam, s.d_mod_cs, c->nz);
+    return cudaGetLastError();
+}
+
+// A schedule's form.  The transforms cost a fixed ~60 us and a modal step ~5
+// at 130 x 98 x 256; the warp-cooperative half-step kernel spends 15 per step
+// (66 x 66 x 64: 14 + 0.8 against 4 + 2.3), so where it applies it keeps the
+// schedules of up to seven steps.  Every other half-step kernel is slower than
+// the modal form from five steps on (101 x 75 x 128: 50 against 101 us,
+// 258 x 194 x 256: 551 against 1034; shorter schedules are not a solver's).
+bool modal_ready(const bph_ctx *c, const Schedule &s) {
+    return c->modal && s.d_mod_rad && !(c->adi_warp && s.nsteps <= 7);
+}
+
+// The grid-wide FP32 refinement cycle costs more than a modal cycle in FP64
+// (258 x 194 x 512, ten steps: 2500 against 880 us), so the mixed form runs
+// the latter where that refinement would be its choice.
+bool modal_converged(const bph_ctx *c, const Schedule &s, bool mixed) {
+    return modal_ready(c, s) && (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
+}
+
+cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, const double *R, double *Y, int chunk,
+                         int ninst, const int *inst_map, const int *slot_map, int nslots, cudaStream_t st, bool pdl) {
+    ModalArgs a = base_args(c);
+    a.P = P;
+    a.R = R;
+    a.Y = Y;
+    a.slot_map = slot_map;
+    a.nslots = nslots;
+    a.rad = s.d_mod_rad;
+    a.cs = s.d_mod_cs;
+    a.dt = s.d_dt;
+    a.nsteps = s.nsteps;
+    const int threads = tile_threads(c);
+    for (int r0 = 0; r0 < ninst; r0 += chunk) {
+        const int rows = ninst - r0 < chunk ? ninst - r0 : chunk;
+        const long long blocks = (long long)rows * nslots;
+        a.inst_map = inst_map ? inst_map + r0 : nullptr;
+        a.inst0 = r0;
+        a.E = c->d_modE;
+        a.source = cold ? kColdResidual : kResidual;
+        cudaError_t e = launch(c, (const void *)k_modal_fwd<kNT>, blocks * a.ntile, threads, fwd_smem(c), a, st, pdl);
+        if (e == cudaSuccess)
+            e = launch(c, radial_kernel<false>(c), blocks * a.groups, kLines * radial_nseg(c), radial_smem(c), a, st, pdl);
+        a.E = c->d_modE + (size_t)a.mtiles * a.ksteps * 128;
+        a.add = cold ? 0 : 1;
+        if (e == cudaSuccess) 
+            e = launch(c, (const void *)k_modal_inv<kNT>, blocks * a.ntile, threads, inv_smem(c), a, st, pdl);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// Converged form: the modal residual (and, warm, the modal potential) of
+// ninst instances; cycles on them; a potential back in P.  The FP64 form takes
+// the one before the last step and runs that step in half-step form: the
+// residual it reports is the half-step iteration's, whose rounding floor its
+// last vertical half-step sets.  The mixed form takes the last one.
+cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R, double *Y, double *phi, int ninst,
+                               const int *inst_map) {
+    ModalArgs a = base_args(c);
+    a.P = P;
+    a.R = R;
+    a.Y = Y;
+    a.inst_map = inst_map;
+    a.E = c->d_modE;
+    a.source = cold ? kColdResidual : kResidual;
+    const long long blocks = (long long)ninst * c->N * a.ntile;
+    cudaError_t e = launch(c, (const void *)k_modal_fwd<kNT>, blocks, tile_threads(c), fwd_smem(c), a, c->stream, c->pdl);
+    if (e != cudaSuccess) return e;
+    if (cold) return cudaMemsetAsync(phi, 0, sizeof(double) * (size_t)ninst * modal_size(c), c->stream);
+    a.Y = phi;
+    a.source = kPotential;
+    return launch(c, (const void *)k_modal_fwd<kNT>, blocks, tile_threads(c), fwd_smem(c), a, c->stream, c->pdl);
+}
+
+cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double *phi, double *pre, int ninst,
+                               double *norms) {
+    ModalArgs a = base_args(c);
+    a.Y = Y;
+    a.phi = phi;
+    a.pre = pre;
+    a.rad = s.d_mod_rad;
+    a.cs = s.d_mod_cs;
+    a.dt = s.d_dt;
+    a.nsteps = s.nsteps;
+    a.norms = norms;
+    return launch(c, radial_kernel<true>(c), (long long)ninst * c->N * a.groups, kLines * radial_nseg(c), radial_smem(c), a,
+                  c->stream, c->pdl);
+}
+
+cudaError_t launch_modal_end(bph_ctx *c, double *P, double *pre, int ninst, const int *inst_map) {
+    ModalArgs a = base_args(c);
+    a.P = P;
+    a.Y = pre;
+    a.inst_map = inst_map;
+    a.E = c->d_modE + (size_t)a.mtiles * a.ksteps * 128;
+    return launch(c, (const void *)k_modal_inv<kNT>, (long long)ninst * c->N * a.ntile, tile_threads(c), inv_smem(c), a,
+                  c->stream, c->pdl);
+}
+
+}  // namespace bph
