@@ -230,60 +230,55 @@ __global__ void __launch_bounds__(256) k_modal_inv(ModalArgs a) {
     __syncthreads();
     const int g = lane >> 2, t = lane & 3;
     for (int mt = warp; mt < a.mtiles; mt += nwarps) {
-        double acc[NT][4];
-        tile_product<NT>(a, sx, 1, ld, mt, lane, acc);
-        if (mt + nwarps >= a.mtiles) pdl_trigger();
         double *p = Pg + (long long)(16 * mt + g + 1) * numr + j0 + 2 * t + 1;
         const bool k0 = 16 * mt + g < nz, k1 = 16 * mt + g + 8 < nz;
-        if (a.add) {  // every load before the first store: they may not pass it
-            double old[NT][4];
+        double old[NT][4], acc[NT][4];  // the old potential arrives under the products
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    old[n][v] = ((v < 2 ? k0 : k1) && j0 + 8 * n + 2 * t + (v & 1) < nr)
-                                    ? p[(v >> 1) * 8 * numr + 8 * n + (v & 1)]
-                                    : 0.0;
-#pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) acc[n][v] += old[n][v];
-        }
+            for (int v = 0; v < 4; ++v)
+                old[n][v] = (a.add && (v < 2 ? k0 : k1) && j0 + 8 * n + 2 * t + (v & 1) < nr)
+                                ? p[(v >> 1) * 8 * numr + 8 * n + (v & 1)]
+                                : 0.0;
+        tile_product<NT>(a, sx, 1, ld, mt, lane, acc);
+        if (mt + nwarps >= a.mtiles) pdl_trigger();
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int v = 0; v < 4; ++v)
                 if ((v < 2 ? k0 : k1) && j0 + 8 * n + 2 * t + (v & 1) < nr)
-                    p[(v >> 1) * 8 * numr + 8 * n + (v & 1)] = acc[n][v];
+                    p[(v >> 1) * 8 * numr + 8 * n + (v & 1)] = old[n][v] + acc[n][v];
     }
 }
 
 // Radial factor block of one (step, slot): per radius the pairs (1/bet,
-// a/bet), then the pairs (G, K) of the forward and backward segment carries,
-// then gam_{j+1}; radii padded to whole segments with zeros.
-__host__ __device__ inline int radial_block(int nseg, int seg) { return 5 * nseg * seg; }
+// -a/bet) of the way down, the pairs (-gam_{j+1}, G) of the way up with the
+// forward segment carry, then the backward carries K; padded to `rows` radii
+// with zeros.
+__host__ __device__ constexpr int radial_block(int rows) { return 5 * rows; }
 
 __global__ void k_pack_modal(const double *__restrict__ rad, double *__restrict__ out, int nr, int nseg, int seg) {
     // one block per (step, slot), one thread per segment
+    const int rows = nseg * seg;
     const double *src = rad + (long long)blockIdx.x * kAdiFactors * nr;
-    double *dst = out + (long long)blockIdx.x * radial_block(nseg, seg);
-    double *carry = dst + 2 * nseg * seg, *gam = dst + 4 * nseg * seg;
+    double *dst = out + (long long)blockIdx.x * radial_block(rows);
+    double *back = dst + 2 * rows, *kk = dst + 4 * rows;
     const int s = threadIdx.x;
     double G = 1.0, K = 1.0;
     for (int e = 0; e < seg; ++e) {
         const int j = s * seg + e;
         const bool in = j < nr;
-        const double dd = in ? src[nr + j] : 0.0;
-        G = in ? G * -dd : 0.0;
+        const double dd = in ? -src[nr + j] : 0.0;
+        G = in ? G * dd : 0.0;
         dst[2 * j] = in ? src[j] : 0.0;
         dst[2 * j + 1] = dd;
-        carry[2 * j] = G;
-        gam[j] = (j + 1 < nr) ? src[2 * nr + j + 1] : 0.0;
+        back[2 * j] = (j + 1 < nr) ? -src[2 * nr + j + 1] : 0.0;
+        back[2 * j + 1] = G;
     }
     for (int e = seg - 1; e >= 0; --e) {
         const int j = s * seg + e;
         K = (j + 1 < nr) ? K * -src[2 * nr + j + 1] : 0.0;
-        carry[2 * j + 1] = K;
+        kk[j] = K;
     }
 }
 
@@ -309,12 +304,16 @@ __global__ void k_modal_coef(const double *__restrict__ dt, const double *__rest
 // potential's modal coefficients advance in phi, pre takes those before the
 // cycle's last step (the solve ends with that step in half-step form), and the
 // block's partial |update|^2 and |phi|^2 go to norms.
-template <int SEG, bool kCycle>
-__global__ void __launch_bounds__(kLines *kMaxSegs) k_modal_radial(ModalArgs a) {
+// ROWS, the line length the factor blocks are padded to, is a compile-time
+// constant so that every shared-memory operand is one base register and an
+// offset.
+template <int SEG, int ROWS, bool kCycle>
+__global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_modal_radial(ModalArgs a) {
     extern __shared__ __align__(16) double sm[];
-    const int nseg = blockDim.x >> 5, rows = nseg * SEG, block = radial_block(nseg, SEG);
-    double *ends = sm + 2 * block;             // [nseg][32] forward ends
-    double *starts = ends + nseg * kLines;     // [nseg][32] backward starts
+    constexpr int NSEG = ROWS / SEG, block = radial_block(ROWS);
+    const int nseg = blockDim.x >> 5;
+    double *ends = sm + 2 * block;             // [NSEG][32] forward ends
+    double *starts = ends + NSEG * kLines;     // [NSEG][32] backward starts
     const TileIndex ti = tile_index(a, a.groups);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int nr = a.nr, nz = a.nz;
@@ -347,39 +346,55 @@ __global__ void __launch_bounds__(kLines *kMaxSegs) k_modal_radial(ModalArgs a) 
     for (int step = 0; step < a.nsteps; ++step) {
         const double *fac = sm + (step & 1) * block;
         const double2 *pair = reinterpret_cast<const double2 *>(fac) + w * SEG;
-        const double2 *carry = reinterpret_cast<const double2 *>(fac) + rows;
-        const double *gam = fac + 4 * rows + w * SEG;
+        const double2 *back = pair + ROWS;
+        const double *kk = fac + 4 * ROWS + w * SEG;
         const double2 cs = a.cs[(long long)step * nz + q];
         const double dt2 = 2.0 * a.dt[step];
         double y = 0.0;
 #pragma unroll
         for (int e = 0; e < SEG; ++e) {
             const double2 f = pair[e];
-            y = fma(-f.y, y, r[e] * f.x);
+            y = fma(f.y, y, r[e] * f.x);
             x[e] = y;
         }
         ends[w * kLines + lane] = y;
         __syncthreads();  // every warp is past the previous step: its factor buffer is free
         if (step + 1 < a.nsteps) fetch(step + 1);
         double in = 0.0;
-        for (int s = 0; s < w; ++s) in = fma(carry[s * SEG + SEG - 1].x, in, ends[s * kLines + lane]);
+        {
+            const double2 *g = reinterpret_cast<const double2 *>(fac) + ROWS + SEG - 1;
+            const double *en = ends + lane;
+#pragma unroll 4
+            for (int s = 0; s < w; ++s) in = fma(g[s * SEG].y, in, en[s * kLines]);
+        }
         double m = 0.0;
 #pragma unroll
         for (int e = SEG - 1; e >= 0; --e) {
-            m = fma(-gam[e], m, fma(carry[w * SEG + e].x, in, x[e]));
+            const double2 f = back[e];
+            m = fma(f.x, m, fma(f.y, in, x[e]));
             x[e] = m;
         }
         starts[w * kLines + lane] = m;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         in = 0.0;
-        for (int s = nseg - 1; s > w; --s) in = fma(carry[s * SEG].y, in, starts[s * kLines + lane]);
+        {
+            const double *k = fac + 4 * ROWS, *st = starts + lane;
+#pragma unroll 4
+            for (int s = nseg - 1; s > w; --s) in = fma(k[s * SEG], in, st[s * kLines]);
+        }
 #pragma unroll
-        for (int e = 0; e < SEG; ++e) {
-            const double v = fma(carry[w * SEG + e].y, in, x[e]);
-            acc[e] = fma(cs.x, v, acc[e]);
-            r[e] = cs.y * fma(dt2, v, -r[e]);
-            x[e] = cs.x * v;
+        for (int e = 0; e < SEG; e += 2) {
+            const double2 k2 = *reinterpret_cast<const double2 *>(kk + e);
+            const double v0 = fma(k2.x, in, x[e]), v1 = fma(k2.y, in, x[e + 1]);
+            acc[e] = fma(cs.x, v0, acc[e]);
+            acc[e + 1] = fma(cs.x, v1, acc[e + 1]);
+            r[e] = cs.y * fma(dt2, v0, -r[e]);
+            r[e + 1] = cs.y * fma(dt2, v1, -r[e + 1]);
+            if (kCycle) {
+                x[e] = cs.x * v0;
+                x[e + 1] = cs.x * v1;
+            }
         }
     }
     pdl_trigger();
@@ -435,15 +450,20 @@ __global__ void __launch_bounds__(kLines *kMaxSegs) k_modal_radial(ModalArgs a) 
 // smallest grids do not fill the chip).
 int radial_seg(int nr) { return nr <= 64 ? 8 : 16; }
 int radial_nseg(const bph_ctx *c) { return (c->nr + c->modal_seg - 1) / c->modal_seg; }
+int radial_rows(const bph_ctx *c) { return c->nr <= 64 ? 64 : c->nr <= 128 ? 128 : 256; }
 
 template <bool kCycle>
 const void *radial_kernel(const bph_ctx *c) {
-    return c->modal_seg == 8 ? (const void *)k_modal_radial<8, kCycle> : (const void *)k_modal_radial<16, kCycle>;
+    switch (radial_rows(c)) {
+        case 64: return (const void *)k_modal_radial<8, 64, kCycle>;
+        case 128: return (const void *)k_modal_radial<16, 128, kCycle>;
+        default: return (const void *)k_modal_radial<16, 256, kCycle>;
+    }
 }
 
 size_t radial_smem(const bph_ctx *c) {
-    const int n = radial_nseg(c);
-    return sizeof(double) * (2 * (size_t)radial_block(n, c->modal_seg) + 2 * (size_t)n * kLines);
+    const size_t rows = radial_rows(c);
+    return sizeof(double) * (2 * (size_t)radial_block((int)rows) + 2 * rows / c->modal_seg * kLines);
 }
 constexpr int kNT = 4;  // 32 columns per transform tile (64: 161 against 129 us per solve at 130 x 98 x 256)
 size_t fwd_smem(const bph_ctx *c) { return sizeof(double) * (size_t)((c->nz + 7) / 8 * 8) * TileShape<kNT>::ld; }
@@ -503,8 +523,7 @@ int modal_chunk(const bph_ctx *c, int capacity) {
 
 // Decides whether the grid runs the modal form and prepares it.  Lines of up
 // to 256 radii fit a block; the transforms cost 4 nz FMA per zone and solve,
-// and their column tile has to fit in shared memory (nz <= 640), where five
-// half-step pairs cost a fixed ~70.  BPH_ADI_WARP in the environment asks for
+// and their column tile has to fit in shared memory (nz <= 640).  BPH_ADI_WARP in the environment asks for
 // a half-step kernel by name, BPH_ADI_MODAL=0 for the half-step form.
 int modal_configure(bph_ctx *c) {
     c->modal = 0;
@@ -581,7 +600,7 @@ void modal_free(bph_ctx *c) {
 // without room for them the schedule runs the half-step form.
 cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
     if (!c->modal) return cudaSuccess;
-    const size_t rad = (size_t)s.nsteps * c->N * radial_block(radial_nseg(c), c->modal_seg);
+    const size_t rad = (size_t)s.nsteps * c->N * radial_block(radial_rows(c));
     const size_t cs = (size_t)s.nsteps * c->nz;
     if (cudaMalloc((void **)&s.d_mod_rad, sizeof(double) * rad + sizeof(double2) * cs) != cudaSuccess) {
         cudaGetLastError();
@@ -591,7 +610,7 @@ cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
     s.d_mod_cs = reinterpret_cast<double2 *>(s.d_mod_rad + rad);  // rad is even
     c->bytes += sizeof(double) * rad + sizeof(double2) * cs;
     c->launches += 2;
-    const int nseg = radial_nseg(c);
+    const int nseg = radial_rows(c) / c->modal_seg;
     k_pack_modal<<<(unsigned)(s.nsteps * c->N), nseg, 0, c->stream>>>(s.d_rad, s.d_mod_rad, c->nr, nseg, c->modal_seg);
     k_modal_coef<<<(unsigned)s.nsteps, 128, 0, c->stream>>>(s.d_dt, c->d_modlam, s.d_mod_cs, c->nz);
     return cudaGetLastError();
@@ -639,8 +658,7 @@ cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, co
             e = launch(c, radial_kernel<false>(c), blocks * a.groups, kLines * radial_nseg(c), radial_smem(c), a, st, pdl);
         a.E = c->d_modE + (size_t)a.mtiles * a.ksteps * 128;
         a.add = cold ? 0 : 1;
-        if (e == cudaSuccess) 
-            e = launch(c, (const void *)k_modal_inv<kNT>, blocks * a.ntile, threads, inv_smem(c), a, st, pdl);
+        if (e == cudaSuccess) e = launch(c, (const void *)k_modal_inv<kNT>, blocks * a.ntile, threads, inv_smem(c), a, st, pdl);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
