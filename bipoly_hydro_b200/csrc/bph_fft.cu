@@ -1,14 +1,19 @@
 // bph_fft.cu -- azimuthal real FFTs (realft.F90 + the slot reorder of
 // helmadi.F90:132-183 and its inverse :357-411).
 //
-// A CTA takes a tile of 16 consecutive (J,K) columns and all numphi samples
-// of each: every row of the tile is a 128-byte coalesced segment of the
-// Fortran array (J fastest).  The N real samples of a column are packed as
-// M = N/2 complex values in shared memory, transformed by in-place Stockham
-// radix-4 (and one radix-2) passes -- each pass loads its butterfly inputs
-// to registers, synchronises, and stores -- and post-processed into the
-// real spectrum.  Results are written slot-major, which is the layout the
-// ADI kernel reads: the reference's swap_phi_r / swap_r_phi transposes are
+// A block takes a tile of 16 consecutive (J,K) columns and all numphi samples
+// of each: every row of the tile is a 128-byte segment of the Fortran array
+// (J fastest).  The N real samples of a column are M = N/2 complex values,
+// transformed in two steps, M = R1 T: T threads per column hold R1 values
+// each and transform them in registers, exchange them once through shared
+// memory, and do the T-point transforms of the other digit.  The threads'
+// second digits are dealt so that k and M - k, which the real spectrum needs
+// together, meet in one thread (R1 = 2T) or in two lanes of a warp (R1 = T),
+// so the split into the real spectrum and the store to the slots need no
+// further exchange.  (An in-place Stockham pass per radix-4 step wrote and
+// read the tile ten times with a barrier each; it spent 18.8 + 15.9 us at
+// 130 x 98 x 256.)  Results are written slot-major, which is the layout the
+// ADI kernels read: the reference's swap_phi_r / swap_r_phi transposes are
 // this store / load layout.
 //
 // Forward convention (realft isign=+1): F_k = sum_l f_l exp(+2 pi i k l / N).
@@ -20,13 +25,16 @@
 namespace bph {
 namespace {
 
-// Columns per CTA: 8 (64-byte rows) for the 64- and 128-point transforms, so
-// that a grid is several short waves instead of one long one with a tail;
-// 16 (128-byte rows) otherwise.
+constexpr int kTile = 16;  // columns per block
+
+// M = R1 T, both powers of two, R1 = T or 2T.
 template <int M>
-constexpr int tile_cols() {
-    return (M >= 64 && M <= 128) ? 8 : 16;
-}
+struct Split {
+    static constexpr int T = M >= 256 ? 16 : M >= 64 ? 8 : M >= 16 ? 4 : 2;
+    static constexpr int R1 = M / T;
+    static constexpr int kOwn = R1 / T;  // second digits k1 per thread: 1 or 2
+    static_assert(R1 == T || R1 == 2 * T, "R1 = T or 2T");
+};
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -37,68 +45,94 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // a * conj(b)
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
-// One in-place Stockham pass of radix R (4 or 2) over all tile columns.
-// C[n*kTile + c] holds element n of column c; tw[t] = e^{+2 pi i t / M}.
-// SIGN = +1 forward (e^{+i}), -1 inverse.
-template <int M, int R, int SIGN, int NT>
-__device__ __forceinline__ void stockham_pass(double2 *C, const double2 *tw, int Ns) {
-    constexpr int kTile = tile_cols<M>();
-    constexpr int kTotal = kTile * (M / R);
-    constexpr int kItems = (kTotal + NT - 1) / NT;  // butterflies per thread
-    double2 v[kItems][R];
-    const int tid = threadIdx.x;
+// v <- its R-point transform, natural order; S = +1: e^{+i}, -1: e^{-i}.
+template <int S>
+__device__ __forceinline__ double2 times_i(double2 a) {
+    return (S > 0) ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
+}
+template <int S>
+__device__ __forceinline__ void dft4(double2 &a, double2 &b, double2 &c, double2 &d) {
+    const double2 s0 = cadd(a, c), s1 = csub(a, c), s2 = cadd(b, d), s3 = times_i<S>(csub(b, d));
+    a = cadd(s0, s2);
+    b = cadd(s1, s3);
+    c = csub(s0, s2);
+    d = csub(s1, s3);
+}
+template <int R, int S>
+__device__ __forceinline__ void dft(double2 *v) {
+    constexpr double h = 0.70710678118654752440, c1 = 0.92387953251128675613, s1 = 0.38268343236508977173;
+    if (R == 2) {
+        const double2 a = v[0], b = v[1];
+        v[0] = cadd(a, b);
+        v[1] = csub(a, b);
+    } else if (R == 4) {
+        dft4<S>(v[0], v[1], v[2], v[3]);
+    } else if (R == 8) {
+        double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft4<S>(e[0], e[1], e[2], e[3]);
+        dft4<S>(o[0], o[1], o[2], o[3]);
+        o[1] = cmul(o[1], make_double2(h, S * h));
+        o[2] = times_i<S>(o[2]);
+        o[3] = cmul(o[3], make_double2(-h, S * h));
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        int it = tid + i * NT;
-        if (kTotal % NT != 0 && it >= kTotal) break;
-        int c = it % kTile, j = it / kTile;
-        int k = j % Ns;
-        int tstep = k * (M / (Ns * R));
+        for (int k = 0; k < 4; ++k) {
+            v[k] = cadd(e[k], o[k]);
+            v[k + 4] = csub(e[k], o[k]);
+        }
+    } else {  // 16 = 4 x 4
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            double2 x = C[(j + r * (M / R)) * kTile + c];
-            if (r > 0) {
-                double2 w = tw[r * tstep];
-                x = (SIGN > 0) ? cmul(x, w) : cmulc(x, w);
+        for (int b = 0; b < 4; ++b) dft4<S>(v[b], v[4 + b], v[8 + b], v[12 + b]);
+        // v[4 p + b] holds digit p of column b: twiddle e^{2 pi i b p / 16}
+        v[5] = cmul(v[5], make_double2(c1, S * s1));
+        v[6] = cmul(v[6], make_double2(h, S * h));
+        v[7] = cmul(v[7], make_double2(s1, S * c1));
+        v[9] = cmul(v[9], make_double2(h, S * h));
+        v[10] = times_i<S>(v[10]);
+        v[11] = cmul(v[11], make_double2(-h, S * h));
+        v[13] = cmul(v[13], make_double2(s1, S * c1));
+        v[14] = cmul(v[14], make_double2(-h, S * h));
+        v[15] = cmul(v[15], make_double2(-c1, -S * s1));
+#pragma unroll
+        for (int p = 0; p < 4; ++p) dft4<S>(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
+        // v[4 p + q] = X[p + 4 q]: to natural order
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int q = p + 1; q < 4; ++q) {
+                const double2 x = v[4 * p + q];
+                v[4 * p + q] = v[4 * q + p];
+                v[4 * q + p] = x;
             }
-            v[i][r] = x;
-        }
     }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        int it = tid + i * NT;
-        if (kTotal % NT != 0 && it >= kTotal) break;
-        int c = it % kTile, j = it / kTile;
-        int k = j % Ns;
-        int base = (j / Ns) * Ns * R + k;
-        if (R == 4) {
-            double2 a0 = cadd(v[i][0], v[i][2]), a1 = csub(v[i][0], v[i][2]);
-            double2 a2 = cadd(v[i][1], v[i][3]), d = csub(v[i][1], v[i][3]);
-            double2 a3 = (SIGN > 0) ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);
-            C[(base + 0 * Ns) * kTile + c] = cadd(a0, a2);
-            C[(base + 1 * Ns) * kTile + c] = cadd(a1, a3);
-            C[(base + 2 * Ns) * kTile + c] = csub(a0, a2);
-            C[(base + 3 * Ns) * kTile + c] = csub(a1, a3);
-        } else {
-            C[(base + 0 * Ns) * kTile + c] = cadd(v[i][0], v[i][1]);
-            C[(base + 1 * Ns) * kTile + c] = csub(v[i][0], v[i][1]);
-        }
-    }
-    __syncthreads();
 }
 
-template <int M, int SIGN, int NT>
-__device__ __forceinline__ void fft_tile(double2 *C, const double2 *tw) {
-    int Ns = 1;
-#pragma unroll
-    for (int len = M; len >= 4; len /= 4) {
-        stockham_pass<M, 4, SIGN, NT>(C, tw, Ns);
-        Ns *= 4;
-    }
-    if ((M & 0x55555555) == 0) {  // log2(M) odd: one radix-2 pass remains
-        stockham_pass<M, 2, SIGN, NT>(C, tw, Ns);
-    }
+// Second digits of thread u of a column.  kOwn = 2: u and R1 - u (u = 0: 0 and
+// R1/2), so that k = k1 + R1 k2 of one list pairs with M - k of the other.
+// kOwn = 1: lanes 2i and 2i + 1 of a column (16 lanes apart) take i and R1 - i
+// (i = 0: 0 and R1/2).
+template <int M>
+__device__ __forceinline__ int second_digit(int u, int which) {
+    constexpr int R1 = Split<M>::R1;
+    if (Split<M>::kOwn == 2) return which == 0 ? u : (u == 0 ? R1 / 2 : R1 - u);
+    const int i = u >> 1;
+    return (u & 1) == 0 ? i : (i == 0 ? R1 / 2 : R1 - i);
+}
+
+__device__ __forceinline__ double2 shfl_xor2(double2 v, int mask) {
+    return make_double2(__shfl_xor_sync(0xffffffffu, v.x, mask), __shfl_xor_sync(0xffffffffu, v.y, mask));
+}
+
+// F_k of the real spectrum from the packed transform's values at k and M - k.
+__device__ __forceinline__ double2 real_split(double2 zk, double2 zm, double2 w) {
+    const double2 e = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
+    const double2 o = make_double2(0.5 * (zk.y + zm.y), -0.5 * (zk.x - zm.x));
+    return cadd(e, cmul(w, o));
+}
+// Z_k of the packed transform from the real spectrum at k and M - k.
+__device__ __forceinline__ double2 real_merge(double2 fk, double2 fm, double2 w) {
+    const double2 e = make_double2(0.5 * (fk.x + fm.x), 0.5 * (fk.y - fm.y));
+    const double2 o = cmulc(make_double2(0.5 * (fk.x - fm.x), 0.5 * (fk.y + fm.y)), w);
+    return make_double2(e.x - o.y, e.y + o.x);
 }
 
 // Batched launches: blockIdx.y is the batch position.  in / outp hold each
@@ -117,18 +151,17 @@ struct FftBatch {
 // Threads and shared bytes of a tile (the same for both register budgets).
 template <int M>
 struct FftTile {
-    static constexpr int kThreads = (M >= 256) ? 256 : 128;
-    static constexpr size_t kSmem = sizeof(double2) * ((size_t)M * tile_cols<M>() + M + (M + 1));
+    static constexpr int kThreads = Split<M>::T * kTile;
+    static constexpr size_t kSmem = sizeof(double2) * ((size_t)M * kTile + M + (M + 1));
 };
 
-// Resident CTAs per SM the register budget is sized for (the loads of a
-// tile are all in flight at once; more CTAs hide more of their latency).
-// Dense = 1: eight CTAs of 64 registers per SM for the 128-thread tiles (no
-// spills), chosen by the set-up autotuner or with BPH_FFT_DENSE=1.
+// Resident threads per SM the register budget is sized for: 512 (128
+// registers hold 16 values and a transform's temporaries; a thread has all its
+// loads in flight at once), or, dense, 768.  The set-up autotuner or
+// BPH_FFT_DENSE chooses.
 template <int M, int Dense = 0>
 struct FftShape : FftTile<M> {
-    static constexpr int kMinBlocksFwd = (M >= 256) ? 2 : (Dense ? 8 : 5);
-    static constexpr int kMinBlocksInv = (M >= 256) ? 1 : (Dense ? 8 : 4);
+    static constexpr int kMinBlocks = (Dense ? 768 : 512) / FftTile<M>::kThreads;
 };
 
 // Forward transform of interior columns.  kRho: write R = -4 pi rho_hat
@@ -137,21 +170,20 @@ struct FftShape : FftTile<M> {
 // from the same spectrum: sum_l rho_l e^{i k (l - 1/2) dphi} = e^{i pi k/N} F_k.
 // !kRho: write the warm-start potential into P's interior.
 template <int M, bool kRho, int Dense = 0>
-__global__ void __launch_bounds__(FftTile<M>::kThreads, (FftShape<M, Dense>::kMinBlocksFwd))
+__global__ void __launch_bounds__(FftTile<M>::kThreads, (FftShape<M, Dense>::kMinBlocks))
 k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__restrict__ mom,
           const double2 *__restrict__ g_tw, const double2 *__restrict__ g_tw2, const double2 *__restrict__ g_ph,
           int numr, int numz, int nr, int nz, int mmax, int fm, int isym, double four_pi,
           int *__restrict__ status, long long mstride, FftBatch bt) {
-    constexpr int kTile = tile_cols<M>();
-    constexpr int NT = FftTile<M>::kThreads;
+    constexpr int NT = FftTile<M>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
     extern __shared__ double2 smem[];
-    double2 *C = smem;
+    double2 *C = smem;  // [k1][t][column]
     double2 *tw = C + M * kTile;
     double2 *tw2 = tw + M;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, c = tid % kTile, t = tid / kTile;
     const long long np = (long long)nr * nz;
     const long long nplane = (long long)numr * numz;
-    const long long p0 = (long long)blockIdx.x * kTile;
+    const long long p = (long long)blockIdx.x * kTile + c;
     for (int i = tid; i < M; i += NT) tw[i] = g_tw[i];
     for (int i = tid; i <= M; i += NT) tw2[i] = g_tw2[i];
     pdl_wait();
@@ -164,113 +196,115 @@ k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__re
             status += pos * bt.status_stride;
         }
     }
-    // Load: thread -> (column c fixed, sample pairs n = n0, n0 + NT/kTile, ...);
-    // all global loads are issued before any shared-memory store.
-    static_assert(NT % kTile == 0, "threads must cover whole tile rows");
-    constexpr int kRowsPerPass = NT / kTile, kLoads = M / kRowsPerPass;
-    bool bad = false;
+    const bool valid = p < np;
+    const int jz = valid ? (int)p % nr + 1 : 1, kz = valid ? (int)p / nr + 1 : 1;
     {
-        const int c = tid % kTile, n0 = tid / kTile;
-        const long long p = p0 + c;
-        const bool valid = p < np;
-        const double *col = src;
-        if (valid) col = src + ((int)p % nr + 1) + (long long)numr * ((int)p / nr + 1);
-        double2 v[kLoads];
+        // packed values T r + t, all loads in flight
+        const double *col = src + jz + (long long)numr * kz + nplane * (2 * t);
+        double2 v[R1];
 #pragma unroll
-        for (int i = 0; i < kLoads; ++i) {
-            const int n = n0 + i * kRowsPerPass;
-            v[i] = valid ? make_double2(__ldg(col + nplane * (2 * n)), __ldg(col + nplane * (2 * n + 1)))
+        for (int r = 0; r < R1; ++r)
+            v[r] = valid ? make_double2(__ldg(col + nplane * (2 * T * r)), __ldg(col + nplane * (2 * T * r + 1)))
                          : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int i = 0; i < kLoads; ++i) {
-            if (kRho) bad |= !(isfinite(v[i].x) && isfinite(v[i].y));
-            C[(n0 + i * kRowsPerPass) * kTile + c] = v[i];
-        }
-    }
-    if (kRho && bad) atomicOr(status, kStatusNonFinite);
-    __syncthreads();
-    fft_tile<M, +1, NT>(C, tw);
-    pdl_trigger();
-    // Post-process pairs (k, M-k) into F_k, F_{M-k}; write slots.  The tile
-    // column of a thread is the same in every iteration (NT % kTile == 0).
-    const int c = tid % kTile;
-    const long long p = p0 + c;
-    if (p >= np) return;
-    const int pi = (int)p;
-    const int jz = pi % nr + 1, kz = pi / nr + 1;
-    const bool zeroed = (jz == numr - 2) || (kz == numz - 2) || (isym == 1 && kz == 1);
-    for (int k = tid / kTile; k <= M / 2; k += NT / kTile) {
-        double2 Fk, Fm;  // F_k and F_{M-k} (for k = 0: F_0 and F_M, both real)
-        if (k == 0) {
-            double2 z = C[c];
-            Fk = make_double2(z.x + z.y, 0.0);
-            Fm = make_double2(z.x - z.y, 0.0);
-        } else if (2 * k == M) {
-            Fk = C[k * kTile + c];
-            Fm = Fk;
-        } else {
-            double2 zk = C[k * kTile + c], zm = C[(M - k) * kTile + c];
-            double2 e = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
-            double2 d = make_double2(zk.x - zm.x, zk.y + zm.y);
-            double2 o = make_double2(0.5 * d.y, -0.5 * d.x);
-            Fk = cadd(e, cmul(tw2[k], o));
-            double2 e2 = make_double2(e.x, -e.y);
-            double2 d2 = make_double2(zm.x - zk.x, zm.y + zk.y);
-            double2 o2 = make_double2(0.5 * d2.y, -0.5 * d2.x);
-            Fm = cadd(e2, cmul(tw2[M - k], o2));
-        }
-        // Slot values: s = k -> Re F_k (F_0 at 0), s = M + k -> -Im F_k, s = M -> F_M.
-        const int ka = k, kb = M - k;
-        double sa_re = Fk.x, sa_im = -Fk.y, sb_re = Fm.x, sb_im = -Fm.y;
         if (kRho) {
-            double *o = out + p;
-            if (k == 0) {
-                o[0] = zeroed ? 0.0 : -(four_pi * sa_re);
-                o[np * M] = zeroed ? 0.0 : -(four_pi * sb_re);
-            } else {
-                o[np * ka] = zeroed ? 0.0 : -(four_pi * sa_re);
-                o[np * (M + ka)] = zeroed ? 0.0 : -(four_pi * sa_im);
-                if (kb != ka) {
-                    o[np * kb] = zeroed ? 0.0 : -(four_pi * sb_re);
-                    o[np * (M + kb)] = zeroed ? 0.0 : -(four_pi * sb_im);
-                }
-            }
-            // Moments for boundary modes m with fm*m in {ka, kb}.
-#pragma unroll 1
-            for (int side = 0; side < 2; ++side) {
-                int kk = side ? kb : ka;
-                if (side && kb == ka) break;
-                if (kk == M) continue;
-                if (kk % fm) continue;
-                int m = kk / fm;
-                if (m >= mmax) continue;
-                double2 F = side ? Fm : Fk;
-                double tc, ts;
-                if (m == 0) {
-                    tc = F.x;
-                    ts = 0.0;
-                } else {
-                    double2 ph = g_ph[m];
-                    tc = ph.x * F.x - ph.y * F.y;
-                    ts = ph.y * F.x + ph.x * F.y;
-                }
-                mom[m * mstride + p] = tc;
-                mom[m * mstride + np + p] = ts;
+            bool bad = false;
+#pragma unroll
+            for (int r = 0; r < R1; ++r) bad |= !(isfinite(v[r].x) && isfinite(v[r].y));
+            if (bad) atomicOr(status, kStatusNonFinite);
+        }
+        dft<R1, +1>(v);
+        __syncthreads();  // the twiddles
+        double2 *mine = C + t * kTile + c;
+        mine[0] = v[0];
+#pragma unroll
+        for (int k = 1; k < R1; ++k) mine[k * T * kTile] = cmul(v[k], tw[t * k]);
+    }
+    __syncthreads();
+    double2 x[kOwn][T];
+    int k1[kOwn];
+#pragma unroll
+    for (int o = 0; o < kOwn; ++o) {
+        k1[o] = second_digit<M>(t, o);
+        const double2 *in = C + k1[o] * T * kTile + c;
+#pragma unroll
+        for (int k2 = 0; k2 < T; ++k2) x[o][k2] = in[k2 * kTile];
+        dft<T, +1>(x[o]);
+    }
+    pdl_trigger();
+    const bool zeroed = (jz == numr - 2) || (kz == numz - 2) || (isym == 1 && kz == 1);
+    const double scale = zeroed ? 0.0 : -four_pi;
+    double *o_ = kRho ? out + p : out + jz + (long long)numr * kz;
+    const long long so = kRho ? np : nplane;
+    // Slot values: s = k -> Re F_k (F_0 at 0), s = M + k -> -Im F_k, s = M -> F_M.
+    auto emit = [&](int k, double2 F) {
+        if (!valid) return;
+        if (!kRho) {
+            o_[so * k] = F.x;
+            o_[so * (M + k)] = -F.y;
+            return;
+        }
+        o_[so * k] = zeroed ? 0.0 : scale * F.x;
+        o_[so * (M + k)] = zeroed ? 0.0 : -(scale * F.y);
+        // the boundary mode m with fm m = k
+        if (k < fm * mmax && k % fm == 0) {
+            const int m = k / fm;
+            const double2 ph = g_ph[m];
+            mom[m * mstride + p] = ph.x * F.x - ph.y * F.y;
+            mom[m * mstride + np + p] = ph.y * F.x + ph.x * F.y;
+        }
+    };
+    auto emit_ends = [&](double2 z) {  // k = 0: F_0 and F_M, both real
+        if (!valid) return;
+        const double f0 = z.x + z.y, fM = z.x - z.y;
+        if (!kRho) {
+            o_[0] = f0;
+            o_[so * M] = fM;
+            return;
+        }
+        o_[0] = zeroed ? 0.0 : scale * f0;
+        o_[so * M] = zeroed ? 0.0 : scale * fM;
+        mom[p] = f0;
+        mom[np + p] = 0.0;
+    };
+    if (kOwn == 2) {
+        constexpr int B = kOwn - 1;
+        if (t > 0) {
+#pragma unroll
+            for (int k2 = 0; k2 < T; ++k2) {
+                const int k = k1[0] + R1 * k2;
+                const double2 a = x[0][k2], b = x[B][T - 1 - k2];
+                emit(k, real_split(a, b, tw2[k]));
+                emit(M - k, real_split(b, a, tw2[M - k]));
             }
         } else {
-            double *o = out + jz + (long long)numr * kz;
-            if (k == 0) {
-                o[0] = sa_re;
-                o[nplane * M] = sb_re;
-            } else {
-                o[nplane * ka] = sa_re;
-                o[nplane * (M + ka)] = sa_im;
-                if (kb != ka) {
-                    o[nplane * kb] = sb_re;
-                    o[nplane * (M + kb)] = sb_im;
-                }
+            emit_ends(x[0][0]);
+            emit(M / 2, x[0][T / 2]);
+#pragma unroll
+            for (int k2 = 1; k2 < T / 2; ++k2) {
+                const int k = R1 * k2;
+                emit(k, real_split(x[0][k2], x[0][T - k2], tw2[k]));
+                emit(M - k, real_split(x[0][T - k2], x[0][k2], tw2[M - k]));
             }
+#pragma unroll
+            for (int k2 = 0; k2 < T; ++k2) {
+                const int k = R1 / 2 + R1 * k2;
+                emit(k, real_split(x[B][k2], x[B][T - 1 - k2], tw2[k]));
+            }
+        }
+    } else {
+        // t = 0 and 1 (the first warp) pair within themselves, others with the lane across
+#pragma unroll
+        for (int k2 = 0; k2 < T; ++k2) {
+            const int k = k1[0] + R1 * k2;
+            double2 zm;
+            if (t >= 2)
+                zm = shfl_xor2(x[0][T - 1 - k2], kTile);
+            else
+                zm = t == 0 ? x[0][(T - k2) % T] : x[0][T - 1 - k2];
+            if (k2 == 0 && t == 0)
+                emit_ends(x[0][0]);
+            else
+                emit(k, (t == 0 && 2 * k2 == T) ? x[0][k2] : real_split(x[0][k2], zm, tw2[k]));
         }
     }
 }
@@ -285,19 +319,18 @@ k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__re
 // phieff = pot - 0.5 omega^2 rhf(J)^2 that the hydro source step forms from
 // pot (source.F90:156, make_source_temp.F90:121), saving it a full pass.
 template <int M, int Dense = 0>
-__global__ void __launch_bounds__(FftTile<M>::kThreads, (FftShape<M, Dense>::kMinBlocksInv))
+__global__ void __launch_bounds__(FftTile<M>::kThreads, (FftShape<M, Dense>::kMinBlocks))
 k_fft_inv(const double *__restrict__ P, double *__restrict__ pot, const double2 *__restrict__ g_tw,
           const double2 *__restrict__ g_tw2, int numr, int numz, int isym, double *__restrict__ phieff,
           const double *__restrict__ rhf, double omega, FftBatch bt) {
-    constexpr int kTile = tile_cols<M>();
-    constexpr int NT = FftTile<M>::kThreads;
+    constexpr int NT = FftTile<M>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
     extern __shared__ double2 smem[];
-    double2 *C = smem;
+    double2 *C = smem;  // [k1][t][column]
     double2 *tw = C + M * kTile;
     double2 *tw2 = tw + M;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, c = tid % kTile, t = tid / kTile;
     const long long nplane = (long long)numr * numz;
-    const long long q0 = (long long)blockIdx.x * kTile;
+    const long long q = (long long)blockIdx.x * kTile + c;
     for (int i = tid; i < M; i += NT) tw[i] = g_tw[i];
     for (int i = tid; i <= M; i += NT) tw2[i] = g_tw2[i];
     pdl_wait();
@@ -306,94 +339,127 @@ k_fft_inv(const double *__restrict__ P, double *__restrict__ pot, const double2 
         P += (long long)(bt.inst ? bt.inst[pos] : pos) * bt.inst_stride;
         pot = bt.outp[pos];
     }
-    // Load slots: thread -> (column c fixed, slot pairs (k, M+k)); all global
-    // loads are issued before any shared-memory store.
-    constexpr int kRowsPerPass = NT / kTile, kLoads = M / kRowsPerPass;
+    const bool valid = q < nplane;
     {
-        const int c = tid % kTile, k0 = tid / kTile;
-        const long long q = q0 + c;
-        const bool valid = q < nplane;
-        int jz = 0, kz = 0;
-        if (valid) {
-            jz = (int)q % numr;
-            kz = (int)q / numr;
-        }
+        const int jz = valid ? (int)q % numr : 0, kz = valid ? (int)q / numr : 0;
         const int js = (jz == 0) ? 1 : jz;
         const int ks = (kz == 0 && isym != 1) ? 1 : kz;
         const bool axis = valid && (jz == 0) && (isym != 3);
         const double *col = P + js + (long long)numr * ks;
-        // two batches of loads in flight (register budget of kMinBlocksInv CTAs per SM)
-        constexpr int kBatch = (kLoads >= 16) ? kLoads / 2 : kLoads;
+        double2 x[kOwn][T];
+        int k1[kOwn];
 #pragma unroll
-        for (int i0 = 0; i0 < kLoads; i0 += kBatch) {
-            double a[kBatch], b[kBatch];
+        for (int o = 0; o < kOwn; ++o) {
+            k1[o] = second_digit<M>(t, o);
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int k = k0 + (i0 + i) * kRowsPerPass;
-                a[i] = valid ? __ldg(col + nplane * k) : 0.0;
-                b[i] = valid ? __ldg(col + nplane * (M + k)) : 0.0;
+            for (int k2 = 0; k2 < T; ++k2) {
+                const int k = k1[o] + R1 * k2;
+                x[o][k2] = valid ? make_double2(__ldg(col + nplane * k), __ldg(col + nplane * (M + k)))
+                                 : make_double2(0.0, 0.0);
             }
+        }
+        __syncthreads();  // the twiddles
+        // F_k = slot_k - i slot_{M+k}; k = 0 keeps (F_0, F_M), both real.  R1 is even, so the
+        // axis columns' sign (-1)^k is that of k1.
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int k = k0 + (i0 + i) * kRowsPerPass;
-                double2 v;
-                if (k == 0) {
-                    v = make_double2(a[i], b[i]);  // (F_0, F_M): both real
-                } else {
-                    v = make_double2(a[i], -b[i]);  // F_k = slot_k - i slot_{M+k}
-                    if (axis && (k & 1)) v = make_double2(-v.x, -v.y);
+        for (int o = 0; o < kOwn; ++o) {
+            const double s = (axis && (k1[o] & 1)) ? -1.0 : 1.0;
+#pragma unroll
+            for (int k2 = 0; k2 < T; ++k2)
+                if (k2 > 0 || k1[o] > 0) x[o][k2] = make_double2(s * x[o][k2].x, -s * x[o][k2].y);
+        }
+        // Z_k = E_k + i O_k
+        if (kOwn == 2) {
+            constexpr int B = kOwn - 1;
+            if (t > 0) {
+#pragma unroll
+                for (int k2 = 0; k2 < T; ++k2) {
+                    const int k = k1[0] + R1 * k2;
+                    const double2 a = x[0][k2], b = x[B][T - 1 - k2];
+                    x[0][k2] = real_merge(a, b, tw2[k]);
+                    x[B][T - 1 - k2] = real_merge(b, a, tw2[M - k]);
                 }
-                C[k * kTile + c] = v;
+            } else {
+                const double2 f = x[0][0];
+                x[0][0] = make_double2(0.5 * (f.x + f.y), 0.5 * (f.x - f.y));
+#pragma unroll
+                for (int k2 = 1; k2 < T / 2; ++k2) {
+                    const int k = R1 * k2;
+                    const double2 a = x[0][k2], b = x[0][T - k2];
+                    x[0][k2] = real_merge(a, b, tw2[k]);
+                    x[0][T - k2] = real_merge(b, a, tw2[M - k]);
+                }
+#pragma unroll
+                for (int k2 = 0; k2 < T / 2; ++k2) {
+                    const int k = R1 / 2 + R1 * k2;
+                    const double2 a = x[B][k2], b = x[B][T - 1 - k2];
+                    x[B][k2] = real_merge(a, b, tw2[k]);
+                    x[B][T - 1 - k2] = real_merge(b, a, tw2[M - k]);
+                }
+            }
+        } else {
+            if (t >= 2) {  // with the lane across (the first warp holds t = 0 and 1)
+#pragma unroll
+                for (int k2 = 0; k2 < T / 2; ++k2) {
+                    const int ka = k1[0] + R1 * k2, kb = k1[0] + R1 * (T - 1 - k2);
+                    const double2 a = x[0][k2], b = x[0][T - 1 - k2];
+                    const double2 fa = shfl_xor2(b, kTile), fb = shfl_xor2(a, kTile);
+                    x[0][k2] = real_merge(a, fa, tw2[ka]);
+                    x[0][T - 1 - k2] = real_merge(b, fb, tw2[kb]);
+                }
+            } else if (t == 0) {
+                const double2 f = x[0][0];
+                x[0][0] = make_double2(0.5 * (f.x + f.y), 0.5 * (f.x - f.y));
+#pragma unroll
+                for (int k2 = 1; k2 < T / 2; ++k2) {
+                    const double2 a = x[0][k2], b = x[0][T - k2];
+                    x[0][k2] = real_merge(a, b, tw2[R1 * k2]);
+                    x[0][T - k2] = real_merge(b, a, tw2[M - R1 * k2]);
+                }
+            } else {
+#pragma unroll
+                for (int k2 = 0; k2 < T / 2; ++k2) {
+                    const int k = R1 / 2 + R1 * k2;
+                    const double2 a = x[0][k2], b = x[0][T - 1 - k2];
+                    x[0][k2] = real_merge(a, b, tw2[k]);
+                    x[0][T - 1 - k2] = real_merge(b, a, tw2[M - k]);
+                }
             }
         }
-    }
-    __syncthreads();
-    // Pre-process into Z_k = E_k + i O_k.
-    for (int it = tid; it < kTile * (M / 2 + 1); it += NT) {
-        int c = it % kTile, k = it / kTile;
-        if (k == 0) {
-            double2 f = C[c];
-            C[c] = make_double2(0.5 * (f.x + f.y), 0.5 * (f.x - f.y));
-        } else if (2 * k != M) {
-            double2 fk = C[k * kTile + c], fm = C[(M - k) * kTile + c];
-            double2 e = make_double2(0.5 * (fk.x + fm.x), 0.5 * (fk.y - fm.y));
-            double2 d = make_double2(0.5 * (fk.x - fm.x), 0.5 * (fk.y + fm.y));
-            double2 o = cmulc(d, tw2[k]);
-            double2 e2 = make_double2(e.x, -e.y);
-            double2 d2 = make_double2(0.5 * (fm.x - fk.x), 0.5 * (fm.y + fk.y));
-            double2 o2 = cmulc(d2, tw2[M - k]);
-            C[k * kTile + c] = make_double2(e.x - o.y, e.y + o.x);
-            C[(M - k) * kTile + c] = make_double2(e2.x - o2.y, e2.y + o2.x);
+#pragma unroll
+        for (int o = 0; o < kOwn; ++o) {
+            dft<T, -1>(x[o]);
+            double2 *dst = C + k1[o] * T * kTile + c;
+            dst[0] = x[o][0];
+#pragma unroll
+            for (int n = 1; n < T; ++n) dst[n * kTile] = cmulc(x[o][n], tw[n * k1[o]]);
         }
     }
     __syncthreads();
-    fft_tile<M, -1, NT>(C, tw);
-    pdl_trigger();
-    const double scale = 1.0 / (double)M;
+    double2 v[R1];
     {
-        const int c = tid % kTile, n0 = tid / kTile;
-        const long long q = q0 + c;
-        if (q < nplane) {
-            double *col = pot + q;
+        const double2 *in = C + t * kTile + c;
 #pragma unroll
-            for (int i = 0; i < kLoads; ++i) {
-                const int n = n0 + i * kRowsPerPass;
-                const double2 z = C[n * kTile + c];
-                col[nplane * (2 * n)] = z.x * scale;
-                col[nplane * (2 * n + 1)] = z.y * scale;
-            }
-            if (phieff) {
-                const double r = rhf[(int)q % numr];
-                const double cen = 0.5 * omega * omega * r * r;
-                double *pe = phieff + q;
+        for (int k = 0; k < R1; ++k) v[k] = in[k * T * kTile];
+    }
+    dft<R1, -1>(v);
+    pdl_trigger();
+    if (!valid) return;
+    const double scale = 1.0 / (double)M;
+    double *col = pot + q + nplane * (2 * t);
 #pragma unroll
-                for (int i = 0; i < kLoads; ++i) {
-                    const int n = n0 + i * kRowsPerPass;
-                    const double2 z = C[n * kTile + c];
-                    pe[nplane * (2 * n)] = z.x * scale - cen;
-                    pe[nplane * (2 * n + 1)] = z.y * scale - cen;
-                }
-            }
+    for (int r = 0; r < R1; ++r) {
+        col[nplane * (2 * T * r)] = v[r].x * scale;
+        col[nplane * (2 * T * r + 1)] = v[r].y * scale;
+    }
+    if (phieff) {
+        const double rad = rhf[(int)q % numr];
+        const double cen = 0.5 * omega * omega * rad * rad;
+        double *pe = phieff + q + nplane * (2 * t);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) {
+            pe[nplane * (2 * T * r)] = v[r].x * scale - cen;
+            pe[nplane * (2 * T * r + 1)] = v[r].y * scale - cen;
         }
     }
 }
@@ -417,7 +483,6 @@ cudaError_t set_fft_attrs(bph_ctx *c) {
 template <int M>
 cudaError_t fwd_rho(bph_ctx *c, const double *rho, double *R, double *mom, long long mstride, int *status,
                     FftBatch bt, int npos) {
-    constexpr int kTile = tile_cols<M>();
     unsigned blocks = (unsigned)((c->np + kTile - 1) / kTile);
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg =
@@ -433,7 +498,6 @@ cudaError_t fwd_rho(bph_ctx *c, const double *rho, double *R, double *mom, long 
 
 template <int M>
 cudaError_t fwd_pot(bph_ctx *c, const double *pot) {
-    constexpr int kTile = tile_cols<M>();
     unsigned blocks = (unsigned)((c->np + kTile - 1) / kTile);
     k_fft_fwd<M, false><<<blocks, FftTile<M>::kThreads, FftTile<M>::kSmem, c->stream>>>(
         pot, c->d_P, nullptr, c->d_tw, c->d_tw2, c->d_ph, c->g.numr, c->g.numz, c->nr, c->nz, c->g.mmax, c->fm,
@@ -443,7 +507,6 @@ cudaError_t fwd_pot(bph_ctx *c, const double *pot) {
 
 template <int M>
 cudaError_t inv(bph_ctx *c, double *pot, double *phieff, double omega, const double *P, FftBatch bt, int npos) {
-    constexpr int kTile = tile_cols<M>();
     unsigned blocks = (unsigned)((c->nplane + kTile - 1) / kTile);
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg =
