@@ -560,7 +560,11 @@ int solve_device(bph_ctx *c, const double *d_rho, double *d_pot, const Schedule 
     BPH_CUDA(launch_fft_fwd_rho(c, d_rho));
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (c->green) BPH_CUDA(cudaStreamIsCapturing(c->stream, &cap));
-    const bool split = c->overlap && (c->adi_seg || modal_ready(c, s)) && c->nfree > 0 && c->nfree < c->N;
+    // A handful of free slots is not worth a second stream (66 x 66 x 64, 5 of 64: 53.3 us against
+    // 50.5), and beside slots beyond shared memory the contraction finds no idle SM (258 x 194 x 512:
+    // 1592 against 1578); else the overlap pays (101 x 75 x 128: 107 against 117, 130 x 98 x 256: 169
+    // against 187).
+    const bool split = c->overlap && c->adi_seg && 8 * c->nfree >= c->N && c->nfree < c->N;
     if (c->green && cap == cudaStreamCaptureStatusNone && split) {
         // contraction on partition 0, free-slot ADI on partition 1, both from the forward FFT
         BPH_CUDA(cudaEventRecord(c->ev_fft, c->stream));
