@@ -588,7 +588,7 @@ int solve_device(bph_ctx *c, const double *d_rho, double *d_pot, const Schedule 
         BPH_CUDA(cudaStreamWaitEvent(c->side_stream, c->ev_fft, 0));
         BPH_CUDA(launch_adi_slots(c, s, cold, c->d_slot_map, c->nfree, c->side_stream, false));
         BPH_CUDA(cudaEventRecord(c->ev_free, c->side_stream));
-        BPH_CUDA(launch_green_contract(c));  // also writes the Dirichlet slots
+        BPH_CUDA(launch_green_contract(c, true, true));  // also writes the Dirichlet slots
         BPH_CUDA(launch_adi_slots(c, s, cold, c->d_slot_map + c->nfree, c->N - c->nfree, c->stream, c->pdl));
         BPH_CUDA(cudaStreamWaitEvent(c->stream, c->ev_free, 0));
         PdlOff off(c);

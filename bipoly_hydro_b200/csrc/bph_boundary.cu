@@ -231,11 +231,13 @@ __global__ void k_boundary_slots(const double *__restrict__ S, const double2 *__
 // Tile warps (one tile (I, J) over the item's heights): a ring of kRing
 // stages of kStageH heights per warp; lane l copies its 16 bytes of each
 // height's 512 (evict-first) and one of the 32 moments a height needs
-// ((cos, sin) pairs of the rows 8I.. and the columns 8J..).  Lane
-// (r = l / 4, c0 = 2 (l % 4)) then accumulates
+// ((cos, sin) pairs of the rows 8I.. and the columns 8J..).  A half-warp
+// takes every other height, and a lane two rows and two columns of its tile:
+// six 16-byte shared-memory words for 16 FMA, where a row and two columns per
+// lane over the whole warp took eight.  It accumulates
 //   row part:    sum_k H(8I + r, 8J + c, k) mom(8J + c, k)   -> S[8I + r]
 //   column part: sum_k H(8I + r, 8J + c, k) mom(8I + r, k)   -> S[8J + c]
-// for c = c0, c0 + 1 (the column part is the mirrored tile (J, I), unused
+// (the column part is the mirrored tile (J, I), unused
 // when I == J).  The radii r_j of G = H r_j scale the sums at the end;
 // shuffles reduce them over the tile's rows and columns in a fixed order.
 //
@@ -261,6 +263,7 @@ struct CompactArgs {
     unsigned int *cnt;  // arrival counters (compact::counters)
     long long np, part_m, part_h;
     int nr, nz, nzp, nb, nb8, npair, nsets, stride, top_ctas, side_ctas, mmax, nh, hp;
+    int tiles_first;  // item order: every mode's tile sets before the side groups, or mode by mode
     SlotOut so;
 };
 
@@ -268,6 +271,7 @@ constexpr int kRing = 4;                            // stages in a tile warp's r
 constexpr int kStageH = compact::kStageHeights;     // heights per stage
 constexpr int kHeightDoubles = 64 + 32;     // a height: 64 tile elements, 16 (cos, sin) moment pairs
 constexpr int kStageDoubles = kStageH * kHeightDoubles;
+static_assert(kStageH % 2 == 0, "a stage is shared by two half-warps");
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cpa16(void *dst, const void *src) {
@@ -306,10 +310,19 @@ __device__ __forceinline__ void compact_item(const CompactArgs &a, int it, doubl
     const int nr = a.nr, nz = a.nz;
     const long long np = a.np;
     const int per_m = a.top_ctas + a.side_ctas;
-    const int per_mode_items = a.nh * per_m;
-    const int m = it / per_mode_items;
-    const int rem = it % per_mode_items;
-    const int h = rem / per_m, role = rem % per_m;
+    int m, h, role;
+    if (a.tiles_first) {
+        const int ntop = a.mmax * a.nh * a.top_ctas;
+        const bool top = it < ntop;
+        const int per = top ? a.top_ctas : a.side_ctas, rel = top ? it : it - ntop;
+        m = rel / (a.nh * per);
+        h = rel % (a.nh * per) / per;
+        role = rel % per + (top ? 0 : a.top_ctas);
+    } else {
+        m = it / (a.nh * per_m);
+        h = it % (a.nh * per_m) / per_m;
+        role = it % per_m;
+    }
     const int k0 = min(h * a.hp, nz), k1 = min(k0 + a.hp, nz);
     const double *mc = a.mom + 2LL * m * np;
     double *pmode = a.part + (long long)m * a.part_m;
@@ -324,8 +337,9 @@ __device__ __forceinline__ void compact_item(const CompactArgs &a, int it, doubl
             double *ring = csm + warp * kRing * kStageDoubles;
             const long long hstride = (long long)a.npair * 64;  // doubles between heights of a tile
             const int nst = (k1 - k0 + kStageH - 1) / kStageH;
-            const int r = lane >> 2, c0 = 2 * (lane & 3);
-            double r0c = 0.0, r0s = 0.0, r1c = 0.0, r1s = 0.0, k0c = 0.0, k0s = 0.0, k1c = 0.0, k1s = 0.0;
+            // half-warp hw takes every other height; its lane (rp, c0 / 2) rows rp and rp + 4, columns c0 and c0 + 1
+            const int hw = lane >> 4, rp = (lane >> 2) & 3, c0 = 2 * (lane & 3);
+            double rowc[2][2] = {}, rows[2][2] = {}, colc[2][2] = {}, cols[2][2] = {};  // [row][column], (cos, sin)
             unsigned long long evict_first;
             asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(evict_first));
             // the lane's table bytes and moment of height k0; both advance by fixed strides per height
@@ -383,52 +397,66 @@ __device__ __forceinline__ void compact_item(const CompactArgs &a, int it, doubl
                 cpa_commit();
                 const double *st = ring + (sidx & (kRing - 1)) * kStageDoubles;
 #pragma unroll
-                for (int hh = 0; hh < kStageH; ++hh) {
+                for (int hh = 0; hh < kStageH; hh += 2) {
                     // heights past k1 within the last stage are zero tiles (padding above nz)
-                    const double *sh = st + hh * kHeightDoubles;
-                    const double2 t = *reinterpret_cast<const double2 *>(sh + 2 * lane);
-                    const double2 x0 = *reinterpret_cast<const double2 *>(sh + 64 + 2 * (8 + c0));
-                    const double2 x1 = *reinterpret_cast<const double2 *>(sh + 64 + 2 * (9 + c0));
-                    const double2 y = *reinterpret_cast<const double2 *>(sh + 64 + 2 * r);
-                    r0c = fma(t.x, x0.x, r0c);
-                    r0s = fma(t.x, x0.y, r0s);
-                    r1c = fma(t.y, x1.x, r1c);
-                    r1s = fma(t.y, x1.y, r1s);
-                    k0c = fma(t.x, y.x, k0c);
-                    k0s = fma(t.x, y.y, k0s);
-                    k1c = fma(t.y, y.x, k1c);
-                    k1s = fma(t.y, y.y, k1s);
+                    const double *sh = st + (hh + hw) * kHeightDoubles;
+                    double2 t[2], x[2], y[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        t[i] = *reinterpret_cast<const double2 *>(sh + 8 * (rp + 4 * i) + c0);
+                        x[i] = *reinterpret_cast<const double2 *>(sh + 64 + 2 * (8 + c0 + i));
+                        y[i] = *reinterpret_cast<const double2 *>(sh + 64 + 2 * (rp + 4 * i));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const double g = c ? t[i].y : t[i].x;
+                            rowc[i][c] = fma(g, x[c].x, rowc[i][c]);
+                            rows[i][c] = fma(g, x[c].y, rows[i][c]);
+                            colc[i][c] = fma(g, y[i].x, colc[i][c]);
+                            cols[i][c] = fma(g, y[i].y, cols[i][c]);
+                        }
                 }
             }
             cpa_wait<0>();
             // G = H r_j: the row part takes the columns' radii, the column part the row's
-            const int jr = min(kTile * I + r, nr - 1);
-            const int jc0 = min(kTile * J + c0, nr - 1), jc1 = min(kTile * J + c0 + 1, nr - 1);
-            const double wr = a.rw[jr], w0 = a.rw[jc0], w1 = a.rw[jc1];
-            double rc = w0 * r0c + w1 * r1c, rs = w0 * r0s + w1 * r1s;
-            double cc0 = wr * k0c, cs0 = wr * k0s, cc1 = wr * k1c, cs1 = wr * k1s;
+            const double wr[2] = {a.rw[min(kTile * I + rp, nr - 1)], a.rw[min(kTile * I + rp + 4, nr - 1)]};
+            const double wc[2] = {a.rw[min(kTile * J + c0, nr - 1)], a.rw[min(kTile * J + c0 + 1, nr - 1)]};
+            double rc[2], rs[2], cc[2], cs[2];
 #pragma unroll
-            for (int off = 1; off <= 2; off <<= 1) {
-                rc += __shfl_xor_sync(0xffffffffu, rc, off);
-                rs += __shfl_xor_sync(0xffffffffu, rs, off);
+            for (int i = 0; i < 2; ++i) {
+                rc[i] = wc[0] * rowc[i][0] + wc[1] * rowc[i][1];
+                rs[i] = wc[0] * rows[i][0] + wc[1] * rows[i][1];
+                cc[i] = wr[0] * colc[0][i] + wr[1] * colc[1][i];
+                cs[i] = wr[0] * cols[0][i] + wr[1] * cols[1][i];
             }
+            // rows over the four column lanes, columns over the four row lanes, both over the half-warps
 #pragma unroll
-            for (int off = 4; off <= 16; off <<= 1) {
-                cc0 += __shfl_xor_sync(0xffffffffu, cc0, off);
-                cs0 += __shfl_xor_sync(0xffffffffu, cs0, off);
-                cc1 += __shfl_xor_sync(0xffffffffu, cc1, off);
-                cs1 += __shfl_xor_sync(0xffffffffu, cs1, off);
+            for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                for (int o = 0; o < 3; ++o) {
+                    const int ro = o == 0 ? 1 : o == 1 ? 2 : 16, co = o == 0 ? 4 : o == 1 ? 8 : 16;
+                    rc[i] += __shfl_xor_sync(0xffffffffu, rc[i], ro);
+                    rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], ro);
+                    cc[i] += __shfl_xor_sync(0xffffffffu, cc[i], co);
+                    cs[i] += __shfl_xor_sync(0xffffffffu, cs[i], co);
+                }
             }
             double *pp = part + (long long)q * kPartPair;  // [row | column][8][cos, sin]
-            if ((lane & 3) == 0) {
-                pp[2 * r] = rc;
-                pp[2 * r + 1] = rs;
+            if (hw == 0 && (lane & 3) == 0) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    pp[2 * (rp + 4 * i)] = rc[i];
+                    pp[2 * (rp + 4 * i) + 1] = rs[i];
+                }
             }
             if (lane < 4) {
-                pp[16 + 2 * c0] = cc0;
-                pp[16 + 2 * c0 + 1] = cs0;
-                pp[16 + 2 * c0 + 2] = cc1;
-                pp[16 + 2 * c0 + 3] = cs1;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    pp[16 + 2 * (c0 + i)] = cc[i];
+                    pp[16 + 2 * (c0 + i) + 1] = cs[i];
+                }
             }
         } else {
             pdl_wait();
@@ -658,7 +686,7 @@ int compact_configure(bph_ctx *c) {
     return BPH_OK;
 }
 
-cudaError_t launch_green_compact_contract(bph_ctx *c, bool write_slots) {
+cudaError_t launch_green_compact_contract(bph_ctx *c, bool write_slots, bool shared) {
     const compact::Dims d = compact::dims(c->nr, c->nz, c->g.isym);
     CompactArgs a;
     a.T = c->d_gtile;
@@ -693,6 +721,12 @@ cudaError_t launch_green_compact_contract(bph_ctx *c, bool write_slots) {
     a.hp = d.hp;
     a.nzp = d.nzp;
 
+    // A tile set takes about twice a side group's time, so with a few waves the tile sets go first
+    // and the last wave is one of short items (66 x 66: 23.8 -> 21.4 us, 130 x 98: 63.9 -> 59.2).
+    // Mode by mode the compute of the side rows runs under the tiles' loads, which many waves
+    // (258 x 194: 340 against 363 us) and a solve that shares the SMs with the free slots' ADI
+    // (130 x 98 x 256: 165 against 172 us) want.
+    a.tiles_first = !shared && compact::items(d, c->g.mmax) < 4 * 444;
     a.part_h = compact::part_height_doubles(d);
     ++c->launches;
     cudaLaunchAttribute attr[1];
@@ -702,8 +736,8 @@ cudaError_t launch_green_compact_contract(bph_ctx *c, bool write_slots) {
     return cudaLaunchKernelExC(&cfg, compact_kernel(d.kpl), args);
 }
 
-cudaError_t launch_green_contract(bph_ctx *c, bool write_slots) {
-    if (c->compact) return launch_green_compact_contract(c, write_slots);
+cudaError_t launch_green_contract(bph_ctx *c, bool write_slots, bool shared) {
+    if (c->compact) return launch_green_compact_contract(c, write_slots, shared);
     dim3 grid((unsigned)((c->nb + kContractRows - 1) / kContractRows), (unsigned)c->g.mmax,
               (unsigned)c->contract_split);
     SlotOut so;

@@ -1,8 +1,8 @@
 // bph_fft.cu -- azimuthal real FFTs (realft.F90 + the slot reorder of
 // helmadi.F90:132-183 and its inverse :357-411).
 //
-// A block takes a tile of 16 consecutive (J,K) columns and all numphi samples
-// of each: every row of the tile is a 128-byte segment of the Fortran array
+// A block takes a tile of 16 (or 32) consecutive (J,K) columns and all numphi
+// samples of each: every row of the tile is a 128-byte segment of the Fortran array
 // (J fastest).  The N real samples of a column are M = N/2 complex values,
 // transformed in two steps, M = R1 T: T threads per column hold R1 values
 // each and transform them in registers, exchange them once through shared
@@ -25,7 +25,14 @@
 namespace bph {
 namespace {
 
-constexpr int kTile = 16;  // columns per block
+// Columns per block: 16, a 128-byte row segment; 32 for the 128-point forward
+// transform, whose tiles start one zone into a row and so touch a sector more
+// than their length (130 x 98 x 256: 15.8 -> 13.9 us; the inverse, on whole
+// rows, 9.9 with 16 and 10.5 with 32).
+template <int M, bool kFwd>
+constexpr int tile_cols() {
+    return M == 128 && kFwd ? 32 : 16;
+}
 
 // M = R1 T, both powers of two, R1 = T or 2T.
 template <int M>
@@ -149,19 +156,22 @@ struct FftBatch {
 };
 
 // Threads and shared bytes of a tile (the same for both register budgets).
-template <int M>
+template <int M, bool kFwd>
 struct FftTile {
-    static constexpr int kThreads = Split<M>::T * kTile;
-    static constexpr size_t kSmem = sizeof(double2) * ((size_t)M * kTile + M + (M + 1));
+    static constexpr int kCols = tile_cols<M, kFwd>();
+    static constexpr int kThreads = Split<M>::T * kCols;
+    static constexpr size_t kSmem = sizeof(double2) * ((size_t)M * kCols + M + (M + 1));
+    static_assert(Split<M>::kOwn == 2 || kCols == 16, "paired lanes are 16 apart");
 };
 
 // Resident threads per SM the register budget is sized for: 512 (128
 // registers hold 16 values and a transform's temporaries; a thread has all its
 // loads in flight at once), or, dense, 768.  The set-up autotuner or
-// BPH_FFT_DENSE chooses.
-template <int M, int Dense = 0>
-struct FftShape : FftTile<M> {
-    static constexpr int kMinBlocks = (Dense ? 768 : 512) / FftTile<M>::kThreads;
+// BPH_FFT_DENSE chooses for single transforms; batched ones run against HBM
+// and take the first (130 x 98 x 256, batch of 16: 1788 against 1890 us).
+template <int M, bool kFwd, int Dense = 0>
+struct FftShape : FftTile<M, kFwd> {
+    static constexpr int kMinBlocks = (Dense ? 768 : 512) / FftTile<M, kFwd>::kThreads;
 };
 
 // Forward transform of interior columns.  kRho: write R = -4 pi rho_hat
@@ -170,12 +180,12 @@ struct FftShape : FftTile<M> {
 // from the same spectrum: sum_l rho_l e^{i k (l - 1/2) dphi} = e^{i pi k/N} F_k.
 // !kRho: write the warm-start potential into P's interior.
 template <int M, bool kRho, int Dense = 0>
-__global__ void __launch_bounds__(FftTile<M>::kThreads, (FftShape<M, Dense>::kMinBlocks))
+__global__ void __launch_bounds__((FftTile<M, true>::kThreads), (FftShape<M, true, Dense>::kMinBlocks))
 k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__restrict__ mom,
           const double2 *__restrict__ g_tw, const double2 *__restrict__ g_tw2, const double2 *__restrict__ g_ph,
           int numr, int numz, int nr, int nz, int mmax, int fm, int isym, double four_pi,
           int *__restrict__ status, long long mstride, FftBatch bt) {
-    constexpr int NT = FftTile<M>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
+    constexpr int kTile = tile_cols<M, true>(), NT = FftTile<M, true>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
     extern __shared__ double2 smem[];
     double2 *C = smem;  // [k1][t][column]
     double2 *tw = C + M * kTile;
@@ -319,11 +329,11 @@ k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__re
 // phieff = pot - 0.5 omega^2 rhf(J)^2 that the hydro source step forms from
 // pot (source.F90:156, make_source_temp.F90:121), saving it a full pass.
 template <int M, int Dense = 0>
-__global__ void __launch_bounds__(FftTile<M>::kThreads, (FftShape<M, Dense>::kMinBlocks))
+__global__ void __launch_bounds__((FftTile<M, false>::kThreads), (FftShape<M, false, Dense>::kMinBlocks))
 k_fft_inv(const double *__restrict__ P, double *__restrict__ pot, const double2 *__restrict__ g_tw,
           const double2 *__restrict__ g_tw2, int numr, int numz, int isym, double *__restrict__ phieff,
           const double *__restrict__ rhf, double omega, FftBatch bt) {
-    constexpr int NT = FftTile<M>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
+    constexpr int kTile = tile_cols<M, false>(), NT = FftTile<M, false>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
     extern __shared__ double2 smem[];
     double2 *C = smem;  // [k1][t][column]
     double2 *tw = C + M * kTile;
@@ -466,28 +476,30 @@ k_fft_inv(const double *__restrict__ P, double *__restrict__ pot, const double2 
 
 template <int M>
 cudaError_t set_fft_attrs(bph_ctx *c) {
-    size_t smem = FftTile<M>::kSmem;
-    cudaError_t e = cudaFuncSetAttribute(k_fft_fwd<M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int fwd = (int)FftTile<M, true>::kSmem, inv = (int)FftTile<M, false>::kSmem;
+    cudaError_t e = cudaFuncSetAttribute(k_fft_fwd<M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fft_fwd<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k_fft_fwd<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fft_inv<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k_fft_inv<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fft_fwd<M, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k_fft_fwd<M, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fft_inv<M, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    c->fft_smem_fwd = c->fft_smem_inv = (int)smem;
+        e = cudaFuncSetAttribute(k_fft_inv<M, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, inv);
+    c->fft_smem_fwd = fwd;
+    c->fft_smem_inv = inv;
     return e;
 }
 
 template <int M>
 cudaError_t fwd_rho(bph_ctx *c, const double *rho, double *R, double *mom, long long mstride, int *status,
                     FftBatch bt, int npos) {
+    constexpr int kTile = tile_cols<M, true>();
     unsigned blocks = (unsigned)((c->np + kTile - 1) / kTile);
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg =
-        launch_config(c, dim3(blocks, (unsigned)npos), dim3(FftTile<M>::kThreads), FftTile<M>::kSmem, attr);
-    if (c->fft_dense)
+        launch_config(c, dim3(blocks, (unsigned)npos), dim3(FftTile<M, true>::kThreads), FftTile<M, true>::kSmem, attr);
+    if (c->fft_dense && !bt.in)
         return cudaLaunchKernelEx(&cfg, k_fft_fwd<M, true, 1>, rho, R, mom, (const double2 *)c->d_tw,
                                   (const double2 *)c->d_tw2, (const double2 *)c->d_ph, c->g.numr, c->g.numz, c->nr,
                                   c->nz, c->g.mmax, c->fm, c->g.isym, c->four_pi, status, mstride, bt);
@@ -498,8 +510,9 @@ cudaError_t fwd_rho(bph_ctx *c, const double *rho, double *R, double *mom, long 
 
 template <int M>
 cudaError_t fwd_pot(bph_ctx *c, const double *pot) {
+    constexpr int kTile = tile_cols<M, true>();
     unsigned blocks = (unsigned)((c->np + kTile - 1) / kTile);
-    k_fft_fwd<M, false><<<blocks, FftTile<M>::kThreads, FftTile<M>::kSmem, c->stream>>>(
+    k_fft_fwd<M, false><<<blocks, FftTile<M, true>::kThreads, FftTile<M, true>::kSmem, c->stream>>>(
         pot, c->d_P, nullptr, c->d_tw, c->d_tw2, c->d_ph, c->g.numr, c->g.numz, c->nr, c->nz, c->g.mmax, c->fm,
         c->g.isym, c->four_pi, c->d_status, 0, FftBatch());
     return cudaGetLastError();
@@ -507,11 +520,12 @@ cudaError_t fwd_pot(bph_ctx *c, const double *pot) {
 
 template <int M>
 cudaError_t inv(bph_ctx *c, double *pot, double *phieff, double omega, const double *P, FftBatch bt, int npos) {
+    constexpr int kTile = tile_cols<M, false>();
     unsigned blocks = (unsigned)((c->nplane + kTile - 1) / kTile);
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg =
-        launch_config(c, dim3(blocks, (unsigned)npos), dim3(FftTile<M>::kThreads), FftTile<M>::kSmem, attr);
-    if (c->fft_dense)
+        launch_config(c, dim3(blocks, (unsigned)npos), dim3(FftTile<M, false>::kThreads), FftTile<M, false>::kSmem, attr);
+    if (c->fft_dense && !bt.outp)
         return cudaLaunchKernelEx(&cfg, k_fft_inv<M, 1>, P, pot, (const double2 *)c->d_tw, (const double2 *)c->d_tw2,
                                   c->g.numr, c->g.numz, c->g.isym, phieff, (const double *)c->d_grid, omega, bt);
     return cudaLaunchKernelEx(&cfg, k_fft_inv<M>, P, pot, (const double2 *)c->d_tw, (const double2 *)c->d_tw2,

@@ -281,7 +281,8 @@ cudaError_t launch_fft_inv(bph_ctx *c, double *pot, double *phieff = nullptr, do
                            const double *P = nullptr);
 // write_slots: the contraction also writes the Dirichlet slots of P (the
 // fused form of launch_boundary_slots, which stays for phase timing).
-cudaError_t launch_green_contract(bph_ctx *c, bool write_slots = true);
+// shared: other work runs beside it on the SMs.
+cudaError_t launch_green_contract(bph_ctx *c, bool write_slots = true, bool shared = false);
 cudaError_t launch_boundary_slots(bph_ctx *c);
 // ninst instances of slot arrays P/R; block row i solves instance d_inst_map[i]
 // (nullptr: instance i).
