@@ -206,6 +206,9 @@ struct bph_ctx {
     // ADI in the vertical eigenbasis (bph_modal.cu)
     int modal = 0;                     // 1: the FP64 ADI runs there
     int modal_seg = 0;                 // radii per segment of a radial line
+    int modal_p1 = 0;                  // first factor of the split transforms (0: dense)
+    int modal_beta1 = 0;               // multiplier of its angles
+    int *d_modtab = nullptr;           // split form: signed heights of (a1, a2)
     double *d_modE = nullptr;          // packed fragments of E, then of E^T (one allocation with the next three)
     double *d_modlam = nullptr;        // [nz] gamma lambda_q
     double *d_modY = nullptr;          // [N][nr][nz, even] modal residual / update

@@ -59,7 +59,13 @@ struct ModalArgs {
     int numr, numz, nr, nz, ldq, N, isym, mtiles, ksteps;
     int nsteps, source, add;
     double gamma;
+    // split transforms (p1 > 0)
+    const double *Cs;        // packed A fragments of the cosine matrix, then of the sine matrix
+    const int *tab;          // [p1][h2]: +-(k + 1) of (a1, a2), 0: none
+    int h2, mt2, ks2;        // rows of the second factor's matrices, their 16-row tiles and 8-row steps
+    double s1[4][4], c1[4][4];  // sines and cosines of the first factor
 };
+
 
 // What k_modal_fwd transforms.
 enum { kResidual = 0, kColdResidual = 1, kPotential = 2 };
@@ -124,14 +130,13 @@ __device__ __forceinline__ void tile_product(const ModalArgs &a, const double *s
     }
 }
 
-// Block: 8 NT columns of a slot, all rows.  The residual is formed once per
-// column tile, a warp per band of rows with the rows below and at hand kept
-// in registers, and stays in shared memory as the B operand.
+// What a block transforms, 8 NT columns of a slot with all rows, into
+// sx[row][column]: the residual is formed once per column tile, a warp per
+// band of rows with the rows below and at hand kept in registers.  Waits for
+// the previous kernel.
 template <int NT>
-__global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
-    extern __shared__ double sx[];
+__device__ __forceinline__ void source_tile(const ModalArgs &a, const TileIndex &ti, double *sx) {
     constexpr int ld = TileShape<NT>::ld;
-    const TileIndex ti = tile_index(a, a.ntile);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, numr = a.numr, j0 = ti.tile * TileShape<NT>::cols;
     const long long np = (long long)nr * nz, nplane = (long long)numr * a.numz;
@@ -139,7 +144,6 @@ __global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
     const double *__restrict__ Rs = a.R + (ti.inst * a.N + ti.slot) * np;
     const bool dirichlet = a.isym == 1;
     const int per = (nz + nwarps - 1) / nwarps, k0 = warp * per, k1 = min(nz, k0 + per);
-    for (int e = threadIdx.x; e < (8 * a.ksteps - nz) * ld; e += blockDim.x) sx[nz * ld + e] = 0.0;
     pdl_wait();
     for (int cc = lane; cc < TileShape<NT>::cols; cc += 32) {
         const int j = j0 + cc;
@@ -179,6 +183,19 @@ __global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
             for (int k = k0; k < k1; ++k) sx[k * ld + cc] = p[(long long)(k + 1) * numr];
         }
     }
+}
+
+// Block: 8 NT columns of a slot; the tile stays in shared memory as the B
+// operand.
+template <int NT>
+__global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
+    extern __shared__ double sx[];
+    constexpr int ld = TileShape<NT>::ld;
+    const TileIndex ti = tile_index(a, a.ntile);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int nr = a.nr, nz = a.nz, j0 = ti.tile * TileShape<NT>::cols;
+    for (int e = threadIdx.x; e < (8 * a.ksteps - nz) * ld; e += blockDim.x) sx[nz * ld + e] = 0.0;
+    source_tile<NT>(a, ti, sx);
     __syncthreads();
     double *Yb = a.Y + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
     const int g = lane >> 2, t = lane & 3;
@@ -248,6 +265,218 @@ __global__ void __launch_bounds__(256) k_modal_inv(ModalArgs a) {
             for (int v = 0; v < 4; ++v)
                 if ((v < 2 ? k0 : k1) && j0 + 8 * n + 2 * t + (v & 1) < nr)
                     p[(v >> 1) * 8 * numr + 8 * n + (v & 1)] = old[n][v] + acc[n][v];
+    }
+}
+
+// ---- split transforms ---------------------------------------------------
+//
+// With a reflecting bottom E[q][k] = 2 / sqrt(L) cos(2 pi (2k+1)(2q+1) / (4L)),
+// L = 2 nz + 1.  The sign of 2k+1 is free, so take a = +-(2k+1) and b =
+// +-(2q+1) congruent to 1 modulo 4; then the entry is +-sin(2 pi beta a b / L)
+// with 4 beta = 1 modulo L: a sine transform of odd functions on Z/L.  Where
+// L = p1 p2 with coprime factors, a = (a1, a2) by remainders (Good 1958,
+// Thomas 1963) and
+//   sin(2 pi beta a b / L) = sin1(a1 b1) cos2(a2 b2) + cos1(a1 b1) sin2(a2 b2),
+// so the matrix product becomes p1 products of size (p2 + 1) / 2:
+//   P(b1, a2) = sum_a1 f(a1, a2) sin1(a1 b1),  Q likewise with cos1,
+//   Y(+-b1, b2) = sum_a2 Q sin2(a2 b2) +- P cos2(a2 b2),
+// a2 and b2 in 0 .. (p2 - 1) / 2, b1 in 0 .. (p1 - 1) / 2.  The sums over a1
+// are a few FMA per zone, in place in the tile; the products stay on the
+// tensor cores (192 heights, 385 = 7 x 55: 56 of 288 fragment products).  The
+// modal array's columns are ordered by (b1, sign, b2), so that both kernels
+// move whole runs of it; the order and the signs of the modes mean nothing to
+// the radial steps.
+__host__ __device__ inline int run_plus(int b1, int h2) { return b1 == 0 ? -1 : (h2 - 1) + (b1 - 1) * (2 * h2 - 1); }
+__host__ __device__ inline int run_minus(int b1, int h2) { return run_plus(b1, h2) + h2 - 1; }
+
+// The sums over a1 of one column and a2, in place: at(a1) is the place of
+// f(a1, a2), sg(a1) its sign (0: no such value).
+template <int P1, class At, class Sg>
+__device__ __forceinline__ void first_factor(const ModalArgs &a, int a2, At at, Sg sg) {
+    constexpr int h = (P1 - 1) / 2;
+    double f[P1], *place[P1];
+#pragma unroll
+    for (int i = 0; i < P1; ++i) {
+        const double w = sg(i);
+        place[i] = at(i);
+        f[i] = w != 0.0 ? w * *place[i] : 0.0;
+    }
+    double P[h + 1], Q[h + 1];
+    Q[0] = f[0];
+#pragma unroll
+    for (int i = 1; i <= h; ++i) Q[0] += f[i] + f[P1 - i];
+#pragma unroll
+    for (int b = 1; b <= h; ++b) {
+        P[b] = 0.0;
+        Q[b] = f[0];
+#pragma unroll
+        for (int i = 1; i <= h; ++i) {
+            P[b] = fma(f[i] - f[P1 - i], a.s1[i][b], P[b]);
+            Q[b] = fma(f[i] + f[P1 - i], a.c1[i][b], Q[b]);
+        }
+    }
+    if (a2 > 0) *place[0] = Q[0];
+#pragma unroll
+    for (int b = 1; b <= h; ++b) {
+        *place[b] = P[b];
+        if (a2 > 0) *place[P1 - b] = Q[b];
+    }
+}
+
+// accP = cos2 P, accQ = sin2 Q for row tile mt; the row of (group, a2) and
+// column n starts at px[...], qx[...] (one offset per lane and step).
+template <int NT, class Row>
+__device__ __forceinline__ void second_factor(const ModalArgs &a, const double *sx, int nstr, int mt, int lane, bool with_p,
+                                              Row row, double (*accP)[4], double (*accQ)[4]) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) accP[n][v] = accQ[n][v] = 0.0;
+    const double2 *cp = reinterpret_cast<const double2 *>(a.Cs + (long long)mt * a.ks2 * 128) + 2 * lane;
+    const double2 *sp = cp + (long long)a.mt2 * a.ks2 * 64;
+    const double *bp = sx + g * nstr;
+    for (int ks = 0; ks < a.ks2; ++ks) {
+        const int r0 = 8 * ks + t, r1 = r0 + 4;
+        {
+            const double2 a01 = __ldg(sp + 64 * ks), a23 = __ldg(sp + 64 * ks + 1);
+            const double *b0 = bp + row(false, r0), *b1 = bp + row(false, r1);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) dmma(accQ[n], a01, a23, b0[8 * n * nstr], b1[8 * n * nstr]);
+        }
+        if (with_p) {
+            const double2 a01 = __ldg(cp + 64 * ks), a23 = __ldg(cp + 64 * ks + 1);
+            const double *b0 = bp + row(true, r0), *b1 = bp + row(true, r1);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) dmma(accP[n], a01, a23, b0[8 * n * nstr], b1[8 * n * nstr]);
+        }
+    }
+}
+
+template <int NT, int P1>
+__global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
+    extern __shared__ double sx[];
+    constexpr int ld = TileShape<NT>::ld, cols = TileShape<NT>::cols, h = (P1 - 1) / 2;
+    const TileIndex ti = tile_index(a, a.ntile);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int nr = a.nr, nz = a.nz, h2 = a.h2, k2 = 8 * a.ks2, j0 = ti.tile * cols;
+    int *tab = reinterpret_cast<int *>(sx + nz * ld);  // [P1][h2]
+    int *rows = tab + P1 * h2;                         // [Q0 .. Qh, P1 .. Ph][k2]: row offsets
+    for (int i = threadIdx.x; i < P1 * h2; i += blockDim.x) tab[i] = a.tab[i];
+    for (int i = threadIdx.x; i < P1 * k2; i += blockDim.x) {
+        // past h2 the matrices are zero, and so is the sine's first column: any row will do there
+        const int grp = i / k2, a2 = min(i % k2, h2 - 1);
+        const int a1 = grp == 0 ? 0 : grp <= h ? P1 - grp : grp - h;
+        const int at = (grp <= h && a2 == 0) ? 1 : a2;
+        rows[i] = (abs(a.tab[a1 * h2 + at]) - 1) * ld;
+    }
+    source_tile<NT>(a, ti, sx);
+    __syncthreads();
+    for (int i = threadIdx.x; i < h2 * cols; i += blockDim.x) {
+        const int c = i % cols, a2 = i / cols;
+        first_factor<P1>(
+            a, a2, [&](int a1) { return sx + max(abs(tab[a1 * h2 + a2]) - 1, 0) * ld + c; },
+            [&](int a1) {
+                const int t = tab[a1 * h2 + a2];
+                return t > 0 ? 1.0 : t < 0 ? -1.0 : 0.0;
+            });
+    }
+    __syncthreads();
+    double *Yb = a.Y + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
+    const int g = lane >> 2, t = lane & 3;
+    for (int u = warp; u < (h + 1) * a.mt2; u += nwarps) {
+        const int b1 = u / a.mt2, mt = u % a.mt2;
+        double accP[NT][4], accQ[NT][4];
+        const int *rq = rows + b1 * k2, *rp = rows + (h + b1) * k2;
+        second_factor<NT>(a, sx, 1, mt, lane, b1 > 0, [&](bool p, int r) { return p ? rp[r] : rq[r]; }, accP, accQ);
+        if (u + nwarps >= (h + 1) * a.mt2) pdl_trigger();
+        const int plus = run_plus(b1, h2), minus = run_minus(b1, h2);
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int j = j0 + 8 * n + 2 * t + (v & 1), b2 = 16 * mt + g + 8 * (v >> 1);
+                if (b2 >= h2 || j >= nr) continue;
+                double *y = Yb + (long long)j * a.ldq + b2;
+                if (b1 > 0 || b2 > 0) y[plus] = accQ[n][v] + accP[n][v];
+                if (b1 > 0 && b2 > 0) y[minus] = accQ[n][v] - accP[n][v];
+            }
+    }
+}
+
+template <int NT, int P1>
+__global__ void __launch_bounds__(256, 2) k_modal_inv_split(ModalArgs a) {
+    extern __shared__ __align__(16) double sx[];
+    constexpr int cols = TileShape<NT>::cols, h = (P1 - 1) / 2;
+    const int ld = inv_ld(a.ksteps);
+    const TileIndex ti = tile_index(a, a.ntile);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int nr = a.nr, nz = a.nz, numr = a.numr, h2 = a.h2, j0 = ti.tile * cols;
+    int *tab = reinterpret_cast<int *>(sx + cols * ld);
+    for (int i = threadIdx.x; i < P1 * h2; i += blockDim.x) tab[i] = a.tab[i];
+    const double *Yb = a.Y + (((long long)ti.row * a.N + ti.slot) * nr + j0) * a.ldq;
+    double *Pg = a.P + (ti.inst * a.N + ti.slot) * (long long)numr * a.numz;
+    pdl_wait();
+    for (int cc = warp; cc < cols; cc += nwarps) {
+        double *row = sx + cc * ld;
+        if (j0 + cc < nr) {
+            for (int q = 2 * lane; q < a.ldq; q += 64) {
+                const unsigned d = (unsigned)__cvta_generic_to_shared(row + q);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(Yb + (long long)cc * a.ldq + q));
+            }
+        } else {
+            for (int q = lane; q < nz; q += 32) row[q] = 0.0;
+        }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int cc = warp; cc < cols; cc += nwarps)
+        for (int a2 = lane; a2 < h2; a2 += 32)
+            first_factor<P1>(
+                a, a2,
+                [&](int a1) {
+                    const int at = a1 == 0 ? a2 - 1 : a1 <= h ? run_plus(a1, h2) + a2 : run_minus(P1 - a1, h2) + a2;
+                    return sx + cc * ld + max(at, 0);
+                },
+                [&](int a1) { return a2 > 0 || (a1 > 0 && a1 <= h) ? 1.0 : 0.0; });
+    __syncthreads();
+    const int g = lane >> 2, t = lane & 3;
+    for (int u = warp; u < (h + 1) * a.mt2; u += nwarps) {
+        const int b1 = u / a.mt2, mt = u % a.mt2;
+        const int plus = run_plus(b1, h2), minus = b1 == 0 ? -1 : run_minus(b1, h2);
+        double accP[NT][4], accQ[NT][4];
+        // past h2 the matrices are zero, and so is the sine's first column: any value will do there
+        second_factor<NT>(a, sx, ld, mt, lane, b1 > 0,
+                          [&](bool p, int r) { return p ? plus + min(r, h2 - 1) : minus + max(min(r, h2 - 1), 1); }, accP,
+                          accQ);
+        if (u + nwarps >= (h + 1) * a.mt2) pdl_trigger();
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            if (side && b1 == 0) break;
+            double old[NT][4];
+            int tr[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int b2 = 16 * mt + g + 8 * r;
+                tr[r] = (b2 < h2 && !(side && b2 == 0)) ? tab[(side ? P1 - b1 : b1) * h2 + b2] : 0;
+            }
+            double *p = Pg + j0 + 2 * t + 1;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    old[n][v] = (a.add && tr[v >> 1] && j0 + 8 * n + 2 * t + (v & 1) < nr)
+                                    ? p[(long long)abs(tr[v >> 1]) * numr + 8 * n + (v & 1)]
+                                    : 0.0;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (tr[v >> 1] && j0 + 8 * n + 2 * t + (v & 1) < nr) {
+                        const double x = side ? accQ[n][v] - accP[n][v] : accQ[n][v] + accP[n][v];
+                        p[(long long)abs(tr[v >> 1]) * numr + 8 * n + (v & 1)] = old[n][v] + (tr[v >> 1] > 0 ? x : -x);
+                    }
+        }
     }
 }
 
@@ -468,7 +697,46 @@ size_t radial_smem(const bph_ctx *c) {
 constexpr int kNT = 4;  // 32 columns per transform tile (64: 161 against 129 us per solve at 130 x 98 x 256)
 size_t fwd_smem(const bph_ctx *c) { return sizeof(double) * (size_t)((c->nz + 7) / 8 * 8) * TileShape<kNT>::ld; }
 size_t inv_smem(const bph_ctx *c) { return sizeof(double) * (size_t)TileShape<kNT>::cols * inv_ld((c->nz + 7) / 8); }
+// Dynamic shared bytes and kernels of the transforms in use.
+size_t fwd_bytes(const bph_ctx *c) {
+    if (!c->modal_p1) return fwd_smem(c);
+    const int h2 = ((2 * c->nz + 1) / c->modal_p1 + 1) / 2, k2 = (h2 + 7) / 8 * 8;
+    return sizeof(double) * (size_t)c->nz * TileShape<kNT>::ld + sizeof(int) * (size_t)c->modal_p1 * (h2 + k2);
+}
+size_t inv_bytes(const bph_ctx *c) {
+    if (!c->modal_p1) return inv_smem(c);
+    const int h2 = ((2 * c->nz + 1) / c->modal_p1 + 1) / 2;
+    return inv_smem(c) + sizeof(int) * (size_t)c->modal_p1 * h2;
+}
+const void *fwd_kernel(const bph_ctx *c) {
+    switch (c->modal_p1) {
+        case 3: return (const void *)k_modal_fwd_split<kNT, 3>;
+        case 5: return (const void *)k_modal_fwd_split<kNT, 5>;
+        case 7: return (const void *)k_modal_fwd_split<kNT, 7>;
+        default: return (const void *)k_modal_fwd<kNT>;
+    }
+}
+const void *inv_kernel(const bph_ctx *c) {
+    switch (c->modal_p1) {
+        case 3: return (const void *)k_modal_inv_split<kNT, 3>;
+        case 5: return (const void *)k_modal_inv_split<kNT, 5>;
+        case 7: return (const void *)k_modal_inv_split<kNT, 7>;
+        default: return (const void *)k_modal_inv<kNT>;
+    }
+}
+
+// Fragment products (16 x 8 x 8, per eight columns) of one transform: dense, or
+// split with first factor p1 (0: p1 does not apply to the height).
+int dense_products(int nz) { return ((nz + 15) / 16) * ((nz + 7) / 8); }
+int split_products(int nz, int isym, int p1) {
+    const int L = 2 * nz + 1, p2 = L / p1;
+    if (isym == 1 || L % p1 || p2 % p1 == 0 || p2 < p1) return 0;
+    const int h2 = (p2 + 1) / 2;
+    return p1 * ((h2 + 15) / 16) * ((h2 + 7) / 8);
+}
+
 int tile_threads(const bph_ctx *c) {
+    if (c->modal_p1) return 256;
     const int mt = (c->nz + 15) / 16;
     const int rounds = (mt + 7) / 8;
     const int w = (mt + rounds - 1) / rounds;
@@ -493,6 +761,21 @@ ModalArgs base_args(const bph_ctx *c) {
     a.mtiles = (c->nz + 15) / 16;
     a.ksteps = (c->nz + 7) / 8;
     a.gamma = c->gamma;
+    if (c->modal_p1) {
+        const int h = (c->modal_p1 - 1) / 2;
+        a.h2 = ((2 * c->nz + 1) / c->modal_p1 + 1) / 2;
+        a.mt2 = (a.h2 + 15) / 16;
+        a.ks2 = (a.h2 + 7) / 8;
+        a.Cs = c->d_modE;
+        a.tab = c->d_modtab;
+        const double w = 2.0 * std::acos(-1.0) / c->modal_p1;
+        for (int i = 0; i <= h; ++i)
+            for (int b = 0; b <= h; ++b) {
+                const int r = (c->modal_beta1 * i * b) % c->modal_p1;
+                a.s1[i][b] = std::sin(w * r);
+                a.c1[i][b] = std::cos(w * r);
+            }
+    }
     return a;
 }
 
@@ -519,6 +802,61 @@ int modal_chunk(const bph_ctx *c, int capacity) {
     const size_t fit = (48ull << 20) / (sizeof(double) * modal_size(c));
     const int most = fit < 1 ? 1 : fit > 64 ? 64 : (int)fit;
     return capacity < most ? capacity : most;
+}
+
+// Tables of the split form: the signed heights of (a1, a2), the packed second
+// factors (wave: 2 / sqrt(L) cos over a period of 4 L), and the eigenvalues in
+// the modal array's order.
+static void split_tables(bph_ctx *c, const std::vector<double> &wave, std::vector<double> &pack, std::vector<int> &tab,
+                         std::vector<double> &lam) {
+    const int nz = c->nz, L = 2 * nz + 1, p1 = c->modal_p1, p2 = L / p1, h = (p1 - 1) / 2, h2 = (p2 + 1) / 2;
+    const int alpha = (L % 4 == 1) ? 1 : 3;  // alpha L = 1 modulo 4
+    const int beta = (int)(((1LL - (long long)alpha * L) / 4 % L + L) % L);
+    auto inverse = [](int v, int m) {
+        for (int x = 1; x < m; ++x)
+            if ((long long)v % m * x % m == 1) return x;
+        return 0;
+    };
+    c->modal_beta1 = (int)((long long)beta * inverse(p2, p1) % p1);
+    const int beta2 = (int)((long long)beta * inverse(p1, p2) % p2);
+    tab.assign((size_t)p1 * h2, 0);
+    for (int k = 0; k < nz; ++k) {
+        const int u = 2 * k + 1, a = (u % 4 == 1) ? u : L - u % L;
+        int x1 = a % p1, x2 = a % p2, sg = 1;
+        if (x2 >= h2 || (x2 == 0 && x1 > h)) {
+            x1 = (p1 - x1) % p1;
+            x2 = (p2 - x2) % p2;
+            sg = -1;
+        }
+        tab[(size_t)x1 * h2 + x2] = sg * (k + 1);
+    }
+    // cos(2 pi r / p2) sits at 4 p1 r of the period 4 L, the sine a quarter period (L) on
+    const double sign = (alpha == 1) ? -1.0 : 1.0;
+    auto entry = [&](int b2, int a2, bool sine) -> double {
+        if (b2 >= h2 || a2 >= h2) return 0.0;
+        const long long r = (long long)beta2 * a2 % p2 * b2 % p2;
+        return sign * wave[(size_t)((4LL * p1 * r + (sine ? 3LL * L : 0)) % (4LL * L))];
+    };
+    const int mt2 = (h2 + 15) / 16, ks2 = (h2 + 7) / 8;
+    const size_t frag = (size_t)mt2 * ks2 * 128;
+    pack.assign(2 * frag, 0.0);
+    for (int m = 0; m < mt2; ++m)
+        for (int k = 0; k < ks2; ++k)
+            for (int l = 0; l < 32; ++l)
+                for (int v = 0; v < 4; ++v) {
+                    const int row = 16 * m + l / 4 + 8 * (v & 1), col = 8 * k + l % 4 + 4 * (v >> 1);
+                    const size_t at = ((size_t)m * ks2 + k) * 128 + 4 * l + v;
+                    pack[at] = entry(row, col, false);
+                    pack[frag + at] = entry(row, col, true);
+                }
+    std::vector<double> by_q(lam);
+    for (int b1 = 0; b1 <= h; ++b1)
+        for (int b2 = 0; b2 < h2; ++b2) {
+            const int p = tab[(size_t)b1 * h2 + b2];
+            if (p) lam[(size_t)(run_plus(b1, h2) + b2)] = by_q[(size_t)(std::abs(p) - 1)];
+            if (b1 > 0 && b2 > 0)
+                lam[(size_t)(run_minus(b1, h2) + b2)] = by_q[(size_t)(std::abs(tab[(size_t)(p1 - b1) * h2 + b2]) - 1)];
+        }
 }
 
 // Decides whether the grid runs the modal form and prepares it.  Lines of up
@@ -554,9 +892,23 @@ int modal_configure(bph_ctx *c) {
         const long long i = dirichlet ? (long long)(q + 1) * (k + 1) : (2LL * q + 1) * (2LL * k + 1);
         return wave[(size_t)(i % period)];
     };
+    // the split form where it leaves at most two thirds of the products (192 heights: 56 of 288)
+    c->modal_p1 = 0;
+    int least = 2 * dense_products(nz) / 3;
+    const char *ps = std::getenv("BPH_MODAL_SPLIT");
+    for (int p1 : {3, 5, 7}) {
+        const int n = (ps && ps[0] == '0') ? 0 : split_products(nz, c->g.isym, p1);
+        if (n > 0 && n <= least) {
+            least = n;
+            c->modal_p1 = p1;
+        }
+    }
     const size_t frag = (size_t)mt * ks * 128;
     std::vector<double> pack(2 * frag);
-    for (int m = 0; m < mt; ++m)
+    std::vector<int> tab;
+    if (c->modal_p1) split_tables(c, wave, pack, tab, lam);
+    else
+      for (int m = 0; m < mt; ++m)
         for (int k = 0; k < ks; ++k)
             for (int l = 0; l < 32; ++l) {
                 const int g = l / 4, t = l % 4;
@@ -569,7 +921,8 @@ int modal_configure(bph_ctx *c) {
             }
     // one allocation: both fragment arrays, the eigenvalues, the norm partials, one instance's modal array
     const size_t norms = 2 * (size_t)c->N * modal_groups(c), lams = ((size_t)nz + 1) / 2 * 2;
-    const size_t all = pack.size() + lams + norms + modal_size(c);
+    const size_t tabs = (tab.size() + 3) / 4 * 2;  // doubles that hold the index table
+    const size_t all = pack.size() + lams + norms + tabs + modal_size(c);
     if (cudaMalloc((void **)&c->d_modE, sizeof(double) * all) != cudaSuccess) {
         cudaGetLastError();  // no room: the half-step kernels need none of it
         c->d_modE = nullptr;
@@ -577,13 +930,16 @@ int modal_configure(bph_ctx *c) {
     }
     c->d_modlam = c->d_modE + pack.size();
     c->d_modnorm = c->d_modlam + lams;
-    c->d_modY = c->d_modnorm + norms;
+    c->d_modtab = reinterpret_cast<int *>(c->d_modnorm + norms);
+    c->d_modY = c->d_modnorm + norms + tabs;
     c->bytes += sizeof(double) * all;
     pack.insert(pack.end(), lam.begin(), lam.end());
     BPH_CUDA(cudaMemcpyAsync(c->d_modE, pack.data(), sizeof(double) * pack.size(), cudaMemcpyHostToDevice, c->stream));
-    BPH_CUDA(cudaStreamSynchronize(c->stream));  // pack is this call's own
-    BPH_CUDA(raise_smem_limit((const void *)k_modal_fwd<kNT>, (int)fwd_smem(c)));
-    BPH_CUDA(raise_smem_limit((const void *)k_modal_inv<kNT>, (int)inv_smem(c)));
+    if (!tab.empty())
+        BPH_CUDA(cudaMemcpyAsync(c->d_modtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, c->stream));
+    BPH_CUDA(cudaStreamSynchronize(c->stream));  // pack and tab are this call's own
+    BPH_CUDA(raise_smem_limit(fwd_kernel(c), (int)fwd_bytes(c)));
+    BPH_CUDA(raise_smem_limit(inv_kernel(c), (int)inv_bytes(c)));
     BPH_CUDA(raise_smem_limit(radial_kernel<false>(c), (int)radial_smem(c)));
     BPH_CUDA(raise_smem_limit(radial_kernel<true>(c), (int)radial_smem(c)));
     c->modal = 1;
@@ -653,12 +1009,12 @@ cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, co
         a.inst0 = r0;
         a.E = c->d_modE;
         a.source = cold ? kColdResidual : kResidual;
-        cudaError_t e = launch(c, (const void *)k_modal_fwd<kNT>, blocks * a.ntile, threads, fwd_smem(c), a, st, pdl);
+        cudaError_t e = launch(c, fwd_kernel(c), blocks * a.ntile, threads, fwd_bytes(c), a, st, pdl);
         if (e == cudaSuccess)
             e = launch(c, radial_kernel<false>(c), blocks * a.groups, kLines * radial_nseg(c), radial_smem(c), a, st, pdl);
         a.E = c->d_modE + (size_t)a.mtiles * a.ksteps * 128;
         a.add = cold ? 0 : 1;
-        if (e == cudaSuccess) e = launch(c, (const void *)k_modal_inv<kNT>, blocks * a.ntile, threads, inv_smem(c), a, st, pdl);
+        if (e == cudaSuccess) e = launch(c, inv_kernel(c), blocks * a.ntile, threads, inv_bytes(c), a, st, pdl);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -679,12 +1035,12 @@ cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R
     a.E = c->d_modE;
     a.source = cold ? kColdResidual : kResidual;
     const long long blocks = (long long)ninst * c->N * a.ntile;
-    cudaError_t e = launch(c, (const void *)k_modal_fwd<kNT>, blocks, tile_threads(c), fwd_smem(c), a, c->stream, c->pdl);
+    cudaError_t e = launch(c, fwd_kernel(c), blocks, tile_threads(c), fwd_bytes(c), a, c->stream, c->pdl);
     if (e != cudaSuccess) return e;
     if (cold) return cudaMemsetAsync(phi, 0, sizeof(double) * (size_t)ninst * modal_size(c), c->stream);
     a.Y = phi;
     a.source = kPotential;
-    return launch(c, (const void *)k_modal_fwd<kNT>, blocks, tile_threads(c), fwd_smem(c), a, c->stream, c->pdl);
+    return launch(c, fwd_kernel(c), blocks, tile_threads(c), fwd_bytes(c), a, c->stream, c->pdl);
 }
 
 cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double *phi, double *pre, int ninst,
@@ -708,7 +1064,7 @@ cudaError_t launch_modal_end(bph_ctx *c, double *P, double *pre, int ninst, cons
     a.Y = pre;
     a.inst_map = inst_map;
     a.E = c->d_modE + (size_t)a.mtiles * a.ksteps * 128;
-    return launch(c, (const void *)k_modal_inv<kNT>, (long long)ninst * c->N * a.ntile, tile_threads(c), inv_smem(c), a,
+    return launch(c, inv_kernel(c), (long long)ninst * c->N * a.ntile, tile_threads(c), inv_bytes(c), a,
                   c->stream, c->pdl);
 }
 

@@ -22,6 +22,11 @@ GRIDS = [
     (258, 20, 16, 2, 5),   # the longest line
     (259, 12, 16, 2, 5),   # past it: half-step kernels
     (20, 146, 16, 3, 3),   # heights past 128
+    (20, 12, 16, 2, 4),    # split transforms: 21 = 3 x 7, second factor below one fragment
+    (37, 24, 16, 3, 3),    # 45 = 5 x 9, factors not prime
+    (34, 54, 32, 2, 6),    # 105 = 7 x 15 (and 3 x 35, 5 x 21)
+    (21, 118, 16, 2, 4),   # 233: prime, dense
+    (70, 194, 16, 2, 5),   # 385 = 7 x 55, the production height
 ]
 
 
