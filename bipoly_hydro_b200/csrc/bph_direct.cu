@@ -91,6 +91,55 @@ __device__ __forceinline__ void tc_transform(const float *A, int lda, float *Xt,
     const int cp = nrp / 16;
     for (int cp0 = 0; cp0 < cp; cp0 += cpb) {
         const int ncp = min(cpb, cp - cp0), tiles = (nzp / 32) * ncp;
+        // Rows in units of 48 and an even number of column pairs: one 48 x 32 tile per warp, which
+        // splits 20 operand values for 36 products where three 32 x 16 tiles split 36.
+        const int half = ncp / 2;
+        if (nzp % 48 == 0 && ncp % 2 == 0 && (nzp / 48) * half <= kWarpsD) {
+            float acc[3][4][4];
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) acc[m][n][v] = 0.f;
+            const bool on = warp < (nzp / 48) * half;
+            const int i0 = on ? 48 * (warp / half) : 0, c0 = 16 * cp0 + 32 * (warp % half);
+            if (on) {
+                for (int k0 = 0; k0 < nzp; k0 += 8) {
+                    uint32_t bh[4][2], bl[4][2];
+#pragma unroll
+                    for (int n = 0; n < 4; ++n)
+#pragma unroll
+                        for (int v = 0; v < 2; ++v)
+                            split_tf32(Xt[direct::b_offset(c0, n, k0, g, t, ldk, v)], bh[n][v], bl[n][v]);
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) {
+                        uint32_t ah[4], al[4];
+#pragma unroll
+                        for (int v = 0; v < 4; ++v)
+                            split_tf32(A[direct::a_offset(i0, m, k0, g, t, lda, v)], ah[v], al[v]);
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) mma_tf32(acc[m][n], al, bh[n][0], bh[n][1]);
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) mma_tf32(acc[m][n], ah, bl[n][0], bl[n][1]);
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) mma_tf32(acc[m][n], ah, bh[n][0], bh[n][1]);
+                    }
+                }
+            }
+            __syncthreads();  // every product of this block has read its columns
+            if (on) {
+#pragma unroll
+                for (int m = 0; m < 3; ++m)
+#pragma unroll
+                    for (int n = 0; n < 4; ++n)
+#pragma unroll
+                        for (int v = 0; v < 4; ++v)
+                            Xt[direct::d_offset(i0, m, c0, n, g, t, ldk, v)] = acc[m][n][v];
+            }
+            __syncthreads();
+            continue;
+        }
         float acc[kTilesPerWarp][2][2][4];
 #pragma unroll
         for (int r = 0; r < kTilesPerWarp; ++r) {
