@@ -196,7 +196,7 @@ cudaError_t contract_batch_launch(bph_ctx *c, bph_batch *b, long long mstride) {
 //     d0 (group, 2t), d1 (group, 2t + 1), d2 (group + 8, 2t), d3 (group + 8, 2t + 1)
 constexpr int kDmmaWarps = 8;
 constexpr int kDmmaStages = 4;  // 8-zone steps per staged chunk
-constexpr int kDmmaPipe = 3;    // chunks in flight (cp.async stages)
+constexpr int kDmmaPipe = 2;    // chunk buffers (cp.async stages); two CTAs per SM cover each other's waits
 
 constexpr int kDmmaMaxTiles = 8;  // column tiles of 8 per launch (64 columns)
 
@@ -218,7 +218,7 @@ struct DmmaSmem {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(kDmmaWarps * 32, 1)
+__global__ void __launch_bounds__(kDmmaWarps * 32, 2)
 k_contract_dmma(const double *__restrict__ G, const double *__restrict__ mom, long long mstride, long long np, int nb,
                 int c0, int ncol, double *__restrict__ C, long long cstride, unsigned int *__restrict__ counters,
                 double *__restrict__ partials) {
@@ -393,7 +393,7 @@ cudaError_t contract_dmma_launch_nt(bph_ctx *c, bph_batch *b, long long mstride,
     return cudaLaunchKernelExC(&cfg, (const void *)k_contract_dmma<NT>, args);
 }
 
-// Slices of the zone range (one CTA per SM): the count, up to kBatchSplitMax
+// Slices of the zone range (two CTAs per SM): the count, up to kBatchSplitMax
 // with at least 64 steps of 8 zones per slice and at least two waves, whose
 // last wave is the fullest.
 int dmma_splits(const bph_ctx *c) {
@@ -407,8 +407,8 @@ int dmma_splits(const bph_ctx *c) {
     for (int ns = 1; ns <= kBatchSplitMax; ++ns) {
         if (ns > 1 && nk / ns < 64) break;
         const long long ctas = base * ns;
-        const long long waves = (ctas + sms - 1) / sms;
-        const double eff = (double)ctas / (double)(waves * sms) + (waves >= 2 ? 0.25 : 0.0);
+        const long long waves = (ctas + 2 * sms - 1) / (2 * sms);
+        const double eff = (double)ctas / (double)(waves * 2 * sms) + (waves >= 2 ? 0.25 : 0.0);
         if (eff > best_eff + 1e-9) {
             best_eff = eff;
             best = ns;
