@@ -141,21 +141,65 @@ void dt_schedule(const HostCoef &h, int numr, int nsteps, double *dt) {
 }
 
 void free_schedule(bph_ctx *c, Schedule &s) {
-    dev_free(s.d_dt);
-    dev_free(s.d_rad);
-    dev_free(s.d_ver);
-    for (int k = 0; k < 2; ++k) {
-        dev_free(s.d_rad_pk[k]);
-        dev_free(s.d_ver_pk[k]);
-    }
-    dev_free(s.d_warp_rad);
-    dev_free(s.d_warp_ver);
-    dev_free(s.d_warp_rad32);
-    dev_free(s.d_warp_ver32);
-    dev_free(s.d_mod_rad);
+    dev_free(s.arena);
     free(s.h_dt);
     s = Schedule();
     (void)c;
+}
+
+// The schedule's arrays in one allocation (eleven separate ones cost a small
+// grid's set-up a third of its time); modal: with the modal form's.
+int schedule_arena(bph_ctx *c, Schedule &s, int nsteps, bool modal) {
+    size_t total = 0;
+    auto room = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t n = (size_t)nsteps, nN = n * c->N;
+    const size_t dt = room(sizeof(double) * n), rad = room(sizeof(double) * nN * kAdiFactors * c->nr),
+                 ver = room(sizeof(double) * n * kAdiFactors * c->nz);
+    const size_t r64 = room(sizeof(double) * nN * packed_block<double>(c->nr)),
+                 v64 = room(sizeof(double) * n * packed_block<double>(c->nz)),
+                 r32 = room(sizeof(float) * nN * packed_block<float>(c->nr)),
+                 v32 = room(sizeof(float) * n * packed_block<float>(c->nz));
+    size_t wr = 0, wv = 0, wr32 = 0, wv32 = 0, mr = 0, mc = 0;
+    if (c->adi_warp) {
+        wr = room(sizeof(double) * nN * warp_block_doubles(c->nr));
+        wv = room(sizeof(double) * n * warp_block_doubles(c->nz));
+        if (c->mixed_warp) {
+            wr32 = room(sizeof(float) * nN * warp_block_doubles(c->nr));
+            wv32 = room(sizeof(float) * n * warp_block_doubles(c->nz));
+        }
+    }
+    if (modal) {
+        mr = room(sizeof(double) * nN * modal_radial_doubles(c));
+        mc = room(sizeof(double2) * n * c->nz);
+    }
+    char *p = nullptr;
+    const int rc = dev_alloc(c, &p, total);
+    if (rc) return rc;
+    s.arena = p;
+    s.d_dt = reinterpret_cast<double *>(p + dt);
+    s.d_rad = reinterpret_cast<double *>(p + rad);
+    s.d_ver = reinterpret_cast<double *>(p + ver);
+    s.d_rad_pk[0] = p + r64;
+    s.d_ver_pk[0] = p + v64;
+    s.d_rad_pk[1] = p + r32;
+    s.d_ver_pk[1] = p + v32;
+    if (c->adi_warp) {
+        s.d_warp_rad = reinterpret_cast<double *>(p + wr);
+        s.d_warp_ver = reinterpret_cast<double *>(p + wv);
+        if (c->mixed_warp) {
+            s.d_warp_rad32 = reinterpret_cast<float *>(p + wr32);
+            s.d_warp_ver32 = reinterpret_cast<float *>(p + wv32);
+        }
+    }
+    if (modal) {
+        s.d_mod_rad = reinterpret_cast<double *>(p + mr);
+        s.d_mod_cs = reinterpret_cast<double2 *>(p + mc);
+    }
+    return BPH_OK;
 }
 
 // Builds (or returns the cached) schedule for nsteps ADI steps.
@@ -171,37 +215,20 @@ int get_schedule(bph_ctx *c, int nsteps, Schedule **out) {
     host_coefficients(c, h);
     s.h_dt = (double *)malloc(sizeof(double) * nsteps);
     dt_schedule(h, c->g.numr, nsteps, s.h_dt);
-    int rc;
-    if ((rc = dev_alloc(c, &s.d_dt, nsteps))) return rc;
-    if ((rc = dev_alloc(c, &s.d_rad, (size_t)nsteps * c->N * kAdiFactors * c->nr))) return rc;
-    if ((rc = dev_alloc(c, &s.d_ver, (size_t)nsteps * kAdiFactors * c->nz))) return rc;
+    int rc = schedule_arena(c, s, nsteps, c->modal != 0);
+    // without room for the modal form's arrays the schedule runs the half-step form
+    if (rc == BPH_ERR_NOMEM && c->modal) rc = schedule_arena(c, s, nsteps, false);
+    if (rc) {
+        free_schedule(c, s);
+        return rc;
+    }
     BPH_CUDA(cudaMemcpyAsync(s.d_dt, s.h_dt, sizeof(double) * nsteps, cudaMemcpyHostToDevice, c->stream));
     s.nsteps = nsteps;
     static long long next_build_id = 1;
     s.build_id = next_build_id++;
     BPH_CUDA(launch_adi_factors(c, s));
-    {
-        double *r64, *v64;
-        float *r32, *v32;
-        if ((rc = dev_alloc(c, &r64, (size_t)nsteps * c->N * packed_block<double>(c->nr)))) return rc;
-        s.d_rad_pk[0] = r64;
-        if ((rc = dev_alloc(c, &v64, (size_t)nsteps * packed_block<double>(c->nz)))) return rc;
-        s.d_ver_pk[0] = v64;
-        if ((rc = dev_alloc(c, &r32, (size_t)nsteps * c->N * packed_block<float>(c->nr)))) return rc;
-        s.d_rad_pk[1] = r32;
-        if ((rc = dev_alloc(c, &v32, (size_t)nsteps * packed_block<float>(c->nz)))) return rc;
-        s.d_ver_pk[1] = v32;
-    }
     BPH_CUDA(launch_pack_factors(c, s));
-    if (c->adi_warp) {
-        if ((rc = dev_alloc(c, &s.d_warp_rad, (size_t)nsteps * c->N * warp_block_doubles(c->nr)))) return rc;
-        if ((rc = dev_alloc(c, &s.d_warp_ver, (size_t)nsteps * warp_block_doubles(c->nz)))) return rc;
-        if (c->mixed_warp) {
-            if ((rc = dev_alloc(c, &s.d_warp_rad32, (size_t)nsteps * c->N * warp_block_doubles(c->nr)))) return rc;
-            if ((rc = dev_alloc(c, &s.d_warp_ver32, (size_t)nsteps * warp_block_doubles(c->nz)))) return rc;
-        }
-        BPH_CUDA(launch_pack_warp(c, s));
-    }
+    if (c->adi_warp) BPH_CUDA(launch_pack_warp(c, s));
     BPH_CUDA(modal_pack(c, s));
     BPH_CUDA(cudaStreamSynchronize(c->stream));
     *out = &s;

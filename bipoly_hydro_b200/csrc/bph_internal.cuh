@@ -69,6 +69,7 @@ __host__ __device__ inline int packed_block(int n) {
 
 struct Schedule {
     int nsteps = 0;
+    void *arena = nullptr;    // the one allocation that holds every device array below
     double *d_dt = nullptr;   // [nsteps]
     double *d_rad = nullptr;  // [nsteps][N][kAdiFactors][nr] radial Thomas factors
     double *d_ver = nullptr;  // [nsteps][kAdiFactors][nz]    vertical Thomas factors
@@ -421,6 +422,7 @@ void modal_free(bph_ctx *c);
 int modal_groups(const bph_ctx *c);
 size_t modal_size(const bph_ctx *c);  // doubles of one instance's modal array
 int modal_chunk(const bph_ctx *c, int capacity);  // instances per pass of a batch's launch_modal
+size_t modal_radial_doubles(const bph_ctx *c);  // of one (step, slot) radial factor block
 cudaError_t modal_pack(bph_ctx *c, Schedule &s);
 bool modal_ready(const bph_ctx *c, const Schedule &s);
 // Whether converged cycles of schedule s run there (mixed: in place of the

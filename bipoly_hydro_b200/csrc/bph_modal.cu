@@ -952,19 +952,11 @@ void modal_free(bph_ctx *c) {
     c->modal = 0;
 }
 
-// A schedule's radial blocks and step coefficients (after launch_adi_factors);
-// without room for them the schedule runs the half-step form.
+size_t modal_radial_doubles(const bph_ctx *c) { return (size_t)radial_block(radial_rows(c)); }
+
+// A schedule's radial blocks and step coefficients (after launch_adi_factors).
 cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
-    if (!c->modal) return cudaSuccess;
-    const size_t rad = (size_t)s.nsteps * c->N * radial_block(radial_rows(c));
-    const size_t cs = (size_t)s.nsteps * c->nz;
-    if (cudaMalloc((void **)&s.d_mod_rad, sizeof(double) * rad + sizeof(double2) * cs) != cudaSuccess) {
-        cudaGetLastError();
-        s.d_mod_rad = nullptr;
-        return cudaSuccess;
-    }
-    s.d_mod_cs = reinterpret_cast<double2 *>(s.d_mod_rad + rad);  // rad is even
-    c->bytes += sizeof(double) * rad + sizeof(double2) * cs;
+    if (!s.d_mod_rad) return cudaSuccess;
     c->launches += 2;
     const int nseg = radial_rows(c) / c->modal_seg;
     k_pack_modal<<<(unsigned)(s.nsteps * c->N), nseg, 0, c->stream>>>(s.d_rad, s.d_mod_rad, c->nr, nseg, c->modal_seg);
