@@ -1425,9 +1425,9 @@ cudaError_t launch_adi_slots(bph_ctx *c, const Schedule &sch, bool cold, const i
     return cudaLaunchKernelExC(&cfg, seg_kernel<double, false>(c->adi_seg, c->adi_full, c->adi_pf), args);
 }
 
-cudaError_t launch_adi_defect(bph_ctx *c, const Schedule &sch) {
+cudaError_t launch_adi_defect(bph_ctx *c, const Schedule &sch, const int *skip) {
     if (!c->adi_mixed_smem) return cudaErrorNotSupported;
-    if (c->mixed_kind == BPH_MIXED_DIRECT) return launch_defect_direct(c, c->d_P, c->d_R, 1, nullptr, c->d_red);
+    if (c->mixed_kind == BPH_MIXED_DIRECT) return launch_defect_direct(c, c->d_P, c->d_R, 1, nullptr, c->d_red, skip);
     AdiArgs a = make_args(c, sch, 0, sch.nsteps, false);
     a.norms = c->d_red;
     a.rad_pk = sch.d_rad_pk[1];  // float blocks for the FP32 kernels

@@ -19,6 +19,10 @@ namespace bph {
 namespace {
 
 constexpr int kCheckThreads = 256;
+// Cycles per pass of the while node's body where a cycle can be skipped: an
+// iteration of the node costs more than the two launches of a skipped cycle,
+// and most solves take three or four cycles.
+constexpr int kBodyCycles = 4;
 
 __global__ void k_conv_init(ConvState *st, double tol, int max_cycles, int mixed) {
     st->tol = tol;
@@ -27,13 +31,18 @@ __global__ void k_conv_init(ConvState *st, double tol, int max_cycles, int mixed
     st->max_cycles = max_cycles;
     st->cycles = 0;
     st->mixed = mixed;
+    st->done = 0;
 }
 
 // red[2 i] = sum over slot i of |update|^2, red[2 i + 1] = |phi|^2 (Parseval
 // weights included).  Fixed-order reduction (deterministic).
 __global__ void __launch_bounds__(kCheckThreads) k_conv_check(const double *__restrict__ red, int N, ConvState *st,
-                                                              cudaGraphConditionalHandle cond) {
+                                                              cudaGraphConditionalHandle cond, bool last) {
     __shared__ double sn[kCheckThreads], sd[kCheckThreads];
+    if (st->done) {
+        if (last && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
+        return;
+    }
     double num = 0.0, den = 0.0;
     for (int i = threadIdx.x; i < N; i += kCheckThreads) {
         num += red[2 * i];
@@ -60,7 +69,8 @@ __global__ void __launch_bounds__(kCheckThreads) k_conv_check(const double *__re
         st->cycles = cyc;
         st->upd = upd;
         st->prev = upd;
-        cudaGraphSetConditional(cond, stop ? 0u : 1u);
+        st->done = stop ? 1 : 0;
+        if (last) cudaGraphSetConditional(cond, stop ? 0u : 1u);
     }
 }
 
@@ -96,24 +106,30 @@ static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t
         c->stream = cs;
         c->pdl = false;  // plain serial edges inside the loop body
         cudaError_t ce = cudaSuccess;
-        if (modal) {
-            ce = launch_modal_cycle(c, s, c->d_modY, c->d_prev, mixed ? nullptr : c->d_modpre, 1, c->d_modnorm);
-        } else if (mixed) {
-            ce = launch_adi_defect(c, s);
-        } else if (c->adi_seg) {  // the update norms come from the sweep's write-back
-            ce = launch_adi(c, s, 0, s.nsteps, false, nullptr, nullptr, 1, nullptr, c->d_red);
-        } else {
-            ce = cudaMemcpyAsync(c->d_prev, c->d_P, sizeof(double) * (size_t)c->N * c->nplane,
-                                 cudaMemcpyDeviceToDevice, cs);
-            if (ce == cudaSuccess) ce = launch_adi(c, s, 0, s.nsteps, false);
-            if (ce == cudaSuccess) ce = launch_update_norm(c, c->d_red);
+        const bool skips = modal || (mixed && c->mixed_kind == BPH_MIXED_DIRECT);
+        const int reps = skips ? kBodyCycles : 1;
+        for (int r = 0; r < reps && ce == cudaSuccess; ++r) {
+            const int *skip = skips && r > 0 ? &c->d_conv->done : nullptr;
+            if (modal) {
+                ce = launch_modal_cycle(c, s, c->d_modY, c->d_prev, mixed ? nullptr : c->d_modpre, 1, c->d_modnorm, skip);
+            } else if (mixed) {
+                ce = launch_adi_defect(c, s, skip);
+            } else if (c->adi_seg) {  // the update norms come from the sweep's write-back
+                ce = launch_adi(c, s, 0, s.nsteps, false, nullptr, nullptr, 1, nullptr, c->d_red);
+            } else {
+                ce = cudaMemcpyAsync(c->d_prev, c->d_P, sizeof(double) * (size_t)c->N * c->nplane,
+                                     cudaMemcpyDeviceToDevice, cs);
+                if (ce == cudaSuccess) ce = launch_adi(c, s, 0, s.nsteps, false);
+                if (ce == cudaSuccess) ce = launch_update_norm(c, c->d_red);
+            }
+            if (ce == cudaSuccess) {
+                k_conv_check<<<1, kCheckThreads, 0, cs>>>(modal ? c->d_modnorm : c->d_red,
+                                                          modal ? c->N * modal_groups(c) : c->N, c->d_conv, cond,
+                                                          r + 1 == reps);
+                ce = cudaGetLastError();
+            }
+            ++c->launches;
         }
-        if (ce == cudaSuccess) {
-            k_conv_check<<<1, kCheckThreads, 0, cs>>>(modal ? c->d_modnorm : c->d_red,
-                                                      modal ? c->N * modal_groups(c) : c->N, c->d_conv, cond);
-            ce = cudaGetLastError();
-        }
-        ++c->launches;
         c->stream = keep;
         c->pdl = keep_pdl;
         cudaGraph_t body = nullptr;

@@ -44,6 +44,7 @@ struct DirectArgs {
     const double *sig;         // [nz] vertical shifts gamma lambda_q (FP64)
     const double *brb;         // [N][numr] radial diagonal
     const double *alphar, *betar, *bzb;
+    const int *skip;  // not 0: nothing to do (nullptr: always run)
     double *norms;             // per (instance, slot) |delta|^2, |phi|^2
     const int *inst_map;       // instance of each block row (nullptr: row)
     int N, numr, numz, nr, nz, nrp, nzp, ldk, lda, cpb, isym;  // cpb: column pairs per transform block
@@ -217,6 +218,7 @@ __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_all;
 __global__ void __launch_bounds__(kDThreads, 2) k_defect_direct(DirectArgs a) {
     extern __shared__ __align__(16) float dsm[];
     __shared__ double red[2][kWarpsD];
+    if (a.skip && *a.skip) return;
     const int nzp = a.nzp, ldk = a.ldk, nr = a.nr, nz = a.nz, numr = a.numr;
     float *Xt = dsm;                                              // [nrp][ldk]: r, E r, y, delta
     double *bd = reinterpret_cast<double *>(dsm + a.off_bd);      // radial diagonal of the slot
@@ -418,7 +420,7 @@ int direct_configure(bph_ctx *c) {
 }
 
 cudaError_t launch_defect_direct(bph_ctx *c, double *P, const double *R, int nrows, const int *inst_map,
-                                 double *norms) {
+                                 double *norms, const int *skip) {
     if (!c->mixed_smem_kind[BPH_MIXED_DIRECT] || !c->d_dir32 || !c->d_dirS || !norms) return cudaErrorNotSupported;
     const direct::Shape d = direct::shape(c->nr, c->nz);
     const size_t ne = (size_t)d.nzp * d.lda;
@@ -433,6 +435,7 @@ cudaError_t launch_defect_direct(bph_ctx *c, double *P, const double *R, int nro
     a.betar = c->d_betar;
     a.bzb = c->d_bzb;
     a.norms = norms;
+    a.skip = skip;
     a.inst_map = inst_map;
     a.N = c->N;
     a.numr = c->g.numr;

@@ -95,6 +95,7 @@ struct Schedule {
 struct ConvState {
     double tol, prev, upd;
     int max_cycles, cycles, mixed;
+    int done;  // the loop has stopped: the body's remaining cycles return at once
 };
 
 // Instantiated while-graph of a converged form and what it captured.
@@ -303,7 +304,8 @@ cudaError_t launch_adi_plain(bph_ctx *c, const Schedule &s, int step0, int nstep
 // (pdl: with programmatic dependent launch on that stream).
 cudaError_t launch_adi_slots(bph_ctx *c, const Schedule &s, bool cold, const int *d_slots, int nslots,
                              cudaStream_t st, bool pdl);
-cudaError_t launch_adi_defect(bph_ctx *c, const Schedule &s);
+// skip (direct kind): the cycle returns at once when *skip is not 0.
+cudaError_t launch_adi_defect(bph_ctx *c, const Schedule &s, const int *skip = nullptr);
 // Slots too large for shared memory (bph_adi_large.cu): the drop-in ADI on
 // the slot array P with source R, and one FP32 refinement cycle (work area
 // c->d_work32: r, delta and two [N][np] buffers).
@@ -378,7 +380,7 @@ int compact_configure(bph_ctx *c);
 // one launch with no scratch in global memory.
 int direct_configure(bph_ctx *c);
 cudaError_t launch_defect_direct(bph_ctx *c, double *P, const double *R, int nrows, const int *inst_map,
-                                 double *norms);
+                                 double *norms, const int *skip = nullptr);
 cudaError_t launch_green_compact(bph_ctx *c);
 // Warp-cooperative FP64 ADI (bph_adi_warp.cu).  warp_configure selects it
 // for the grids it covers (c->adi_warp != 0) and packs the per-slot
@@ -415,7 +417,7 @@ int fft_configure(bph_ctx *c);
 // schedule on ninst instances (row r: instance inst_map[r], slots
 // slot_map[0..nslots) of each), chunk instances per pass in Y.  Converged form: begin (modal residual in Y,
 // modal potential in phi, ninst times modal_size each), cycles (partial norms
-// [ninst][N][modal_groups][2]), end (a potential back into P: pre, the
+// [ninst][N][modal_groups][2]; with *skip not 0 a cycle returns at once), end (a potential back into P: pre, the
 // caller running that step with launch_adi_plain, or phi).
 int modal_configure(bph_ctx *c);
 void modal_free(bph_ctx *c);
@@ -433,7 +435,7 @@ cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, co
 cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R, double *Y, double *phi, int ninst,
                                const int *inst_map);
 cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double *phi, double *pre, int ninst,
-                               double *norms);
+                               double *norms, const int *skip = nullptr);
 cudaError_t launch_modal_end(bph_ctx *c, double *P, double *pre, int ninst, const int *inst_map);
 // Context references (bph_api.cu): a batch takes one at creation and gives
 // it back at its destruction; the last release frees the device state.

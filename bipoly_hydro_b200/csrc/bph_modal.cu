@@ -55,6 +55,7 @@ struct ModalArgs {
     const double2 *cs;       // [nsteps][nz] (2 dt / (dt + lambda), (dt - lambda) / (dt + lambda))
     const double *dt;        // [nsteps]
     double *norms;           // converged form: [row][N][groups][2]
+    const int *skip;         // converged form: not 0: nothing to do (nullptr: always run)
     int inst0, nslots, ntile, groups;
     int numr, numz, nr, nz, ldq, N, isym, mtiles, ksteps;
     int nsteps, source, add;
@@ -543,6 +544,7 @@ __global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_mod
     const int nseg = blockDim.x >> 5;
     double *ends = sm + 2 * block;             // [NSEG][32] forward ends
     double *starts = ends + NSEG * kLines;     // [NSEG][32] backward starts
+    if (kCycle && a.skip && *a.skip) return;
     const TileIndex ti = tile_index(a, a.groups);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int nr = a.nr, nz = a.nz;
@@ -1036,7 +1038,7 @@ cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R
 }
 
 cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double *phi, double *pre, int ninst,
-                               double *norms) {
+                               double *norms, const int *skip) {
     ModalArgs a = base_args(c);
     a.Y = Y;
     a.phi = phi;
@@ -1046,6 +1048,7 @@ cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double 
     a.dt = s.d_dt;
     a.nsteps = s.nsteps;
     a.norms = norms;
+    a.skip = skip;
     return launch(c, radial_kernel<true>(c), (long long)ninst * c->N * a.groups, kLines * radial_nseg(c), radial_smem(c), a,
                   c->stream, c->pdl);
 }
