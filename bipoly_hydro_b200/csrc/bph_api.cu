@@ -1,11 +1,11 @@
 // bph_api.cu -- the C ABI (include/bph.h): context setup (potsetup.F90),
 // the solve driver (potential_solver.F90) and its host/device entry points.
 //
-// One solve is five kernels on the context's stream:
+// One solve is four stages on the context's stream:
 //   k_fft_fwd<rho>     rho -> R = -4 pi rho_hat (slot-major) + moments
-//   k_green_contract   moments x Green tables -> S
-//   k_boundary_slots   S -> Dirichlet slots of P (top, side, bottom)
-//   k_adi              nsteps ADI steps per slot on P
+//   k_green_compact    moments x Green tables -> S and the Dirichlet slots of P (top, side, bottom)
+//   ADI                nsteps ADI steps per slot on P: one kernel of half-steps (bph_adi_warp.cu) or
+//                      the three of the vertical eigenbasis (bph_modal.cu)
 //   k_fft_inv          P -> pot, with the axis and equator conditions
 // A warm start reuses the Fourier-space potential P of the previous solve,
 // which is what the reference's forward transform of its kept potp gives
@@ -520,7 +520,6 @@ int setup_impl(bph_ctx *c) {
     if ((rc = adi_configure(c))) return rc;
     if ((rc = warp_configure(c))) return rc;
     if ((rc = direct_configure(c))) return rc;
-    if ((rc = modal_configure(c))) return rc;
     if ((rc = contract_configure(c))) return rc;
     if ((rc = noalloc_setup(c))) return rc;
     {
@@ -547,6 +546,7 @@ int setup_impl(bph_ctx *c) {
         if ((rc = dev_alloc(c, &c->d_W, (size_t)c->N * c->nplane))) return rc;
         if ((rc = dev_alloc(c, &c->d_W2, (size_t)c->N * c->np))) return rc;
     }
+    if ((rc = modal_configure(c))) return rc;  // after every allocation the context cannot do without
     Schedule *s;
     if ((rc = get_schedule(c, 5, &s))) return rc;
     if ((rc = get_schedule(c, 20, &s))) return rc;

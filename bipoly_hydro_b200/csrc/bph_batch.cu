@@ -182,10 +182,11 @@ cudaError_t contract_batch_launch(bph_ctx *c, bph_batch *b, long long mstride) {
 // mma.sync m16n8k8 .f64), the batched boundary contraction for every batch
 // size.  Warp w of a CTA owns a 16-row tile of boundary rows b and all
 // 8 NT columns c of the launch's column block; the CTA's 8 warps share one
-// (mode, slice of zones).  Per 8-zone step a warp streams its 16 x 8 table
-// tile (four 8-byte evict-first loads per thread, prefetched kDmmaStages
-// steps ahead so that ~64 KB of table bytes per SM are in flight) and reads
-// the moment fragments (L1: every warp of the CTA reads the same ones).
+// (mode, slice of zones).  The CTA copies chunks of 32 zones, its 128 table
+// rows (evict-first) and the moment columns, into one of two shared-memory
+// buffers by cp.async while it multiplies the other; two CTAs per SM cover
+// each other's chunk barriers (130 x 98 x 256, n = 16: 1783 -> 1740 us per
+// call against one CTA with three buffers).
 // Slices write partial sums; the last CTA of each (mode, row group) to
 // arrive adds them in slice order (deterministic) and writes C.
 //   A (16 x 8, row major) = G[m][b0 + r][k0 + q]      (table rows)
@@ -550,7 +551,6 @@ int bph_batch_create(bph_ctx_t *c, int capacity, bph_batch_t **out) {
     int rc = BPH_OK;
     if (!rc) rc = batch_alloc(b, &b->d_P, (size_t)capacity * c->N * c->nplane);
     if (!rc) rc = batch_alloc(b, &b->d_R, (size_t)capacity * c->N * c->np);
-    if (!rc && c->modal) (void)batch_alloc(b, &b->d_mody, (size_t)modal_chunk(c, capacity) * modal_size(c));
     if (!rc) rc = batch_alloc(b, &b->d_mom, (size_t)c->g.mmax * capacity * 2 * c->np);
     if (!rc) rc = batch_alloc(b, &b->d_C, (size_t)c->g.mmax * 2 * capacity * c->nb);
     if (!rc && large) rc = batch_alloc(b, &b->d_LW, (size_t)capacity * c->N * c->np);
@@ -593,6 +593,8 @@ int bph_batch_create(bph_ctx_t *c, int capacity, bph_batch_t **out) {
             rc = BPH_ERR_NOMEM;
         }
     }
+    // last and optional: without room for it the batch runs the half-step form
+    if (!rc && c->modal) (void)batch_alloc(b, &b->d_mody, (size_t)modal_chunk(c, capacity) * modal_size(c));
     if (!rc) {
         e = cudaMemsetAsync(b->d_P, 0, sizeof(double) * (size_t)capacity * c->N * c->nplane, c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mom, 0, sizeof(double) * (size_t)c->g.mmax * capacity * 2 * c->np,
@@ -841,6 +843,21 @@ int batch_enqueue(bph_batch *b, int n, const double *const *d_in, double *const 
     return BPH_OK;
 }
 
+// At least need doubles of FP32 work array.
+static int batch_work32(bph_batch *b, size_t need) {
+    if (need <= b->work32_doubles) return BPH_OK;
+    if (b->d_work32) {
+        cudaStreamSynchronize(b->c->stream);
+        cudaFree(b->d_work32);
+        b->bytes -= sizeof(double) * b->work32_doubles;
+        b->d_work32 = nullptr;
+        b->work32_doubles = 0;
+    }
+    const int rc = batch_alloc(b, &b->d_work32, need);
+    if (!rc) b->work32_doubles = need;
+    return rc;
+}
+
 int batch_reserve_converged(bph_batch *b, bool mixed) {
     bph_ctx *c = b->c;
     int rc;
@@ -851,15 +868,25 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
     const bool want_modal = c->modal && (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
     if (want_modal && !b->d_mnorm) {
         const size_t norms = 2ull * b->cap * c->N * modal_groups(c);
-        if ((b->d_prev || !batch_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)) &&
-            (b->d_mod || !batch_alloc(b, &b->d_mod, (size_t)b->cap * modal_size(c))) &&
-            (b->d_modpre || !batch_alloc(b, &b->d_modpre, (size_t)b->cap * modal_size(c))) &&
+        const size_t each = (size_t)b->cap * modal_size(c);
+        const bool had_prev = b->d_prev != nullptr;
+        if ((had_prev || !batch_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)) &&
+            !batch_alloc(b, &b->d_mod, each) && !batch_alloc(b, &b->d_modpre, each) &&
             cudaMallocHost((void **)&b->h_mnorm, sizeof(double) * norms) == cudaSuccess)
             (void)batch_alloc(b, &b->d_mnorm, norms);
-        if (!b->d_mnorm) {
+        if (!b->d_mnorm) {  // give back what was had: the other forms need the room
             cudaGetLastError();
             if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
             b->h_mnorm = nullptr;
+            auto give_back = [&](double *&p, size_t count) {
+                if (!p) return;
+                cudaFree(p);
+                b->bytes -= sizeof(double) * count;
+                p = nullptr;
+            };
+            give_back(b->d_mod, each);
+            give_back(b->d_modpre, each);
+            if (!had_prev) give_back(b->d_prev, (size_t)b->cap * c->N * c->nplane);
         }
     }
     // FP64 on the grid-wide kernels: the previous cycle's slot arrays (the segmented kernel
@@ -873,18 +900,7 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
     if (mixed && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && !(b->d_mnorm && !c->adi_warp)) need = 2ull * b->cap * c->N * c->np;
     if (mixed && c->mixed_kind == BPH_MIXED_ADI_WARP)
         need = ((size_t)b->cap * c->N * c->np + 1) / 2;
-    if (need > b->work32_doubles) {
-        if (b->d_work32) {
-            cudaStreamSynchronize(c->stream);
-            cudaFree(b->d_work32);
-            b->bytes -= sizeof(double) * b->work32_doubles;
-            b->d_work32 = nullptr;
-            b->work32_doubles = 0;
-        }
-        if ((rc = batch_alloc(b, &b->d_work32, need))) return rc;
-        b->work32_doubles = need;
-    }
-    return BPH_OK;
+    return batch_work32(b, need);
 }
 
 // Sums the per-slot norm pairs of instance i: sqrt(sum |a|^2 / sum |b|^2).
@@ -920,6 +936,9 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
             BPH_CUDA(cudaMemsetAsync(b->d_P + (size_t)inst[i] * c->N * c->nplane, 0, ibytes, c->stream));
     if ((rc = batch_prologue(b, n, d_in, d_map, per_pos))) return rc;
     const bool modal = modal_converged(c, *s, cv.mixed) && b->d_mnorm;
+    if (cv.mixed && !modal && c->mixed_kind == BPH_MIXED_ADI_GLOBAL &&
+        (rc = batch_work32(b, 2ull * b->cap * c->N * c->np)))
+        return rc;
     const int mpairs = modal ? c->N * modal_groups(c) : 0;  // norm pairs per position
     if (modal) BPH_CUDA(launch_modal_begin(c, cv.cold, b->d_P, b->d_R, b->d_mod, b->d_prev, n, d_map));
     std::vector<double> prev_upd((size_t)n, INFINITY);

@@ -726,7 +726,8 @@ cudaError_t launch_green_compact_contract(bph_ctx *c, bool write_slots, bool sha
     // Mode by mode the compute of the side rows runs under the tiles' loads, which many waves
     // (258 x 194: 340 against 363 us) and a solve that shares the SMs with the free slots' ADI
     // (130 x 98 x 256: 165 against 172 us) want.
-    a.tiles_first = !shared && compact::items(d, c->g.mmax) < 4 * 444;
+    constexpr int kWave = 148 * 3;  // resident CTAs
+    a.tiles_first = !shared && compact::items(d, c->g.mmax) < 4 * kWave;
     a.part_h = compact::part_height_doubles(d);
     ++c->launches;
     cudaLaunchAttribute attr[1];
