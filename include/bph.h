@@ -307,7 +307,7 @@ int bph_copy_moments(bph_ctx_t *ctx, double *host_out, size_t n);
 #define BPH_PHASE_FFT_RHO 0   /* k_fft_fwd: rho -> -4 pi rho_hat + moments */
 #define BPH_PHASE_CONTRACT 1  /* k_green_contract: tables x moments -> S and the Dirichlet slots */
 #define BPH_PHASE_SLOTS 2     /* k_boundary_slots: S -> Dirichlet slots (standalone form; solves write them in the contraction) */
-#define BPH_PHASE_ADI 3       /* k_adi: nsteps warm ADI steps */
+#define BPH_PHASE_ADI 3       /* nsteps warm ADI steps of every slot, in the form the grid and nsteps run */
 #define BPH_PHASE_FFT_INV 4   /* k_fft_inv: slots -> pot */
 
 /* Enqueues exactly one phase of a solve on the context's stream (device
@@ -349,13 +349,14 @@ int bph_green_contract_noalloc(bph_ctx_t *ctx, const double *d_mom, double *d_S)
 #define BPH_INFO_MIXED_FORWARD_NS 7   /* setup-time duration of a 10-step forwarding-form launch, ns (0: not timed) */
 #define BPH_INFO_MIXED_INCREMENT_NS 8 /* the same for the increment form */
 #define BPH_INFO_ADI_PREFETCH 9       /* bulk-copy factor prefetch: bit 0 FP64 ADI, bit 1 FP32 refinement ADI */
-#define BPH_INFO_ADI_KERNEL 10        /* FP64 drop-in ADI kernel in use (BPH_ADI_KERNEL_*) */
+#define BPH_INFO_ADI_KERNEL 10        /* FP64 half-step ADI kernel of the grid (BPH_ADI_KERNEL_*); schedules that run in
+                                         the vertical eigenbasis do not use it */
 #define BPH_INFO_ADI_WARP_SMEM 11     /* dynamic shared bytes of the warp-cooperative kernel (0: not used) */
 #define BPH_INFO_MIXED_WARP_NS 12     /* setup-time duration of a 10-step warp-cooperative refinement launch, ns */
 #define BPH_INFO_GREEN_SMS 13         /* SMs of the contraction's partition in the overlapped solve (0: not requested,
                                          negative: the set-up step that failed) */
 #define BPH_INFO_CONTRACT_KIND 14     /* boundary contraction of the single solve (BPH_CONTRACT_*) */
-#define BPH_INFO_FFT_DENSE 15         /* 1: FFT tiles compiled for eight CTAs per SM (autotuned, or BPH_FFT_DENSE) */
+#define BPH_INFO_FFT_DENSE 15         /* 1: single FFTs with the dense register budget, 768 threads per SM (autotuned, or BPH_FFT_DENSE) */
 #define BPH_INFO_CONTRACT_FULL_NS 16  /* set-up autotune: one full-table contraction, ns (0: not timed) */
 #define BPH_INFO_CONTRACT_COMPACT_NS 17 /* the same for the compact contraction */
 #define BPH_INFO_FFT_NS 18            /* set-up autotune: forward + inverse FFT with regular tiles, ns */
@@ -385,7 +386,10 @@ long long bph_info(const bph_ctx_t *ctx, int what);
  *                            residual r - A delta (more instructions, smaller
  *                            shared-memory footprint).
  *   BPH_MIXED_ADI_GLOBAL     the same cycle with the slot's arrays in global
- *                            memory, for grids whose slots exceed shared memory.
+ *                            memory, for grids whose slots exceed shared memory;
+ *                            where the FP64 cycle in the vertical eigenbasis
+ *                            applies it runs instead (it is the faster one),
+ *                            with the mixed form's stopping rule.
  * All converge to the same discrete solution.  Returns BPH_ERR_INVALID for
  * an on-chip kind that does not fit this grid. */
 #define BPH_CFG_MIXED_ADI 0
