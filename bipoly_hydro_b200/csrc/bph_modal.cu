@@ -78,6 +78,8 @@ __device__ __forceinline__ void dmma(double *c, const double2 &a01, const double
         : "d"(a01.x), "d"(a01.y), "d"(a23.x), "d"(a23.y), "d"(b0), "d"(b1));
 }
 
+constexpr unsigned kAhead = 2 * 148;  // resident blocks of the split transforms and of short radial lines
+
 // Rows of 8 NT columns, padded to 4 modulo the 16 eight-byte banks: the four
 // rows of a B fragment then fall into different banks.
 template <int NT>
@@ -90,10 +92,10 @@ struct TileIndex {
     int tile, slot, row;
     long long inst;
 };
-__device__ __forceinline__ TileIndex tile_index(const ModalArgs &a, int per_slot) {
+__device__ __forceinline__ TileIndex tile_index(const ModalArgs &a, int per_slot, unsigned block) {
     TileIndex t;
-    t.tile = blockIdx.x % per_slot;
-    const int b = blockIdx.x / per_slot;
+    t.tile = block % per_slot;
+    const int b = block / per_slot;
     const int local = b % a.nslots;
     t.row = b / a.nslots;
     t.slot = a.slot_map ? a.slot_map[local] : local;
@@ -192,7 +194,7 @@ template <int NT>
 __global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
     extern __shared__ double sx[];
     constexpr int ld = TileShape<NT>::ld;
-    const TileIndex ti = tile_index(a, a.ntile);
+    const TileIndex ti = tile_index(a, a.ntile, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, j0 = ti.tile * TileShape<NT>::cols;
     for (int e = threadIdx.x; e < (8 * a.ksteps - nz) * ld; e += blockDim.x) sx[nz * ld + e] = 0.0;
@@ -223,7 +225,7 @@ template <int NT>
 __global__ void __launch_bounds__(256) k_modal_inv(ModalArgs a) {
     extern __shared__ __align__(16) double sx[];
     const int ld = inv_ld(a.ksteps);
-    const TileIndex ti = tile_index(a, a.ntile);
+    const TileIndex ti = tile_index(a, a.ntile, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, numr = a.numr, j0 = ti.tile * TileShape<NT>::cols;
     const long long nplane = (long long)numr * a.numz;
@@ -354,11 +356,24 @@ __device__ __forceinline__ void second_factor(const ModalArgs &a, const double *
     }
 }
 
+// Asks L2 for rows of count doubles, stride apart: what the block that takes
+// this one's place will load.  With one or two blocks per SM nothing else
+// covers the HBM latency at a block's start (five steps at 258 x 194 x 512:
+// 660 -> 655 us by the transforms' sources, -> 634 with the radial lines; the
+// inverse's own old potential, asked for under its products, cost 4 us).
+__device__ __forceinline__ void prefetch_rows(const double *p, long long stride, int rows, int count) {
+    const int lines = (count + 14) / 16 + 1;  // 128-byte lines that an unaligned row can touch
+    for (int i = threadIdx.x; i < rows * lines; i += blockDim.x) {
+        const double *at = p + (i / lines) * stride + min(16 * (i % lines), count - 1);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+    }
+}
+
 template <int NT, int P1>
 __global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
     extern __shared__ double sx[];
     constexpr int ld = TileShape<NT>::ld, cols = TileShape<NT>::cols, h = (P1 - 1) / 2;
-    const TileIndex ti = tile_index(a, a.ntile);
+    const TileIndex ti = tile_index(a, a.ntile, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, h2 = a.h2, k2 = 8 * a.ks2, j0 = ti.tile * cols;
     int *tab = reinterpret_cast<int *>(sx + nz * ld);  // [P1][h2]
@@ -372,6 +387,14 @@ __global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
         rows[i] = (abs(a.tab[a1 * h2 + at]) - 1) * ld;
     }
     source_tile<NT>(a, ti, sx);
+    if (blockIdx.x + kAhead < gridDim.x) {
+        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + kAhead);
+        const int jn = tn.tile * cols, count = min(cols, nr - jn);
+        const long long at = tn.inst * a.N + tn.slot;
+        if (a.source != kPotential) prefetch_rows(a.R + at * nr * nz + jn, nr, nz, count);
+        if (a.source != kColdResidual)
+            prefetch_rows(a.P + at * a.numr * a.numz + a.numr + jn + 1, a.numr, nz, count);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < h2 * cols; i += blockDim.x) {
         const int c = i % cols, a2 = i / cols;
@@ -410,7 +433,7 @@ __global__ void __launch_bounds__(256, 2) k_modal_inv_split(ModalArgs a) {
     extern __shared__ __align__(16) double sx[];
     constexpr int cols = TileShape<NT>::cols, h = (P1 - 1) / 2;
     const int ld = inv_ld(a.ksteps);
-    const TileIndex ti = tile_index(a, a.ntile);
+    const TileIndex ti = tile_index(a, a.ntile, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, numr = a.numr, h2 = a.h2, j0 = ti.tile * cols;
     int *tab = reinterpret_cast<int *>(sx + cols * ld);
@@ -428,6 +451,11 @@ __global__ void __launch_bounds__(256, 2) k_modal_inv_split(ModalArgs a) {
         } else {
             for (int q = lane; q < nz; q += 32) row[q] = 0.0;
         }
+    }
+    if (blockIdx.x + kAhead < gridDim.x) {
+        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + kAhead);
+        const int jn = tn.tile * cols;
+        prefetch_rows(a.Y + (((long long)tn.row * a.N + tn.slot) * nr + jn) * a.ldq, a.ldq, min(cols, nr - jn), a.ldq);
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -529,7 +557,9 @@ __global__ void k_modal_coef(const double *__restrict__ dt, const double *__rest
 // a radius are one broadcast word for the warp and the modal array is read
 // and written in whole rows; eight lanes per line with shuffle scans instead
 // spent 250 shared-memory cycles per 512 zones and step (66 us for five steps
-// at 130 x 98 x 256).  A step's factors arrive one step ahead by cp.async.
+// at 130 x 98 x 256).  A step's factors arrive one step ahead by cp.async
+// (with the step's line coefficients beside them: 1183 -> 1209 us for 20 steps
+// at 258 x 194 x 512, the extra registers spill).
 // kCycle (converged form): Y keeps the residual for the next cycle, the
 // potential's modal coefficients advance in phi, pre takes those before the
 // cycle's last step (the solve ends with that step in half-step form), and the
@@ -545,7 +575,7 @@ __global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_mod
     double *ends = sm + 2 * block;             // [NSEG][32] forward ends
     double *starts = ends + NSEG * kLines;     // [NSEG][32] backward starts
     if (kCycle && a.skip && *a.skip) return;
-    const TileIndex ti = tile_index(a, a.groups);
+    const TileIndex ti = tile_index(a, a.groups, blockIdx.x);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int nr = a.nr, nz = a.nz;
     const double *frad = a.rad + (long long)ti.slot * block;
@@ -571,6 +601,16 @@ __global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_mod
     for (int e = 0; e < SEG; ++e) {
         r[e] = (e < count && mine) ? Yq[(long long)e * a.ldq] : 0.0;
         acc[e] = 0.0;
+    }
+    constexpr unsigned ahead = ROWS == 256 ? kAhead / 2 : kAhead;
+    if (blockIdx.x + ahead < gridDim.x) {
+        const TileIndex tn = tile_index(a, a.groups, blockIdx.x + ahead);
+        const int qn = tn.tile * kLines;
+        prefetch_rows(a.Y + ((long long)tn.row * a.N + tn.slot) * nr * a.ldq + qn, a.ldq, nr, min(kLines, nz - qn));
+    }
+    if (kCycle) {  // needed after the steps
+        const int q0 = ti.tile * kLines;
+        prefetch_rows(a.phi + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq + q0, a.ldq, nr, min(kLines, nz - q0));
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
