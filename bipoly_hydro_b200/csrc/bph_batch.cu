@@ -1074,8 +1074,8 @@ struct bph_plan {
     cudaEvent_t fork = nullptr;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};  // cold, warm
     std::vector<long long> build_id[2];            // schedules captured, per kind and part
-    std::vector<long long> launches_part;          // kernel launches of each part per replay
-    int launches = 0;
+    std::vector<long long> launches_part[2];       // kernel launches of each part per replay, per kind (the forms differ)
+    int last = 0;                                  // kind of the last launch
 };
 
 namespace bph {
@@ -1140,10 +1140,7 @@ static int plan_record(bph_plan *pl, bool warm) {
     pl->exec[k] = exec;
     pl->build_id[k].clear();
     for (Schedule *x : sch) pl->build_id[k].push_back(x->build_id);
-    pl->launches_part = counted;
-    long long tot = 0;
-    for (long long v : counted) tot += v;
-    pl->launches = (int)tot;
+    pl->launches_part[k] = counted;
     return BPH_OK;
 }
 
@@ -1252,7 +1249,8 @@ int bph_plan_launch(bph_plan_t *pl, int tstep, void *stream) {
     int rc;
     if (stale && (rc = plan_record(pl, warm))) return rc;
     BPH_CUDA(cudaGraphLaunch(pl->exec[k], (cudaStream_t)stream));
-    for (size_t p = 0; p < pl->parts.size(); ++p) pl->parts[p]->c->launches += pl->launches_part[p];
+    pl->last = k;
+    for (size_t p = 0; p < pl->parts.size(); ++p) pl->parts[p]->c->launches += pl->launches_part[k][p];
     return BPH_OK;
 }
 
@@ -1271,6 +1269,11 @@ int bph_plan_synchronize(bph_plan_t *pl, void *stream) {
     return worst;
 }
 
-int bph_plan_launches(const bph_plan_t *pl) { return pl ? pl->launches : 0; }
+int bph_plan_launches(const bph_plan_t *pl) {
+    long long total = 0;
+    if (pl)
+        for (long long v : pl->launches_part[pl->last]) total += v;
+    return (int)total;
+}
 
 }  // extern "C"

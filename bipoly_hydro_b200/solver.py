@@ -579,7 +579,7 @@ class Plan:
 
     @property
     def launches(self) -> int:
-        """Kernel launches in one replay."""
+        """Kernel launches in one replay of the kind launched last (0 before the first launch)."""
         return int(self._lib.bph_plan_launches(self._h))
 
     def close(self) -> None:

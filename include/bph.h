@@ -202,7 +202,8 @@ int bph_plan_create(int nparts, bph_batch_t *const *batches, const int *counts, 
 int bph_plan_launch(bph_plan_t *plan, int tstep, void *stream);
 /* Waits for the launches on `stream` and reports non-finite densities. */
 int bph_plan_synchronize(bph_plan_t *plan, void *stream);
-/* Kernel launches one replay makes (both kinds record the same count). */
+/* Kernel launches one replay of the kind launched last makes (cold and warm
+ * solves may run different forms of the ADI); 0 before the first launch. */
 int bph_plan_launches(const bph_plan_t *plan);
 int bph_plan_destroy(bph_plan_t *plan);
 
