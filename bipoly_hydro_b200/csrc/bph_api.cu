@@ -963,7 +963,7 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
             BPH_CUDA(cudaStreamSynchronize(c->stream));
             upd = host_ratio(h, pairs);
             bool stop = upd <= tol || cyc >= max_cycles;
-            if (mixed) stop = stop || !(upd == upd) || upd > 0.5 * prev_upd;
+            if (mixed) stop = stop || !(upd == upd) || upd > 0.5 * prev_upd || (modal && upd <= kLeastUpdate);
             if (stop) break;
             prev_upd = upd;
         }

@@ -991,7 +991,7 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
             // also flagged per position by the forward transform)
             bool stop = upd <= cv.tol || !(upd == upd);
             if (!(upd == upd) && cv.mixed) diverged = true;
-            if (cv.mixed) stop = stop || upd > 0.5 * prev_upd[(size_t)i];
+            if (cv.mixed) stop = stop || upd > 0.5 * prev_upd[(size_t)i] || (modal && upd <= kLeastUpdate);
             prev_upd[(size_t)i] = upd;
             done[(size_t)i] = stop;
             all = all && stop;

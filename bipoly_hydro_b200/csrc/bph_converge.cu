@@ -24,13 +24,14 @@ constexpr int kCheckThreads = 256;
 // and most solves take three or four cycles.
 constexpr int kBodyCycles = 4;
 
-__global__ void k_conv_init(ConvState *st, double tol, int max_cycles, int mixed) {
+__global__ void k_conv_init(ConvState *st, double tol, int max_cycles, int mixed, double least) {
     st->tol = tol;
     st->prev = INFINITY;
     st->upd = INFINITY;
     st->max_cycles = max_cycles;
     st->cycles = 0;
     st->mixed = mixed;
+    st->least = least;
     st->done = 0;
 }
 
@@ -63,9 +64,10 @@ __global__ void __launch_bounds__(kCheckThreads) k_conv_check(const double *__re
         const int cyc = st->cycles + 1;
         // Stop at the tolerance or the cycle limit; the mixed form also when a
         // cycle no longer halves the update (its FP32 solves are then at
-        // their accuracy) or the update is not finite.
+        // their accuracy; FP64 cycles: at the least update) or the update is
+        // not finite.
         bool stop = (upd <= st->tol) || (cyc >= st->max_cycles);
-        if (st->mixed) stop = stop || !(upd == upd) || (upd > 0.5 * st->prev);
+        if (st->mixed) stop = stop || !(upd == upd) || (upd > 0.5 * st->prev) || upd <= st->least;
         st->cycles = cyc;
         st->upd = upd;
         st->prev = upd;
@@ -169,7 +171,7 @@ int conv_loop_device(bph_ctx *c, Schedule &s, bool mixed, double tol, int max_cy
         cg.kind = kind;
     }
     ++c->launches;
-    k_conv_init<<<1, 1, 0, c->stream>>>(c->d_conv, tol, max_cycles, mixed ? 1 : 0);
+    k_conv_init<<<1, 1, 0, c->stream>>>(c->d_conv, tol, max_cycles, mixed ? 1 : 0, modal ? kLeastUpdate : 0.0);
     BPH_CUDA(cudaGetLastError());
     BPH_CUDA(cudaGraphLaunch(cg.exec, c->stream));
     return BPH_OK;

@@ -94,9 +94,16 @@ struct Schedule {
 // Converged-loop state on the device (bph_converge.cu).
 struct ConvState {
     double tol, prev, upd;
+    double least;  // mixed: a relative update of this or less ends the loop
     int max_cycles, cycles, mixed;
     int done;  // the loop has stopped: the body's remaining cycles return at once
 };
+
+// The mixed form's refinement stops once a cycle no longer halves the update:
+// FP32 cycles stagnate where they have reached their accuracy.  Cycles in the
+// vertical eigenbasis are FP64 and do not; they stop at the rounding of the
+// potential they update.
+constexpr double kLeastUpdate = 2.220446049250313e-16;
 
 // Instantiated while-graph of a converged form and what it captured.
 struct ConvGraph {

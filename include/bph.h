@@ -390,7 +390,9 @@ long long bph_info(const bph_ctx_t *ctx, int what);
  *                            memory, for grids whose slots exceed shared memory;
  *                            where the FP64 cycle in the vertical eigenbasis
  *                            applies it runs instead (it is the faster one),
- *                            with the mixed form's stopping rule.
+ *                            with the mixed form's stopping rule; it also
+ *                            stops at an update of 2^-52, the rounding of the
+ *                            potential, where FP32 cycles stagnate.
  * All converge to the same discrete solution.  Returns BPH_ERR_INVALID for
  * an on-chip kind that does not fit this grid. */
 #define BPH_CFG_MIXED_ADI 0

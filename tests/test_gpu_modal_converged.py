@@ -1,0 +1,45 @@
+"""Converged solves whose cycles run in the vertical eigenbasis: the stopping rule goes by the
+change of the potential itself, as in the half-step forms, so no solve goes on for a tolerance
+below the potential's rounding."""
+import numpy as np
+import pytest
+
+from bipoly_hydro_b200.solver import MIXED_ADI_GLOBAL
+from tests.helpers import rel_l2, smooth_density
+
+pytestmark = pytest.mark.gpu
+
+# dense and split transforms, segments of 8 and 16 radii, one and several line groups, every symmetry
+GRIDS = [(40, 30, 64, 2, 16), (67, 34, 32, 1, 6), (50, 19, 32, 3, 6), (35, 21, 64, 2, 12), (131, 74, 16, 2, 5)]
+IDS = ["x".join(map(str, g[:3])) + f"-isym{g[3]}" for g in GRIDS]
+
+
+@pytest.mark.parametrize("graph", ["1", "0"], ids=["device-loop", "host-loop"])
+@pytest.mark.parametrize("grid", GRIDS, ids=IDS)
+def test_update_ends_at_rounding(bph, monkeypatch, grid, graph):
+    """Tolerance zero, 100 cycles allowed.  FP64: the loop ends once a cycle leaves the potential
+    as it is.  Mixed: at its rounding, at most two cycles after the FP32 refinement on the same
+    half-steps ends (which stagnates there; a cycle reduces the error several times)."""
+    monkeypatch.setenv("BPH_CONV_GRAPH", graph)
+    g = (grid[0], grid[1], grid[2], 1.0 / (grid[0] - 4), grid[3], grid[4])
+    rhos = [np.asfortranarray(smooth_density(*g[:5], seed=40 + i)) for i in range(2)]
+    cycles = {}
+    for form in ("modal", "half"):
+        if form == "half":
+            monkeypatch.setenv("BPH_ADI_MODAL", "0")
+        s = bph.PotentialSolver(*g)
+        b = bph.Batch(s, capacity=2)
+        ref, _ = s.solve_converged(rhos[0], 10, True, 1e-13, 60)
+        if form == "modal":
+            pot, one = s.solve_converged(rhos[0], 10, True, 0.0, 100)
+            pots, many = b.solve_converged(rhos, 10, True, 0.0, 100)
+            assert one.cycles < 100 and many.cycles < 100
+            assert rel_l2(pot, ref) <= 1e-12 and rel_l2(pots[0], ref) <= 1e-12
+        s.set_mixed_adi(MIXED_ADI_GLOBAL)
+        pot, one = s.solve_converged_mixed(rhos[0], 10, True, 0.0, 100)
+        pots, many = b.solve_converged(rhos, 10, True, 0.0, 100, mixed=True)
+        assert rel_l2(pot, ref) <= 1e-12 and rel_l2(pots[0], ref) <= 1e-12
+        cycles[form] = one.cycles, many.cycles
+        b.close()
+        s.close()
+    assert cycles["modal"][0] <= cycles["half"][0] + 2 and cycles["modal"][1] <= cycles["half"][1] + 2
