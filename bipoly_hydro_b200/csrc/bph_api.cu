@@ -163,7 +163,7 @@ int schedule_arena(bph_ctx *c, Schedule &s, int nsteps, bool modal) {
                  v64 = room(sizeof(double) * n * packed_block<double>(c->nz)),
                  r32 = room(sizeof(float) * nN * packed_block<float>(c->nr)),
                  v32 = room(sizeof(float) * n * packed_block<float>(c->nz));
-    size_t wr = 0, wv = 0, wr32 = 0, wv32 = 0, mr = 0, mc = 0;
+    size_t wr = 0, wv = 0, wr32 = 0, wv32 = 0, mr = 0, mc = 0, md = 0;
     if (c->adi_warp) {
         wr = room(sizeof(double) * nN * warp_block_doubles(c->nr));
         wv = room(sizeof(double) * n * warp_block_doubles(c->nz));
@@ -174,7 +174,8 @@ int schedule_arena(bph_ctx *c, Schedule &s, int nsteps, bool modal) {
     }
     if (modal) {
         mr = room(sizeof(double) * nN * modal_radial_doubles(c));
-        mc = room(sizeof(double2) * n * c->nz);
+        mc = room(sizeof(double2) * (2 * n + 1) * c->nz);
+        md = room(sizeof(double) * (2 * n + 1));
     }
     char *p = nullptr;
     const int rc = dev_alloc(c, &p, total);
@@ -198,6 +199,7 @@ int schedule_arena(bph_ctx *c, Schedule &s, int nsteps, bool modal) {
     if (modal) {
         s.d_mod_rad = reinterpret_cast<double *>(p + mr);
         s.d_mod_cs = reinterpret_cast<double2 *>(p + mc);
+        s.d_mod_dt2 = reinterpret_cast<double *>(p + md);
     }
     return BPH_OK;
 }

@@ -85,10 +85,12 @@ struct Schedule {
     double *d_warp_ver = nullptr;
     float *d_warp_rad32 = nullptr;  // the same blocks in float (warp-cooperative refinement kernel)
     float *d_warp_ver32 = nullptr;
-    // modal ADI (bph_modal.cu): radial factor blocks [nsteps][N][block] and step
-    // coefficients [nsteps][nz] (nullptr: the schedule runs the half-step form)
+    // modal ADI (bph_modal.cu): radial factor blocks [nsteps][N][block], step
+    // coefficients [nsteps, then nsteps + 1 for the refinement's order][nz] and
+    // sums of dt [2 nsteps + 1] (nullptr: the schedule runs the half-step form)
     double *d_mod_rad = nullptr;
     double2 *d_mod_cs = nullptr;
+    double *d_mod_dt2 = nullptr;
 };
 
 // Converged-loop state on the device (bph_converge.cu).

@@ -21,6 +21,16 @@
 // Rounding differs from the half-step form (no 1/(dt + lambda) amplification
 // of the radially stiff components); the iteration is the same one.
 //
+// The mixed form's refinement takes the half-steps in another order: a radial
+// one at the first dt, then (vertical, radial) per step, so that a cycle ends
+// on the radial solve, which the radially stiff components of the residual
+// need (ended on the vertical one, its residual was 2e-10 for 1e-13 at
+// 66 x 66 x 64).  Paired radial first, its n + 1 radial solves (dt a) and n
+// vertical ones (dt b) are the step above with two dt:
+//   phi += (a + b) / (b + lambda_q) delta,
+//   r     = (a - lambda_q) / (b + lambda_q) ((a + b) delta - r),
+// and the last solve alone phi += delta, r = (a - lambda_q) delta.
+//
 // The transforms are the matrix products of the path (2 nz FMA per zone each)
 // and run on the FP64 tensor cores, mma.sync m16n8k8.f64: 37 TFLOP/s
 // measured for the instruction alone against 33 for FMA.
@@ -53,12 +63,13 @@ struct ModalArgs {
     const int *slot_map;     // slot of each block within a row (nullptr: block = slot)
     const double *rad;       // [nsteps][N][block] radial factors
     const double2 *cs;       // [nsteps][nz] (2 dt / (dt + lambda), (dt - lambda) / (dt + lambda))
-    const double *dt;        // [nsteps]
+    const double *dt2;       // [nsteps] 2 dt
     double *norms;           // converged form: [row][N][groups][2]
     const int *skip;         // converged form: not 0: nothing to do (nullptr: always run)
     int inst0, nslots, ntile, groups;
     int numr, numz, nr, nz, ldq, N, isym, mtiles, ksteps;
     int nsteps, source, add;
+    int lagged;              // converged form: the refinement's half-step order (nsteps counts its radial solves)
     double gamma;
     // split transforms (p1 > 0)
     const double *Cs;        // packed A fragments of the cosine matrix, then of the sine matrix
@@ -540,12 +551,18 @@ __global__ void k_pack_modal(const double *__restrict__ rad, double *__restrict_
     }
 }
 
+// Step coefficients: blocks 0 .. nsteps - 1 the schedule's steps, the nsteps + 1
+// after them the refinement's radial solves.
 __global__ void k_modal_coef(const double *__restrict__ dt, const double *__restrict__ lam, double2 *__restrict__ cs,
-                             int nz) {
-    const double d = dt[blockIdx.x];
+                             double *__restrict__ dt2, int nz, int nsteps) {
+    const int i = (int)blockIdx.x - nsteps;  // refinement solve
+    const bool alone = i == nsteps;
+    const double a = dt[i < 0 ? (int)blockIdx.x : i > 0 ? i - 1 : 0], b = i < 0 ? a : alone ? 0.0 : dt[i];
+    if (threadIdx.x == 0) dt2[blockIdx.x] = alone ? 1.0 : a + b;
     for (int q = threadIdx.x; q < nz; q += blockDim.x) {
-        const double den = d + lam[q];
-        cs[(long long)blockIdx.x * nz + q] = make_double2(2.0 * d / den, (d - lam[q]) / den);
+        const double den = b + lam[q];
+        cs[(long long)blockIdx.x * nz + q] =
+            alone ? make_double2(1.0, a - lam[q]) : make_double2((a + b) / den, (a - lam[q]) / den);
     }
 }
 
@@ -586,7 +603,7 @@ __global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_mod
     const double *frad = a.rad + (long long)ti.slot * block;
     const long long fstep = (long long)a.N * block;
     auto fetch = [&](int step) {
-        const double *src = frad + step * fstep;
+        const double *src = frad + (kCycle && a.lagged && step > 0 ? step - 1 : step) * fstep;
         double *dst = sm + (step & 1) * block;
         for (int i = 2 * tid; i < block; i += 2 * blockDim.x) {
             const unsigned d = (unsigned)__cvta_generic_to_shared(dst + i);
@@ -625,13 +642,17 @@ __global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_mod
         const double2 *back = pair + ROWS;
         const double *kk = fac + 4 * ROWS + w * SEG;
         const double2 cs = a.cs[(long long)step * nz + q];
-        const double dt2 = 2.0 * a.dt[step];
+        const double dt2 = a.dt2[step];
         double y = 0.0;
 #pragma unroll
         for (int e = 0; e < SEG; ++e) {
             const double2 f = pair[e];
             y = fma(f.y, y, r[e] * f.x);
             x[e] = y;
+        }
+        if (kCycle && a.lagged && step + 1 == a.nsteps) {  // the solve without a vertical one
+#pragma unroll
+            for (int e = 0; e < SEG; ++e) r[e] = 0.0;
         }
         ends[w * kLines + lane] = y;
         __syncthreads();  // every warp is past the previous step: its factor buffer is free
@@ -1008,7 +1029,8 @@ cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
     c->launches += 2;
     const int nseg = radial_rows(c) / c->modal_seg;
     k_pack_modal<<<(unsigned)(s.nsteps * c->N), nseg, 0, c->stream>>>(s.d_rad, s.d_mod_rad, c->nr, nseg, c->modal_seg);
-    k_modal_coef<<<(unsigned)s.nsteps, 128, 0, c->stream>>>(s.d_dt, c->d_modlam, s.d_mod_cs, c->nz);
+    k_modal_coef<<<(unsigned)(2 * s.nsteps + 1), 128, 0, c->stream>>>(s.d_dt, c->d_modlam, s.d_mod_cs, s.d_mod_dt2,
+                                                                     c->nz, s.nsteps);
     return cudaGetLastError();
 }
 
@@ -1039,7 +1061,7 @@ cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, co
     a.nslots = nslots;
     a.rad = s.d_mod_rad;
     a.cs = s.d_mod_cs;
-    a.dt = s.d_dt;
+    a.dt2 = s.d_mod_dt2;
     a.nsteps = s.nsteps;
     const int threads = tile_threads(c);
     for (int r0 = 0; r0 < ninst; r0 += chunk) {
@@ -1064,7 +1086,8 @@ cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, co
 // ninst instances; cycles on them; a potential back in P.  The FP64 form takes
 // the one before the last step and runs that step in half-step form: the
 // residual it reports is the half-step iteration's, whose rounding floor its
-// last vertical half-step sets.  The mixed form takes the last one.
+// last vertical half-step sets.  The mixed form (pre: nullptr) takes the last
+// one, its cycles in the refinement's half-step order.
 cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R, double *Y, double *phi, int ninst,
                                const int *inst_map) {
     ModalArgs a = base_args(c);
@@ -1090,9 +1113,11 @@ cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double 
     a.phi = phi;
     a.pre = pre;
     a.rad = s.d_mod_rad;
-    a.cs = s.d_mod_cs;
-    a.dt = s.d_dt;
-    a.nsteps = s.nsteps;
+    a.lagged = pre ? 0 : 1;
+    const int first = a.lagged ? s.nsteps : 0;
+    a.cs = s.d_mod_cs + (size_t)first * c->nz;
+    a.dt2 = s.d_mod_dt2 + first;
+    a.nsteps = s.nsteps + a.lagged;
     a.norms = norms;
     a.skip = skip;
     return launch(c, radial_kernel<true>(c), (long long)ninst * c->N * a.groups, kLines * radial_nseg(c), radial_smem(c), a,

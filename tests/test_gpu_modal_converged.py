@@ -43,3 +43,31 @@ def test_update_ends_at_rounding(bph, monkeypatch, grid, graph):
         b.close()
         s.close()
     assert cycles["modal"][0] <= cycles["half"][0] + 2 and cycles["modal"][1] <= cycles["half"][1] + 2
+
+
+@pytest.mark.parametrize("grid", GRIDS, ids=IDS)
+def test_mixed_cycles_are_the_refinement_iteration(bph, monkeypatch, grid):
+    """The FP64 cycles that run in place of the grid-wide FP32 refinement take its half-steps, which
+    end on a radial solve: no more cycles than it (one, where an update meets the tolerance by less
+    than FP32 rounding), and less than a tenth of the residual at which half-steps that end on the
+    vertical solve stagnate (its radially stiff components are the larger by that and more)."""
+    g = (grid[0], grid[1], grid[2], 1.0 / (grid[0] - 4), grid[3], grid[4])
+    rhos = [np.asfortranarray(smooth_density(*g[:5], seed=50 + i)) for i in range(2)]
+    out = {}
+    for form in ("modal", "half"):
+        if form == "half":
+            monkeypatch.setenv("BPH_ADI_MODAL", "0")
+        s = bph.PotentialSolver(*g)
+        s.set_mixed_adi(MIXED_ADI_GLOBAL)
+        b = bph.Batch(s, capacity=2)
+        _, cold = s.solve_converged_mixed(rhos[0], 10, True, 1e-11, 60)
+        _, warm = s.solve_converged_mixed(rhos[1], 10, False, 1e-11, 60)
+        _, many = b.solve_converged(rhos, 10, True, 1e-11, 60, mixed=True)
+        out[form] = (cold, warm, many)
+        if form == "half":
+            _, vertical = s.solve_converged(rhos[0], 10, True, 1e-15, 30)
+        b.close()
+        s.close()
+    for modal, half in zip(out["modal"], out["half"]):
+        assert modal.residual <= 0.1 * vertical.residual
+        assert modal.cycles <= half.cycles + 1
