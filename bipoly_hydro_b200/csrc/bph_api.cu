@@ -278,8 +278,8 @@ int upload(bph_ctx *c, void *dst, const void *src, size_t bytes) {
 // zeroed slot array: r = 0, so the state stays zero) and keeps the faster.
 // Set-up autotuning of the per-grid kernel choices: the boundary contraction
 // (compact or full tables), the FFT tiles (regular or dense) and the FP64
-// ADI kernel (warp-cooperative or segmented, where both apply).  Each
-// candidate runs once untimed and three times timed on zero data, and the
+// ADI kernel (warp-cooperative or segmented, where both apply) and, for tall
+// slots, its form.  Each candidate runs once untimed and three times timed on zero data, and the
 // faster stays; BPH_COMPACT, BPH_FFT_DENSE and BPH_ADI_WARP in the
 // environment force their choice, BPH_AUTOTUNE=0 skips all of it.
 int autotune_setup(bph_ctx *c) {
@@ -336,6 +336,36 @@ int autotune_setup(bph_ctx *c) {
         c->adi_warp = shape;
         timed([&] { return launch_adi_plain(c, *s, 0, 5, false); }, &c->tuned_adi_us[1]);
         if (c->tuned_adi_us[0] < c->tuned_adi_us[1]) c->adi_warp = 0;
+    }
+    // tall slots: half-steps or the vertical eigenbasis, behind the contraction as in a solve
+    if (e == cudaSuccess && modal_tall(c)) {
+        Schedule *s;
+        int rc = get_schedule(c, 5, &s);
+        if (rc) return rc;
+        if (s->d_mod_rad) {
+            Schedule part = *s;
+            float us[2][2] = {};
+            for (int k = 0; k < 2; ++k) {
+                part.nsteps = k ? 5 : 1;
+                timed(
+                    [&] {
+                        cudaError_t f = launch_green_contract(c);
+                        return f == cudaSuccess ? launch_adi_plain(c, *s, 0, part.nsteps, false) : f;
+                    },
+                    &us[0][k]);
+                timed(
+                    [&] {
+                        cudaError_t f = launch_green_contract(c);
+                        return f == cudaSuccess ? launch_modal(c, part, false, c->d_P, c->d_R, c->d_modY, 1, 1, nullptr,
+                                                               nullptr, c->N, c->stream, c->pdl)
+                                                : f;
+                    },
+                    &us[1][k]);
+            }
+            if (e == cudaSuccess) modal_rule(c, us);
+        }
+    } else {
+        modal_rule(c, nullptr);  // the warp kernel may be out
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -549,6 +579,7 @@ int setup_impl(bph_ctx *c) {
         if ((rc = dev_alloc(c, &c->d_W2, (size_t)c->N * c->np))) return rc;
     }
     if ((rc = modal_configure(c))) return rc;  // after every allocation the context cannot do without
+    modal_rule(c, nullptr);
     Schedule *s;
     if ((rc = get_schedule(c, 5, &s))) return rc;
     if ((rc = get_schedule(c, 20, &s))) return rc;
@@ -593,7 +624,8 @@ int solve_device(bph_ctx *c, const double *d_rho, double *d_pot, const Schedule 
     // 50.5), and beside slots beyond shared memory the contraction finds no idle SM (258 x 194 x 512:
     // 1592 against 1578); else the overlap pays (101 x 75 x 128: 107 against 117, 130 x 98 x 256: 169
     // against 187).
-    const bool split = c->overlap && c->adi_seg && 8 * c->nfree >= c->N && c->nfree < c->N;
+    const bool split = c->overlap && c->adi_seg && 8 * c->nfree >= c->N && c->nfree < c->N &&
+                       (!modal_ready(c, s) || modal_overlaps(c));
     if (c->green && cap == cudaStreamCaptureStatusNone && split) {
         // contraction on partition 0, free-slot ADI on partition 1, both from the forward FFT
         BPH_CUDA(cudaEventRecord(c->ev_fft, c->stream));
@@ -1146,6 +1178,8 @@ long long bph_info(const bph_ctx_t *c, int what) {
         case BPH_INFO_FFT_DENSE_NS: return (long long)(1e3f * c->tuned_fft_us[1]);
         case BPH_INFO_ADI_SEG_NS: return (long long)(1e3f * c->tuned_adi_us[0]);
         case BPH_INFO_ADI_WARP_NS: return (long long)(1e3f * c->tuned_adi_us[1]);
+        case BPH_INFO_ADI_MODAL: return c->modal ? c->modal_min : 0;
+        case BPH_INFO_MODAL_SPLIT: return c->modal ? c->modal_p1 : 0;
         case BPH_INFO_MIXED_DIRECT_NS: return (long long)(1e3f * c->mixed_tuned_us[BPH_MIXED_DIRECT]);
         default: return -1;
     }

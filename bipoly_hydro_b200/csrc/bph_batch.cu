@@ -832,7 +832,7 @@ int batch_enqueue(bph_batch *b, int n, const double *const *d_in, double *const 
     Schedule *s = &sch;
     int rc = batch_prologue(b, n, d_in, d_map, per_pos);
     if (rc) return rc;
-    if (modal_ready(c, *s) && b->d_mody)
+    if (modal_ready(c, *s, true) && b->d_mody)
         BPH_CUDA(launch_modal(c, *s, !warm, b->d_P, b->d_R, b->d_mody, modal_chunk(c, b->cap), n, d_map, nullptr, c->N,
                               c->stream, c->pdl));
     else if (c->adi_seg)

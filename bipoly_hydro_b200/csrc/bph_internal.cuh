@@ -216,6 +216,8 @@ struct bph_ctx {
     float *d_r32 = nullptr;            // rounded residual of one solve [N][np] (FP32 warp refinement)
     // ADI in the vertical eigenbasis (bph_modal.cu)
     int modal = 0;                     // 1: the FP64 ADI runs there
+    int modal_min = 0;                 // steps from which a solve's schedule does, and a batch's (modal_rule)
+    int modal_min_batch = 0;
     int modal_seg = 0;                 // radii per segment of a radial line
     int modal_p1 = 0;                  // first factor of the split transforms (0: dense)
     int modal_beta1 = 0;               // multiplier of its angles
@@ -435,7 +437,10 @@ size_t modal_size(const bph_ctx *c);  // doubles of one instance's modal array
 int modal_chunk(const bph_ctx *c, int capacity);  // instances per pass of a batch's launch_modal
 size_t modal_radial_doubles(const bph_ctx *c);  // of one (step, slot) radial factor block
 cudaError_t modal_pack(bph_ctx *c, Schedule &s);
-bool modal_ready(const bph_ctx *c, const Schedule &s);
+bool modal_tall(const bph_ctx *c);
+void modal_rule(bph_ctx *c, const float (*us)[2]);
+bool modal_ready(const bph_ctx *c, const Schedule &s, bool batch = false);
+bool modal_overlaps(const bph_ctx *c);
 // Whether converged cycles of schedule s run there (mixed: in place of the
 // grid-wide FP32 refinement).
 bool modal_converged(const bph_ctx *c, const Schedule &s, bool mixed);

@@ -1034,22 +1034,79 @@ cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
     return cudaGetLastError();
 }
 
-// A schedule's form.  The transforms cost a fixed ~60 us and a modal step ~5
-// at 130 x 98 x 256; the warp-cooperative half-step kernel spends 15 per step
-// (66 x 66 x 64: 14 + 0.8 against 4 + 2.3), so where it applies it keeps the
-// schedules of up to seven steps.  Every other half-step kernel is slower than
-// the modal form from five steps on (101 x 75 x 128: 50 against 101 us,
-// 258 x 194 x 256: 551 against 1034; shorter schedules are not a solver's).
-bool modal_ready(const bph_ctx *c, const Schedule &s) {
-    return c->modal && s.d_mod_rad && !(c->adi_warp && s.nsteps <= 7);
+// A schedule's form: in the eigenbasis from modal_min steps on.  The
+// transforms cost a fixed time and a modal step little; a half-step kernel has
+// no fixed part to speak of.
+//   Warp-cooperative half-steps (130 x 98 x 256: 70 + 4.6 a step in the
+//   eigenbasis against 22 + 10; 66 x 66 x 64: 14 + 0.8 against 4 + 2.3): eight.
+//   The other half-step kernels: two (us for one and for two steps, half-steps
+//   against eigenbasis: 101 x 75 x 128 26 / 44 against 40 / 42, 67 x 45 x 64
+//   15 / 25 against 16 / 17, 258 x 194 x 512 424 / 790 against 485 / 526).
+//   Tall slots, whose transforms' products are long serial chains (serial_steps
+//   of 64 clocks and more each): where the set-up's timing says, which for the
+//   five steps of a warm solve went to the half-steps at 12 x 500 x 32 (131
+//   against 203 us a solve), 8 x 200 x 64 (70 against 83) and 258 x 402 x 16
+//   (545 against 605), and to the eigenbasis at 40 x 400 x 64 (328 against
+//   269), 20 x 300 x 64 (113 against 87) and 20 x 146 x 64 (71 against 58).
+//   The timing has no second stream for the free slots' half-steps, hence a
+//   margin of a tenth.  Untimed: eight.
+// Batches fill the chip better in either form and take the eigenbasis from two
+// steps on (us for one and for sixteen models: 8 x 200 x 64 98 / 466 in
+// half-steps, 89 / 325; 258 x 402 x 16 776 / 3484, 674 / 3411), but for the
+// longest chains on the segmented kernel (20 x 402 x 128 208 / 2067 against
+// 223 / 2177, 12 x 500 x 32 168 / 556 against 232 / 923).
+static int serial_steps(const bph_ctx *c) {
+    if (!c->modal_p1) {
+        const int mt = (c->nz + 15) / 16;
+        return (mt + 7) / 8 * ((c->nz + 7) / 8);
+    }
+    const int h2 = ((2 * c->nz + 1) / c->modal_p1 + 1) / 2, units = (c->modal_p1 + 1) / 2 * ((h2 + 15) / 16);
+    return (units + 7) / 8 * 2 * ((h2 + 7) / 8);
 }
 
-// The grid-wide FP32 refinement cycle costs more than a modal cycle in FP64
-// (258 x 194 x 512, ten steps: 2500 against 880 us), so the mixed form runs
+// Whether the set-up's timing decides: 24 serial steps for the on-chip
+// segmented kernel, 100 for the slower grid-wide ones (the kernel with a
+// thread per line is the slower form from one step on at every height).
+bool modal_tall(const bph_ctx *c) {
+    return c->modal && !c->adi_warp && (c->adi_seg || !c->adi_smem) && serial_steps(c) > (c->adi_seg ? 24 : 100);
+}
+
+// us[form][k]: contraction and ADI of 1 (k = 0) and 5 steps in half-steps and
+// in the eigenbasis, both linear in the steps; nullptr: untimed.
+void modal_rule(bph_ctx *c, const float (*us)[2]) {
+    c->modal_min = c->adi_warp ? 8 : 2;
+    c->modal_min_batch = c->modal_min;
+    if (!modal_tall(c)) return;
+    c->modal_min = 8;
+    if (us) {
+        const float half = (us[0][1] - us[0][0]) / 4, modal = (us[1][1] - us[1][0]) / 4;
+        int n = 2;
+        while (n < 64 && us[1][0] + modal * (n - 1) >= 0.9f * (us[0][0] + half * (n - 1))) ++n;
+        c->modal_min = n;
+    }
+    if (c->adi_seg && serial_steps(c) > 100) c->modal_min_batch = c->modal_min;
+}
+
+bool modal_ready(const bph_ctx *c, const Schedule &s, bool batch) {
+    return c->modal && s.d_mod_rad && s.nsteps >= (batch ? c->modal_min_batch : c->modal_min);
+}
+
+// Converged cycles stay in the eigenbasis, so only the choice between warp
+// kernel and modal steps is one of steps (at most seven: the warp kernel).  The
+// grid-wide FP32 refinement cycle costs more than a modal cycle in FP64
+// (258 x 194 x 512, ten steps: 2500 against 480 us), so the mixed form runs
 // the latter where that refinement would be its choice.
 bool modal_converged(const bph_ctx *c, const Schedule &s, bool mixed) {
-    return modal_ready(c, s) && (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
+    return c->modal && s.d_mod_rad && !(c->adi_warp && s.nsteps <= 7) &&
+           (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
 }
+
+// Whether a solve's slots are worth two passes, the free ones' beside the
+// contraction: below this many zones the kernels of a pass are latency, and
+// two of each cost more than they hide (us per warm solve with and without:
+// 18 x 18 x 16 31 / 18, 50 x 50 x 256 54 / 47, 200 x 30 x 128 92 / 88;
+// 101 x 75 x 128 94 / 100, 110 x 90 x 256 154 / 168).
+bool modal_overlaps(const bph_ctx *c) { return c->np * c->N >= 800000; }
 
 cudaError_t launch_modal(bph_ctx *c, const Schedule &s, bool cold, double *P, const double *R, double *Y, int chunk,
                          int ninst, const int *inst_map, const int *slot_map, int nslots, cudaStream_t st, bool pdl) {

@@ -69,7 +69,7 @@ CONTRACT_FULL, CONTRACT_COMPACT = 1, 2
 INFO_KEYS = ("adi_threads", "adi_smem", "mixed_threads", "mixed_smem", "mixed_ctas_per_sm", "contract_split",
              "mixed_kind", "mixed_forward_ns", "mixed_increment_ns", "adi_prefetch", "adi_kernel", "adi_warp_smem",
              "mixed_warp_ns", "green_sms", "contract_kind", "fft_dense", "contract_full_ns", "contract_compact_ns",
-             "fft_ns", "fft_dense_ns", "adi_seg_ns", "adi_warp_ns", "mixed_direct_ns")
+             "fft_ns", "fft_dense_ns", "adi_seg_ns", "adi_warp_ns", "mixed_direct_ns", "adi_modal", "modal_split")
 
 #: bph_run_phase phase ids.
 PHASE_FFT_RHO, PHASE_CONTRACT, PHASE_SLOTS, PHASE_ADI, PHASE_FFT_INV = range(5)

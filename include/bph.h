@@ -365,6 +365,8 @@ int bph_green_contract_noalloc(bph_ctx_t *ctx, const double *d_mom, double *d_S)
 #define BPH_INFO_ADI_SEG_NS 20        /* set-up autotune: 5 ADI steps of every slot, segmented kernel, ns */
 #define BPH_INFO_ADI_WARP_NS 21       /* the same with the warp-cooperative kernel */
 #define BPH_INFO_MIXED_DIRECT_NS 22   /* setup-time duration of one direct FP32 defect solve, ns (0: not timed) */
+#define BPH_INFO_ADI_MODAL 23         /* steps from which a solve's FP64 ADI runs in the vertical eigenbasis (0: never) */
+#define BPH_INFO_MODAL_SPLIT 24       /* first factor of its split transforms (0: dense) */
 #define BPH_CONTRACT_FULL 1           /* streams the full tables G[m][b][p] */
 #define BPH_CONTRACT_COMPACT 2        /* streams the symmetric tiles and side vectors (2/3 fewer bytes) */
 #define BPH_ADI_KERNEL_WARP 1         /* warp-cooperative line solves, shuffle carries (128x96, 64x64 interiors) */
