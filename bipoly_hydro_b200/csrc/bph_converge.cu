@@ -5,13 +5,14 @@
 // ADI steps and measures ||phi - phi_prev|| / ||phi||; the mixed form
 // (bph_solve_converged_mixed) runs one FP32 refinement cycle that reports
 // ||delta|| / ||phi|| itself.  Instead of a host round trip per cycle, the
-// cycle is the body of a CUDA graph `while` node: after each cycle
-// k_conv_check reduces the per-slot norms, applies the stopping rule and sets
-// the node's condition, so the whole loop is one graph launch and the host
+// loop is one CUDA graph: a cycle, then a `while` node whose body holds the
+// further ones.  After each cycle k_conv_check reduces the per-slot norms,
+// applies the stopping rule and sets the node's condition; the host
 // reads the cycle count once at the end.  The graph is built by stream
 // capture of the same launchers the host loop uses, once per context,
 // schedule and kernel choice.
 #include <cmath>
+#include <vector>
 
 #include "bph_internal.cuh"
 
@@ -19,10 +20,13 @@ namespace bph {
 namespace {
 
 constexpr int kCheckThreads = 256;
-// Cycles per pass of the while node's body where a cycle can be skipped: an
-// iteration of the node costs more than the two launches of a skipped cycle,
-// and most solves take three or four cycles.
-constexpr int kBodyCycles = 4;
+// The first cycle runs ahead of the while node, which a solve of one cycle then
+// does not enter.  Cycles per pass of the node's body where a cycle can be
+// skipped: an iteration of the node costs more than the two launches of a
+// skipped cycle, and most solves take three or four cycles.  (All four in the
+// body: 127 us for the one cycle of a solve that starts converged at
+// 66 x 66 x 64, 112 mixed; one ahead: 119 and 104.)
+constexpr int kBodyCycles = 3;
 
 __global__ void k_conv_init(ConvState *st, double tol, int max_cycles, int mixed, double least) {
     st->tol = tol;
@@ -78,8 +82,57 @@ __global__ void __launch_bounds__(kCheckThreads) k_conv_check(const double *__re
 
 }  // namespace
 
-// Builds the while-graph of one converged form on the context's current
-// arrays and schedule s (the cycle body captured from the launchers).
+// Captures reps cycles of a converged form and their checks on cs into graph g;
+// past the first, a cycle returns at once when the loop has stopped.
+static cudaError_t capture_cycles(bph_ctx *c, Schedule &s, bool mixed, bool modal, int reps, cudaStream_t cs,
+                                  cudaGraph_t g, cudaGraphConditionalHandle cond,
+                                  std::vector<cudaGraphNode_t> *last_nodes) {
+    cudaError_t e = cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    cudaStream_t keep = c->stream;
+    const bool keep_pdl = c->pdl;
+    c->stream = cs;
+    c->pdl = false;  // plain serial edges between the cycles
+    cudaError_t ce = cudaSuccess;
+    for (int r = 0; r < reps && ce == cudaSuccess; ++r) {
+        const int *skip = r > 0 ? &c->d_conv->done : nullptr;
+        if (modal) {
+            ce = launch_modal_cycle(c, s, c->d_modY, c->d_prev, mixed ? nullptr : c->d_modpre, 1, c->d_modnorm, skip);
+        } else if (mixed) {
+            ce = launch_adi_defect(c, s, skip);
+        } else if (c->adi_seg) {  // the update norms come from the sweep's write-back
+            ce = launch_adi(c, s, 0, s.nsteps, false, nullptr, nullptr, 1, nullptr, c->d_red);
+        } else {
+            ce = cudaMemcpyAsync(c->d_prev, c->d_P, sizeof(double) * (size_t)c->N * c->nplane,
+                                 cudaMemcpyDeviceToDevice, cs);
+            if (ce == cudaSuccess) ce = launch_adi(c, s, 0, s.nsteps, false);
+            if (ce == cudaSuccess) ce = launch_update_norm(c, c->d_red);
+        }
+        if (ce == cudaSuccess) {
+            k_conv_check<<<1, kCheckThreads, 0, cs>>>(modal ? c->d_modnorm : c->d_red,
+                                                      modal ? c->N * modal_groups(c) : c->N, c->d_conv, cond,
+                                                      r + 1 == reps);
+            ce = cudaGetLastError();
+        }
+        ++c->launches;
+    }
+    c->stream = keep;
+    c->pdl = keep_pdl;
+    if (ce == cudaSuccess && last_nodes) {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t *nodes = nullptr;
+        size_t count = 0;
+        ce = cudaStreamGetCaptureInfo(cs, &status, nullptr, nullptr, &nodes, &count);
+        if (ce == cudaSuccess) last_nodes->assign(nodes, nodes + count);
+    }
+    cudaGraph_t into = nullptr;
+    e = cudaStreamEndCapture(cs, &into);
+    return e == cudaSuccess ? ce : e;
+}
+
+// Builds the graph of one converged form on the context's current arrays and
+// schedule s (the cycles captured from the launchers): a cycle, then a while
+// node over further ones.
 static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t *out) {
     *out = nullptr;
     const bool modal = modal_converged(c, s, mixed) && (mixed || c->d_modpre);
@@ -89,6 +142,9 @@ static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t
     cudaError_t e = cudaGraphCreate(&g, 0);
     cudaGraphConditionalHandle cond = 0;
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
+    std::vector<cudaGraphNode_t> after;
+    if (e == cudaSuccess) e = capture_cycles(c, s, mixed, modal, 1, cs, g, cond, &after);
     cudaGraphNodeParams p = {};
     cudaGraphNode_t node = nullptr;
     if (e == cudaSuccess) {
@@ -96,48 +152,11 @@ static int build_conv_graph(bph_ctx *c, Schedule &s, bool mixed, cudaGraphExec_t
         p.conditional.handle = cond;
         p.conditional.type = cudaGraphCondTypeWhile;
         p.conditional.size = 1;
-        e = cudaGraphAddNode(&node, g, nullptr, 0, &p);
+        e = cudaGraphAddNode(&node, g, after.data(), after.size(), &p);
     }
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
+    const bool skips = modal || (mixed && c->mixed_kind == BPH_MIXED_DIRECT);
     if (e == cudaSuccess)
-        e = cudaStreamBeginCaptureToGraph(cs, p.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        cudaStream_t keep = c->stream;
-        const bool keep_pdl = c->pdl;
-        c->stream = cs;
-        c->pdl = false;  // plain serial edges inside the loop body
-        cudaError_t ce = cudaSuccess;
-        const bool skips = modal || (mixed && c->mixed_kind == BPH_MIXED_DIRECT);
-        const int reps = skips ? kBodyCycles : 1;
-        for (int r = 0; r < reps && ce == cudaSuccess; ++r) {
-            const int *skip = skips && r > 0 ? &c->d_conv->done : nullptr;
-            if (modal) {
-                ce = launch_modal_cycle(c, s, c->d_modY, c->d_prev, mixed ? nullptr : c->d_modpre, 1, c->d_modnorm, skip);
-            } else if (mixed) {
-                ce = launch_adi_defect(c, s, skip);
-            } else if (c->adi_seg) {  // the update norms come from the sweep's write-back
-                ce = launch_adi(c, s, 0, s.nsteps, false, nullptr, nullptr, 1, nullptr, c->d_red);
-            } else {
-                ce = cudaMemcpyAsync(c->d_prev, c->d_P, sizeof(double) * (size_t)c->N * c->nplane,
-                                     cudaMemcpyDeviceToDevice, cs);
-                if (ce == cudaSuccess) ce = launch_adi(c, s, 0, s.nsteps, false);
-                if (ce == cudaSuccess) ce = launch_update_norm(c, c->d_red);
-            }
-            if (ce == cudaSuccess) {
-                k_conv_check<<<1, kCheckThreads, 0, cs>>>(modal ? c->d_modnorm : c->d_red,
-                                                          modal ? c->N * modal_groups(c) : c->N, c->d_conv, cond,
-                                                          r + 1 == reps);
-                ce = cudaGetLastError();
-            }
-            ++c->launches;
-        }
-        c->stream = keep;
-        c->pdl = keep_pdl;
-        cudaGraph_t body = nullptr;
-        e = cudaStreamEndCapture(cs, &body);
-        if (e == cudaSuccess) e = ce;
-    }
+        e = capture_cycles(c, s, mixed, modal, skips ? kBodyCycles : 1, cs, p.conditional.phGraph_out[0], cond, nullptr);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
     if (cs) cudaStreamDestroy(cs);
     if (g) cudaGraphDestroy(g);

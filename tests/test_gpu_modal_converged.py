@@ -71,3 +71,23 @@ def test_mixed_cycles_are_the_refinement_iteration(bph, monkeypatch, grid):
     for modal, half in zip(out["modal"], out["half"]):
         assert modal.residual <= 0.1 * vertical.residual
         assert modal.cycles <= half.cycles + 1
+
+
+@pytest.mark.parametrize("kind", ["fp64", "global", "direct"])
+def test_device_loop_ends_after_any_cycle(bph, monkeypatch, kind):
+    """The device loop (a cycle, then passes of several) stops after 1 to 9 cycles like the host
+    loop: the same count and the same potential, bit for bit."""
+    g = (40, 30, 64, 1.0 / 36.0, 2, 16)
+    rho = np.asfortranarray(smooth_density(*g[:5], seed=60))
+    out = {}
+    for graph in ("1", "0"):
+        monkeypatch.setenv("BPH_CONV_GRAPH", graph)
+        s = bph.PotentialSolver(*g)
+        if kind != "fp64":
+            s.set_mixed_adi(MIXED_ADI_GLOBAL if kind == "global" else 5)  # 5: the direct defect solve
+        solve = s.solve_converged if kind == "fp64" else s.solve_converged_mixed
+        out[graph] = [solve(rho, 10, True, 0.0, n) for n in range(1, 10)]
+        s.close()
+    for n, (a, b) in enumerate(zip(out["1"], out["0"]), 1):
+        assert a[1].cycles == b[1].cycles and (a[1].cycles == n or kind != "fp64")
+        assert np.array_equal(a[0], b[0])
