@@ -576,7 +576,7 @@ int setup_impl(bph_ctx *c) {
             return BPH_ERR_INVALID;
         }
         if ((rc = dev_alloc(c, &c->d_W, (size_t)c->N * c->nplane))) return rc;
-        if ((rc = dev_alloc(c, &c->d_W2, (size_t)c->N * c->np))) return rc;
+        if ((rc = dev_alloc(c, &c->d_W2, modal_size(c)))) return rc;  // at least N np; a modal array fits
     }
     if ((rc = modal_configure(c))) return rc;  // after every allocation the context cannot do without
     modal_rule(c, nullptr);
@@ -717,11 +717,6 @@ static void ctx_free(bph_ctx *c) {
     if (c->own_stream) cudaStreamSynchronize(c->own_stream);
     if (c->stream && c->stream != c->own_stream) cudaStreamSynchronize(c->stream);
     for (auto &s : c->sched) free_schedule(c, s);
-    double *bufs[] = {c->d_green, c->d_brb,  c->d_elz, c->d_alphar, c->d_betar,     c->d_bzb,
-                      c->d_qcoef, c->d_grid, c->d_R,   c->d_P,      c->d_prev,      c->d_mom,
-                      c->d_S,     c->d_W,    c->d_W2,  c->d_P2,     c->d_red,       c->d_rho_stage, c->d_pot_stage,
-                      c->d_phieff_stage};
-    for (double *p : bufs) dev_free(p);
     dev_free(c->d_tw);
     dev_free(c->d_tw2);
     dev_free(c->d_ph);
@@ -735,13 +730,18 @@ static void ctx_free(bph_ctx *c) {
     conv_graphs_free(c);
     modal_free(c);
     dev_free(c->d_work32);
-    dev_free(c->d_modpre);
+    if (c->d_modpre != c->d_W2) dev_free(c->d_modpre);
     dev_free(c->d_warp_coef);
     dev_free(c->d_warp_coef32);
     dev_free(c->d_r32);
     dev_free(c->d_dir32);
     dev_free(c->d_dirS);
     dev_free(c->d_scf);
+    double *bufs[] = {c->d_green, c->d_brb,  c->d_elz, c->d_alphar, c->d_betar,     c->d_bzb,
+                      c->d_qcoef, c->d_grid, c->d_R,   c->d_P,      c->d_prev,      c->d_mom,
+                      c->d_S,     c->d_W,    c->d_W2,  c->d_P2,     c->d_red,       c->d_rho_stage, c->d_pot_stage,
+                      c->d_phieff_stage};
+    for (double *p : bufs) dev_free(p);
     if (c->side_stream) {
         cudaStreamSynchronize(c->side_stream);
         cudaStreamDestroy(c->side_stream);

@@ -43,7 +43,9 @@ struct bph_batch {
     int *d_stat = nullptr;     // [cap] non-finite flag of each batch position (host-array calls)
     int *h_stat = nullptr;     // [cap] pinned host copy
     int stage_cap = 0;         // positions of the host-array staging buffers
-    double *d_LW = nullptr, *d_LQ = nullptr;  // grid-wide ADI scratch [cap][N][np] (large slots)
+    // grid-wide ADI scratch, each [cap][N][np] (large slots), one after the other: at least cap modal
+    // arrays, which live there (d_mody, d_mod) while the steps are modal
+    double *d_LW = nullptr, *d_LQ = nullptr;
     double *d_prev = nullptr;         // converged FP64 solves: slot arrays of the previous cycle (on first use);
                                       // modal form: the modal potential
     double *d_mod = nullptr;          // modal form: the modal residual (cap times modal_size)
@@ -553,8 +555,8 @@ int bph_batch_create(bph_ctx_t *c, int capacity, bph_batch_t **out) {
     if (!rc) rc = batch_alloc(b, &b->d_R, (size_t)capacity * c->N * c->np);
     if (!rc) rc = batch_alloc(b, &b->d_mom, (size_t)c->g.mmax * capacity * 2 * c->np);
     if (!rc) rc = batch_alloc(b, &b->d_C, (size_t)c->g.mmax * 2 * capacity * c->nb);
-    if (!rc && large) rc = batch_alloc(b, &b->d_LW, (size_t)capacity * c->N * c->np);
-    if (!rc && large) rc = batch_alloc(b, &b->d_LQ, (size_t)capacity * c->N * c->np);
+    if (!rc && large) rc = batch_alloc(b, &b->d_LW, 2 * (size_t)capacity * c->N * c->np);
+    if (!rc && large) b->d_LQ = b->d_LW + (size_t)capacity * c->N * c->np;
     if (!rc) {
         // split-K scratch of the contraction: partial sums for the widest
         // column block (8 per CUDA-core launch, up to 64 per tensor-core
@@ -594,7 +596,10 @@ int bph_batch_create(bph_ctx_t *c, int capacity, bph_batch_t **out) {
         }
     }
     // last and optional: without room for it the batch runs the half-step form
-    if (!rc && c->modal) (void)batch_alloc(b, &b->d_mody, (size_t)modal_chunk(c, capacity) * modal_size(c));
+    if (!rc && c->modal && large)
+        b->d_mody = b->d_LW;
+    else if (!rc && c->modal)
+        (void)batch_alloc(b, &b->d_mody, (size_t)modal_chunk(c, capacity) * modal_size(c));
     if (!rc) {
         e = cudaMemsetAsync(b->d_P, 0, sizeof(double) * (size_t)capacity * c->N * c->nplane, c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mom, 0, sizeof(double) * (size_t)c->g.mmax * capacity * 2 * c->np,
@@ -613,8 +618,10 @@ int bph_batch_destroy(bph_batch_t *b) {
     if (!b) return BPH_OK;
     ::bph::DeviceScope scope_(b->c ? b->c->device : 0);
     if (b->c && b->c->stream) cudaStreamSynchronize(b->c->stream);
-    double *bufs[] = {b->d_P,     b->d_R,     b->d_mom, b->d_C,    b->d_rho_stage, b->d_pot_stage,
-                      b->d_cpart, b->d_LW,    b->d_LQ,  b->d_prev, b->d_cnorm, b->d_work32, b->d_mod, b->d_modpre, b->d_mnorm, b->d_mody};
+    if (b->d_LW) b->d_mody = b->d_mod = nullptr;  // in the scratch
+    double *bufs[] = {b->d_P,     b->d_R,  b->d_mom,  b->d_C,     b->d_rho_stage, b->d_pot_stage, b->d_cpart,
+                      b->d_LW,    b->d_prev, b->d_cnorm, b->d_work32, b->d_mod,     b->d_modpre,    b->d_mnorm,
+                      b->d_mody};
     for (double *p : bufs)
         if (p) cudaFree(p);
     if (b->d_ccnt) cudaFree(b->d_ccnt);
@@ -871,9 +878,10 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
         const size_t each = (size_t)b->cap * modal_size(c);
         const bool had_prev = b->d_prev != nullptr;
         if ((had_prev || !batch_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)) &&
-            !batch_alloc(b, &b->d_mod, each) && !batch_alloc(b, &b->d_modpre, each) &&
+            (b->d_LW || !batch_alloc(b, &b->d_mod, each)) && !batch_alloc(b, &b->d_modpre, each) &&
             cudaMallocHost((void **)&b->h_mnorm, sizeof(double) * norms) == cudaSuccess)
             (void)batch_alloc(b, &b->d_mnorm, norms);
+        if (b->d_LW) b->d_mod = b->d_mnorm ? b->d_LW : nullptr;
         if (!b->d_mnorm) {  // give back what was had: the other forms need the room
             cudaGetLastError();
             if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
@@ -884,7 +892,7 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
                 b->bytes -= sizeof(double) * count;
                 p = nullptr;
             };
-            give_back(b->d_mod, each);
+            give_back(b->d_mod, each);  // (nullptr where it is in the scratch)
             give_back(b->d_modpre, each);
             if (!had_prev) give_back(b->d_prev, (size_t)b->cap * c->N * c->nplane);
         }

@@ -148,7 +148,7 @@ struct bph_ctx {
     double *d_mom = nullptr;     // [mmax][2][np]
     double *d_S = nullptr;       // [mmax][nb][2]
     double *d_W = nullptr;       // ADI work slabs when they do not fit on chip
-    double *d_W2 = nullptr;      // tiled large-grid ADI: the radial half-sweep result [N][np], transposed
+    double *d_W2 = nullptr;      // tiled large-grid ADI: the radial half-sweep result [N][np], transposed (modal_size)
     double *d_P2 = nullptr;      // ADI potential slabs when they do not fit on chip
     double *d_red = nullptr;     // reduction scratch
     double *d_rho_stage = nullptr;
@@ -222,10 +222,11 @@ struct bph_ctx {
     int modal_p1 = 0;                  // first factor of the split transforms (0: dense)
     int modal_beta1 = 0;               // multiplier of its angles
     int *d_modtab = nullptr;           // split form: signed heights of (a1, a2)
-    double *d_modE = nullptr;          // packed fragments of E, then of E^T (one allocation with the next three)
+    double *d_modE = nullptr;          // packed fragments of E, then of E^T (one allocation with the arrays below)
     double *d_modlam = nullptr;        // [nz] gamma lambda_q
     double *d_modY = nullptr;          // [N][nr][nz, even] modal residual / update
-    double *d_modpre = nullptr;        // converged form: potential before a cycle's last step (on first use)
+    double *d_modpre = nullptr;        // converged form: potential before a cycle's last step (on first use; grid-wide
+                                       // half-steps: d_W2, and d_modY is d_W)
     double *d_modnorm = nullptr;       // [N][modal_groups][2] partial update norms of a cycle
     double *d_scf = nullptr;           // SCF-step mass partials and scale (bph_scf.cu)
     void *noalloc_scratch = nullptr;   // device address of the allocation-free contraction's scratch array

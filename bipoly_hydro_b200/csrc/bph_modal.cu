@@ -988,10 +988,14 @@ int modal_configure(bph_ctx *c) {
                     pack[frag + at] = entry(col, row);  // E^T: row = height
                 }
             }
-    // one allocation: both fragment arrays, the eigenvalues, the norm partials, one instance's modal array
+    // One allocation: both fragment arrays, the eigenvalues, the norm partials, one instance's modal
+    // array.  Slots beyond shared memory have their half-steps' scratch, which no solve needs while
+    // its steps are modal (d_W >= N nr (nz + 1)): the modal array and the converged form's earlier
+    // potential, which is back in P before the last half-steps run, live there.
+    const bool scratch = c->adi_smem == 0;
     const size_t norms = 2 * (size_t)c->N * modal_groups(c), lams = ((size_t)nz + 1) / 2 * 2;
     const size_t tabs = (tab.size() + 3) / 4 * 2;  // doubles that hold the index table
-    const size_t all = pack.size() + lams + norms + tabs + modal_size(c);
+    const size_t all = pack.size() + lams + norms + tabs + (scratch ? 0 : modal_size(c));
     if (cudaMalloc((void **)&c->d_modE, sizeof(double) * all) != cudaSuccess) {
         cudaGetLastError();  // no room: the half-step kernels need none of it
         c->d_modE = nullptr;
@@ -1000,7 +1004,8 @@ int modal_configure(bph_ctx *c) {
     c->d_modlam = c->d_modE + pack.size();
     c->d_modnorm = c->d_modlam + lams;
     c->d_modtab = reinterpret_cast<int *>(c->d_modnorm + norms);
-    c->d_modY = c->d_modnorm + norms + tabs;
+    c->d_modY = scratch ? c->d_W : c->d_modnorm + norms + tabs;
+    if (scratch) c->d_modpre = c->d_W2;
     c->bytes += sizeof(double) * all;
     pack.insert(pack.end(), lam.begin(), lam.end());
     BPH_CUDA(cudaMemcpyAsync(c->d_modE, pack.data(), sizeof(double) * pack.size(), cudaMemcpyHostToDevice, c->stream));
