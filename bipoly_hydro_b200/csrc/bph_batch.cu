@@ -28,6 +28,9 @@
 struct bph_batch {
     bph_ctx *c = nullptr;
     int cap = 0;
+    // the one device and the one pinned allocation of a batch's life (the device arrays below that no
+    // first use allocates, and both halves of the position tables and flags)
+    void *arena = nullptr, *h_arena = nullptr;
     double *d_P = nullptr;     // [cap][N][nplane]
     double *d_R = nullptr;     // [cap][N][np]
     double *d_mom = nullptr;   // [mmax][cap][2][np]
@@ -499,6 +502,59 @@ int batch_alloc(bph_batch *b, double **p, size_t count) {
     return BPH_OK;
 }
 
+// Arrival counters of the contraction, for the narrowest row groups (16 rows).
+size_t contract_counters(const bph_ctx *c) { return (size_t)c->g.mmax * ((c->nb + 15) / 16); }
+
+// Bytes of one set of position tables.
+size_t table_bytes(const bph_batch *b) {
+    return ((2 * sizeof(void *) + sizeof(int)) * (size_t)b->cap + 15) / 16 * 16;
+}
+
+// The batch's device arrays in one allocation (ten separate ones, the modal
+// work array among them, took 2.8 ms for four models at 66 x 66 x 64 and 2.3
+// without it; one: 1.9); modal: with the modal work array.
+int batch_arena(bph_batch *b, bool modal) {
+    const bph_ctx *c = b->c;
+    const size_t cap = (size_t)b->cap, slots = cap * c->N;
+    const bool large = !c->adi_seg;
+    size_t total = 0;
+    auto room = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t P = room(sizeof(double) * slots * c->nplane), R = room(sizeof(double) * slots * c->np),
+                 mom = room(sizeof(double) * 2 * cap * c->g.mmax * c->np),
+                 C = room(sizeof(double) * 2 * cap * c->g.mmax * c->nb);
+    const size_t scratch = large ? room(sizeof(double) * 2 * slots * c->np) : 0;
+    // split-K scratch of the contraction: partial sums for the widest column
+    // block (8 per CUDA-core launch, up to 64 per tensor-core launch)
+    const size_t cols = std::max<size_t>(8, std::min<size_t>(8 * kDmmaMaxTiles, 8 * ((2 * cap + 7) / 8)));
+    const size_t cpart = room(sizeof(double) * kBatchSplitMax * c->g.mmax * c->nb * cols),
+                 ccnt = room(sizeof(unsigned int) * contract_counters(c)), tab = room(2 * table_bytes(b)),
+                 stat = room(sizeof(int) * cap);
+    const size_t mody = modal && !large ? room(sizeof(double) * modal_chunk(c, b->cap) * modal_size(c)) : 0;
+    double *base = nullptr;
+    const int rc = batch_alloc(b, &base, total / sizeof(double));
+    if (rc) return rc;
+    char *p = reinterpret_cast<char *>(base);
+    b->arena = base;
+    b->d_P = reinterpret_cast<double *>(p + P);
+    b->d_R = reinterpret_cast<double *>(p + R);
+    b->d_mom = reinterpret_cast<double *>(p + mom);
+    b->d_C = reinterpret_cast<double *>(p + C);
+    if (large) {
+        b->d_LW = reinterpret_cast<double *>(p + scratch);
+        b->d_LQ = b->d_LW + slots * c->np;
+    }
+    b->d_cpart = reinterpret_cast<double *>(p + cpart);
+    b->d_ccnt = reinterpret_cast<unsigned int *>(p + ccnt);
+    for (int k = 0; k < 2; ++k) b->d_tab[k] = p + tab + k * table_bytes(b);
+    b->d_stat = reinterpret_cast<int *>(p + stat);
+    if (modal) b->d_mody = large ? b->d_LW : reinterpret_cast<double *>(p + mody);
+    return BPH_OK;
+}
+
 }  // namespace
 
 // Schedules are shared with the single-solve path (bph_api.cu).
@@ -550,60 +606,31 @@ int bph_batch_create(bph_ctx_t *c, int capacity, bph_batch_t **out) {
     b->c = c;
     ctx_retain(c);  // the context's device state stays until this batch is destroyed
     b->cap = capacity;
-    int rc = BPH_OK;
-    if (!rc) rc = batch_alloc(b, &b->d_P, (size_t)capacity * c->N * c->nplane);
-    if (!rc) rc = batch_alloc(b, &b->d_R, (size_t)capacity * c->N * c->np);
-    if (!rc) rc = batch_alloc(b, &b->d_mom, (size_t)c->g.mmax * capacity * 2 * c->np);
-    if (!rc) rc = batch_alloc(b, &b->d_C, (size_t)c->g.mmax * 2 * capacity * c->nb);
-    if (!rc && large) rc = batch_alloc(b, &b->d_LW, 2 * (size_t)capacity * c->N * c->np);
-    if (!rc && large) b->d_LQ = b->d_LW + (size_t)capacity * c->N * c->np;
+    // BPH_BATCH_CONTRACT=simt: the CUDA-core kernel for up to kBatchOwnMax
+    // positions (comparison only; the tensor-core kernel is the default)
+    const char *g = std::getenv("BPH_BATCH_CONTRACT");
+    b->own_contract = (c->np % 2 == 0) && g && g[0] == 's';
+    // last and optional: without room for the modal work array the batch runs the half-step form
+    int rc = batch_arena(b, c->modal != 0);
+    if (rc == BPH_ERR_NOMEM && c->modal && !large) rc = batch_arena(b, false);
     if (!rc) {
-        // split-K scratch of the contraction: partial sums for the widest
-        // column block (8 per CUDA-core launch, up to 64 per tensor-core
-        // launch) and arrival counters for the narrowest row groups (16 rows)
-        const size_t cols = std::max<size_t>(8, std::min<size_t>(8 * kDmmaMaxTiles, 8 * ((2 * (size_t)capacity + 7) / 8)));
-        rc = batch_alloc(b, &b->d_cpart, (size_t)kBatchSplitMax * c->g.mmax * c->nb * cols);
-        if (!rc) {
-            const size_t ncnt = (size_t)c->g.mmax * ((c->nb + 15) / 16);
-            e = cudaMalloc((void **)&b->d_ccnt, sizeof(unsigned int) * ncnt);
-            if (e == cudaSuccess) e = cudaMemsetAsync(b->d_ccnt, 0, sizeof(unsigned int) * ncnt, c->stream);
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                set_error("batch counter allocation failed: %s", cudaGetErrorString(e));
-                rc = BPH_ERR_NOMEM;
-            }
-        }
-    }
-    if (!rc) {
-        // BPH_BATCH_CONTRACT=simt: the CUDA-core kernel for up to kBatchOwnMax
-        // positions (comparison only; the tensor-core kernel is the default)
-        const char *g = std::getenv("BPH_BATCH_CONTRACT");
-        b->own_contract = (c->np % 2 == 0) && g && g[0] == 's';
-    }
-    if (!rc) {
-        const size_t tab_bytes = (2 * sizeof(void *) + sizeof(int)) * (size_t)capacity;
+        e = cudaMallocHost(&b->h_arena, 2 * table_bytes(b) + sizeof(int) * (size_t)capacity);
         for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-            e = cudaMalloc(&b->d_tab[k], tab_bytes);
-            if (e == cudaSuccess) e = cudaMallocHost(&b->h_tab[k], tab_bytes);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->tab_ev[k], cudaEventDisableTiming);
+            b->h_tab[k] = static_cast<char *>(b->h_arena) + k * table_bytes(b);
+            e = cudaEventCreateWithFlags(&b->tab_ev[k], cudaEventDisableTiming);
         }
-        if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_stat, sizeof(int) * capacity);
-        if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_stat, sizeof(int) * capacity);
+        b->h_stat = reinterpret_cast<int *>(static_cast<char *>(b->h_arena) + 2 * table_bytes(b));
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error("batch map allocation failed: %s", cudaGetErrorString(e));
             rc = BPH_ERR_NOMEM;
         }
     }
-    // last and optional: without room for it the batch runs the half-step form
-    if (!rc && c->modal && large)
-        b->d_mody = b->d_LW;
-    else if (!rc && c->modal)
-        (void)batch_alloc(b, &b->d_mody, (size_t)modal_chunk(c, capacity) * modal_size(c));
     if (!rc) {
         e = cudaMemsetAsync(b->d_P, 0, sizeof(double) * (size_t)capacity * c->N * c->nplane, c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->d_mom, 0, sizeof(double) * (size_t)c->g.mmax * capacity * 2 * c->np,
                                                   c->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(b->d_ccnt, 0, sizeof(unsigned int) * contract_counters(c), c->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "cudaMemsetAsync");
     }
     if (rc) {
@@ -618,20 +645,14 @@ int bph_batch_destroy(bph_batch_t *b) {
     if (!b) return BPH_OK;
     ::bph::DeviceScope scope_(b->c ? b->c->device : 0);
     if (b->c && b->c->stream) cudaStreamSynchronize(b->c->stream);
-    if (b->d_LW) b->d_mody = b->d_mod = nullptr;  // in the scratch
-    double *bufs[] = {b->d_P,     b->d_R,  b->d_mom,  b->d_C,     b->d_rho_stage, b->d_pot_stage, b->d_cpart,
-                      b->d_LW,    b->d_prev, b->d_cnorm, b->d_work32, b->d_mod,     b->d_modpre,    b->d_mnorm,
-                      b->d_mody};
+    if (b->d_LW) b->d_mod = nullptr;  // in the scratch
+    double *bufs[] = {b->d_rho_stage, b->d_pot_stage, b->d_prev, b->d_cnorm, b->d_work32, b->d_mod, b->d_modpre, b->d_mnorm};
     for (double *p : bufs)
         if (p) cudaFree(p);
-    if (b->d_ccnt) cudaFree(b->d_ccnt);
-    for (int k = 0; k < 2; ++k) {
-        if (b->d_tab[k]) cudaFree(b->d_tab[k]);
-        if (b->h_tab[k]) cudaFreeHost(b->h_tab[k]);
+    if (b->arena) cudaFree(b->arena);
+    if (b->h_arena) cudaFreeHost(b->h_arena);
+    for (int k = 0; k < 2; ++k)
         if (b->tab_ev[k]) cudaEventDestroy(b->tab_ev[k]);
-    }
-    if (b->d_stat) cudaFree(b->d_stat);
-    if (b->h_stat) cudaFreeHost(b->h_stat);
     if (b->h_cnorm) cudaFreeHost(b->h_cnorm);
     if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
     if (b->c) ctx_release(b->c);
