@@ -953,8 +953,12 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
     BPH_DEVICE_SCOPE(c);
     Schedule *s;
     if ((rc = get_schedule(c, nsteps, &s))) return rc;
+    // every array before anything of the warm state changes: a call that is refused leaves it
     const bool want_modal = modal_converged(c, *s, mixed);
     if ((!mixed || want_modal) && !c->d_prev && (rc = dev_alloc(c, &c->d_prev, (size_t)c->N * c->nplane))) return rc;
+    if (want_modal && !mixed && !c->d_modpre) (void)dev_alloc(c, &c->d_modpre, modal_size(c));
+    const bool modal = want_modal && (mixed || c->d_modpre);  // no room: the half-step form
+    if (mixed && !modal && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && (rc = ensure_mixed_work(c))) return rc;
     const size_t bytes = sizeof(double) * (size_t)c->ntot;
     const double *d_rho = rho;
     double *d_pot = pot;
@@ -965,9 +969,6 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
         d_pot = c->d_pot_stage;
     }
     if (cold) BPH_CUDA(cudaMemsetAsync(c->d_P, 0, sizeof(double) * (size_t)c->N * c->nplane, c->stream));
-    if (want_modal && !mixed && !c->d_modpre) (void)dev_alloc(c, &c->d_modpre, modal_size(c));
-    const bool modal = want_modal && (mixed || c->d_modpre);  // no room: the half-step form
-    if (mixed && !modal && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && (rc = ensure_mixed_work(c))) return rc;
     BPH_CUDA(launch_fft_fwd_rho(c, d_rho));
     BPH_CUDA(launch_green_contract(c));  // also writes the Dirichlet slots
     const int pairs = modal ? c->N * modal_groups(c) : c->N;  // norm pairs of a cycle

@@ -959,15 +959,16 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
     const size_t ibytes = sizeof(double) * (size_t)c->N * c->nplane;  // one instance's slot arrays
     int top = 0;  // instances 0..top-1 hold every position's norms
     for (int i = 0; i < n; ++i) top = std::max(top, inst[i] + 1);
+    // every array before anything of the warm states changes: a call that is refused leaves them
     if ((rc = batch_reserve_converged(b, cv.mixed))) return rc;
-    if (cv.cold)  // before the Dirichlet slots
-        for (int i = 0; i < n; ++i)
-            BPH_CUDA(cudaMemsetAsync(b->d_P + (size_t)inst[i] * c->N * c->nplane, 0, ibytes, c->stream));
-    if ((rc = batch_prologue(b, n, d_in, d_map, per_pos))) return rc;
     const bool modal = modal_converged(c, *s, cv.mixed) && b->d_mnorm;
     if (cv.mixed && !modal && c->mixed_kind == BPH_MIXED_ADI_GLOBAL &&
         (rc = batch_work32(b, 2ull * b->cap * c->N * c->np)))
         return rc;
+    if (cv.cold)  // before the Dirichlet slots
+        for (int i = 0; i < n; ++i)
+            BPH_CUDA(cudaMemsetAsync(b->d_P + (size_t)inst[i] * c->N * c->nplane, 0, ibytes, c->stream));
+    if ((rc = batch_prologue(b, n, d_in, d_map, per_pos))) return rc;
     const int mpairs = modal ? c->N * modal_groups(c) : 0;  // norm pairs per position
     if (modal) BPH_CUDA(launch_modal_begin(c, cv.cold, b->d_P, b->d_R, b->d_mod, b->d_prev, n, d_map));
     std::vector<double> prev_upd((size_t)n, INFINITY);

@@ -45,3 +45,69 @@ def test_large_slots_keep_no_array_beside_their_scratch(bph, monkeypatch, g):
     assert used["modal"][1] == used["half"][1]
     for a, h in zip(out["modal"], out["half"]):
         assert rel_l2(a, h) <= 1e-12
+
+
+class _Filled:
+    """All but `room` bytes of the device's free memory taken."""
+
+    def __init__(self, room):
+        import torch
+
+        self.torch, self.held = torch, []
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        for unit in (1 << 30, 1 << 26, 1 << 22):
+            free = torch.cuda.mem_get_info()[0]
+            n = max(free - room, 0) // unit
+            if n:
+                self.held.append(torch.empty(n * unit, dtype=torch.uint8, device="cuda"))
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.torch.cuda.synchronize()
+        self.held.clear()
+        self.torch.cuda.empty_cache()
+
+
+def _host(rho):
+    import torch
+
+    return torch.from_numpy(np.ascontiguousarray(rho.ravel(order="F"))).cuda()
+
+
+MB = 1 << 20
+
+
+def test_refused_converged_solve_leaves_the_state(bph, monkeypatch):
+    """A cold mixed solve for whose FP32 work arrays there is no room is refused before it clears the
+    potential that the next warm solve starts from."""
+    g = (202, 152, 128, 1.0 / 198.0, 2, 4)  # work arrays: 61 MB a context, 4 x 31 MB for a batch of 2
+    monkeypatch.setenv("BPH_ADI_MODAL", "0")
+    rhos = [np.asfortranarray(smooth_density(*g[:5], seed=80 + i)) for i in range(2)]
+    dev = [_host(r) for r in rhos]
+    out = {}
+    for refused in (False, True):
+        s = bph.PotentialSolver(*g)
+        b = bph.Batch(s, capacity=2)
+        pot, pots = dev[0].clone(), [d.clone() for d in dev]
+        s.potential_solver_device(dev[0], pot, 0)
+        b.solve_device(dev, pots, 0)
+        s.solve_nsteps_device(dev[0], pot, 10, False)  # the cycle's schedule, ahead
+        if refused:
+            with _Filled(24 * MB):
+                with pytest.raises(bph.BphError) as err:
+                    s.solve_converged_device(dev[1], pot, 10, True, 1e-9, 5, mixed=True)
+                assert err.value.code == bph.BPH_ERR_NOMEM
+                with pytest.raises(bph.BphError) as err:
+                    b.solve_converged_device(dev[::-1], pots, 10, True, 1e-9, 5, mixed=True)
+                assert err.value.code == bph.BPH_ERR_NOMEM
+        s.potential_solver_device(dev[1], pot, 2)
+        b.solve_device(dev[::-1], pots, 2)
+        s.synchronize()
+        out[refused] = [p.cpu().numpy() for p in [pot] + pots]
+        b.close()
+        s.close()
+    for a, w in zip(out[True], out[False]):
+        assert np.array_equal(a, w)
