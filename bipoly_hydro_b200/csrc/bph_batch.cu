@@ -886,20 +886,21 @@ static int batch_work32(bph_batch *b, size_t need) {
     return rc;
 }
 
-int batch_reserve_converged(bph_batch *b, bool mixed) {
+int batch_reserve_converged(bph_batch *b, bool mixed, int nsteps) {
     bph_ctx *c = b->c;
     int rc;
     if (!b->d_cnorm && (rc = batch_alloc(b, &b->d_cnorm, 2ull * b->cap * c->N))) return rc;
     if (!b->h_cnorm) BPH_CUDA(cudaMallocHost((void **)&b->h_cnorm, sizeof(double) * 2 * (size_t)b->cap * c->N));
-    // modal form: modal potential, residual and partial norms; without room for them the other
-    // forms run
-    const bool want_modal = c->modal && (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
+    // modal form: modal potential, residual and partial norms, and for the FP64 form the potential
+    // before a cycle's last step; without room for them the other forms run
+    const bool want_modal = c->modal && !(c->adi_warp && nsteps <= 7) &&
+                            (!mixed || c->mixed_kind == BPH_MIXED_ADI_GLOBAL);
+    const size_t each = (size_t)b->cap * modal_size(c);
     if (want_modal && !b->d_mnorm) {
         const size_t norms = 2ull * b->cap * c->N * modal_groups(c);
-        const size_t each = (size_t)b->cap * modal_size(c);
         const bool had_prev = b->d_prev != nullptr;
         if ((had_prev || !batch_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)) &&
-            (b->d_LW || !batch_alloc(b, &b->d_mod, each)) && !batch_alloc(b, &b->d_modpre, each) &&
+            (b->d_LW || !batch_alloc(b, &b->d_mod, each)) &&
             cudaMallocHost((void **)&b->h_mnorm, sizeof(double) * norms) == cudaSuccess)
             (void)batch_alloc(b, &b->d_mnorm, norms);
         if (b->d_LW) b->d_mod = b->d_mnorm ? b->d_LW : nullptr;
@@ -914,10 +915,10 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
                 p = nullptr;
             };
             give_back(b->d_mod, each);  // (nullptr where it is in the scratch)
-            give_back(b->d_modpre, each);
             if (!had_prev) give_back(b->d_prev, (size_t)b->cap * c->N * c->nplane);
         }
     }
+    if (want_modal && !mixed && b->d_mnorm && !b->d_modpre) (void)batch_alloc(b, &b->d_modpre, each);
     // FP64 on the grid-wide kernels: the previous cycle's slot arrays (the segmented kernel
     // forms the update while writing back)
     if (!mixed && !c->adi_seg && !b->d_prev &&
@@ -926,7 +927,7 @@ int batch_reserve_converged(bph_batch *b, bool mixed) {
     // FP32 work arrays of the refinement: the grid-wide cycle keeps r, delta and two right-hand
     // sides per position; the warp-cooperative one the rounded residual per position
     size_t need = 0;
-    if (mixed && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && !(b->d_mnorm && !c->adi_warp)) need = 2ull * b->cap * c->N * c->np;
+    if (mixed && c->mixed_kind == BPH_MIXED_ADI_GLOBAL && !(want_modal && b->d_mnorm)) need = 2ull * b->cap * c->N * c->np;
     if (mixed && c->mixed_kind == BPH_MIXED_ADI_WARP)
         need = ((size_t)b->cap * c->N * c->np + 1) / 2;
     return batch_work32(b, need);
@@ -960,8 +961,8 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
     int top = 0;  // instances 0..top-1 hold every position's norms
     for (int i = 0; i < n; ++i) top = std::max(top, inst[i] + 1);
     // every array before anything of the warm states changes: a call that is refused leaves them
-    if ((rc = batch_reserve_converged(b, cv.mixed))) return rc;
-    const bool modal = modal_converged(c, *s, cv.mixed) && b->d_mnorm;
+    if ((rc = batch_reserve_converged(b, cv.mixed, cv.nsteps))) return rc;
+    const bool modal = modal_converged(c, *s, cv.mixed) && b->d_mnorm && (cv.mixed || b->d_modpre);
     if (cv.mixed && !modal && c->mixed_kind == BPH_MIXED_ADI_GLOBAL &&
         (rc = batch_work32(b, 2ull * b->cap * c->N * c->np)))
         return rc;

@@ -357,10 +357,10 @@ struct BatchConv {
     bool want_resid = false;
     bool report_divergence = true;  // false: per-position status reports bad densities
 };
-// Norm buffers (FP64: the previous-cycle slot arrays; mixed on grid-wide
-// kernels: the FP32 work arrays) of converged batched calls, allocated ahead
-// of the first one.
-int batch_reserve_converged(bph_batch *b, bool mixed);
+// Arrays of converged batched calls with cycles of nsteps (norms; the modal
+// potential, residual and, FP64, earlier potential, or the previous cycle's
+// slot arrays or FP32 work arrays), allocated ahead of the first one.
+int batch_reserve_converged(bph_batch *b, bool mixed, int nsteps);
 int batch_solve_core(bph_batch *b, int n, const int *instances, const double *const *rho, double *const *pot,
                      bool warm, bool on_device, int *pos_status, BatchConv *conv = nullptr);
 // Raises the dynamic shared memory limit of kernel fn on the current device

@@ -222,7 +222,7 @@ int bph_server_set_converged(bph_server_t *s, int nsteps, double tol, int max_cy
     std::lock_guard<std::mutex> lk(s->mu);
     if (nsteps > 0) {
         // buffers first: a batch the worker takes after the mode changes finds them
-        const int rc = batch_reserve_converged(s->batch, mixed != 0);
+        const int rc = batch_reserve_converged(s->batch, mixed != 0, nsteps);
         if (rc) return rc;
     }
     s->conv_nsteps = nsteps;

@@ -111,3 +111,34 @@ def test_refused_converged_solve_leaves_the_state(bph, monkeypatch):
         s.close()
     for a, w in zip(out[True], out[False]):
         assert np.array_equal(a, w)
+
+
+def test_mixed_batches_hold_no_fp64_array(bph):
+    """Mixed converged solves in the vertical eigenbasis keep the modal potential (and, for slots
+    without the grid-wide scratch, the residual); the FP64 form's earlier potential is allocated by
+    the first FP64 solve.  Both forms work in either order."""
+    for g, arrays in ((LARGE[0], 1), ((40, 30, 64, 1.0 / 36.0, 2, 16), 2)):
+        rhos = [np.asfortranarray(smooth_density(*g[:5], seed=90 + i)) for i in range(3)]
+        out = {}
+        for first in ("mixed", "fp64"):
+            s = bph.PotentialSolver(*g)
+            s.set_mixed_adi(MIXED_ADI_GLOBAL)
+            b = bph.Batch(s, capacity=3)
+            b.solve(rhos, 0)  # the host arrays' staging
+            before = b.device_bytes
+            pots, sizes = {}, {}
+            for form in ("mixed", "fp64") if first == "mixed" else ("fp64", "mixed"):
+                pots[form], _ = b.solve_converged(rhos, 10, True, 1e-11, 60, mixed=form == "mixed")
+                sizes[form] = b.device_bytes - before
+            out[first] = pots
+            slot_arrays = 3 * 8 * g[0] * g[1] * g[2]  # a modal array is smaller than a slot array
+            if first == "mixed":
+                assert sizes["mixed"] <= arrays * slot_arrays + MB
+                assert sizes["fp64"] <= (arrays + 1) * slot_arrays + MB
+            b.close()
+            s.close()
+        for form in ("mixed", "fp64"):
+            for a, w in zip(out["mixed"][form], out["fp64"][form]):
+                assert np.array_equal(a, w)
+        for a, w in zip(out["mixed"]["mixed"], out["mixed"]["fp64"]):
+            assert rel_l2(a, w) <= 1e-9  # tolerance 1e-11 of an update, each cycle reducing it
