@@ -663,10 +663,24 @@ int solve_device(bph_ctx *c, const double *d_rho, double *d_pot, const Schedule 
     return BPH_OK;
 }
 
+// An array that a call cannot do without: the FP64 converged form's optional
+// one gives way to it (its loop's graph, which holds the address, with it).
+template <typename T>
+int must_alloc(bph_ctx *c, T **p, size_t count) {
+    const int rc = dev_alloc(c, p, count);
+    if (rc != BPH_ERR_NOMEM || !c->d_modpre || c->d_modpre == c->d_W2) return rc;
+    cudaStreamSynchronize(c->stream);
+    conv_graph_drop(c->conv[0]);
+    dev_free(c->d_modpre);
+    c->d_modpre = nullptr;
+    c->bytes -= sizeof(double) * modal_size(c);
+    return dev_alloc(c, p, count);
+}
+
 int ensure_staging(bph_ctx *c) {
     int rc;
-    if (!c->d_rho_stage && (rc = dev_alloc(c, &c->d_rho_stage, (size_t)c->ntot))) return rc;
-    if (!c->d_pot_stage && (rc = dev_alloc(c, &c->d_pot_stage, (size_t)c->ntot))) return rc;
+    if (!c->d_rho_stage && (rc = must_alloc(c, &c->d_rho_stage, (size_t)c->ntot))) return rc;
+    if (!c->d_pot_stage && (rc = must_alloc(c, &c->d_pot_stage, (size_t)c->ntot))) return rc;
     return BPH_OK;
 }
 
@@ -920,7 +934,7 @@ namespace bph {
 // Sum of the per-slot (num, den) pairs a norm kernel left in c->d_red.
 int ensure_mixed_work(bph_ctx *c) {
     if (c->d_work32) return BPH_OK;
-    return dev_alloc(c, &c->d_work32, (size_t)c->N * 4 * (size_t)c->np);
+    return must_alloc(c, &c->d_work32, (size_t)c->N * 4 * (size_t)c->np);
 }
 
 static double host_ratio(const std::vector<double> &h, int N) {
@@ -1058,7 +1072,7 @@ int bph_potential_solver_phieff(bph_ctx_t *c, const double *rho, double *pot, do
     if ((rc = get_schedule(c, warm ? 5 : 20, &s))) return rc;
     if (on_device) return solve_device(c, rho, pot, *s, !warm, phieff, omega_frame);
     if ((rc = ensure_staging(c))) return rc;
-    if (!c->d_phieff_stage && (rc = dev_alloc(c, &c->d_phieff_stage, (size_t)c->ntot))) return rc;
+    if (!c->d_phieff_stage && (rc = must_alloc(c, &c->d_phieff_stage, (size_t)c->ntot))) return rc;
     const size_t bytes = sizeof(double) * (size_t)c->ntot;
     BPH_CUDA(cudaMemcpyAsync(c->d_rho_stage, rho, bytes, cudaMemcpyHostToDevice, c->stream));
     if ((rc = solve_device(c, c->d_rho_stage, c->d_pot_stage, *s, !warm, c->d_phieff_stage, omega_frame))) return rc;

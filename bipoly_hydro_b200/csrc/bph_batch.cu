@@ -555,6 +555,37 @@ int batch_arena(bph_batch *b, bool modal) {
     return BPH_OK;
 }
 
+void batch_give_back(bph_batch *b, double *&p, size_t count) {
+    if (!p) return;
+    cudaFree(p);
+    b->bytes -= sizeof(double) * count;
+    p = nullptr;
+}
+
+// Frees what converged solves hold only to run in the eigenbasis (they ask for
+// it anew); true if there was any.
+bool batch_drop_modal(bph_batch *b) {
+    const bph_ctx *c = b->c;
+    const bool any = b->d_mnorm || b->d_modpre;
+    if (any) cudaStreamSynchronize(c->stream);
+    const size_t each = (size_t)b->cap * modal_size(c);
+    if (b->d_LW) b->d_mod = nullptr;  // in the scratch
+    batch_give_back(b, b->d_mod, each);
+    batch_give_back(b, b->d_modpre, each);
+    batch_give_back(b, b->d_mnorm, 2ull * b->cap * c->N * modal_groups(c));
+    if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
+    b->h_mnorm = nullptr;
+    // the grid-wide half-steps' converged form keeps its potential there
+    if (any && c->adi_seg) batch_give_back(b, b->d_prev, (size_t)b->cap * c->N * c->nplane);
+    return any;
+}
+
+// An array that a call cannot do without: what only speeds up other calls gives way to it.
+int batch_must_alloc(bph_batch *b, double **p, size_t count) {
+    const int rc = batch_alloc(b, p, count);
+    return rc == BPH_ERR_NOMEM && batch_drop_modal(b) ? batch_alloc(b, p, count) : rc;
+}
+
 }  // namespace
 
 // Schedules are shared with the single-solve path (bph_api.cu).
@@ -754,8 +785,13 @@ int batch_solve_core(bph_batch *b, int n, const int *instances, const double *co
                 b->d_pot_stage = nullptr;
             }
             b->stage_cap = 0;
-            if ((rc = batch_alloc(b, &b->d_rho_stage, (size_t)n * c->ntot))) return rc;
-            if ((rc = batch_alloc(b, &b->d_pot_stage, (size_t)n * c->ntot))) return rc;
+            if ((rc = batch_must_alloc(b, &b->d_rho_stage, (size_t)n * c->ntot))) return rc;
+            if ((rc = batch_must_alloc(b, &b->d_pot_stage, (size_t)n * c->ntot))) {
+                cudaFree(b->d_rho_stage);  // both or none: its size is not on record yet
+                b->bytes -= sizeof(double) * (size_t)n * c->ntot;
+                b->d_rho_stage = nullptr;
+                return rc;
+            }
             b->stage_cap = n;
         }
         for (int i = 0; i < n; ++i) {
@@ -881,7 +917,7 @@ static int batch_work32(bph_batch *b, size_t need) {
         b->d_work32 = nullptr;
         b->work32_doubles = 0;
     }
-    const int rc = batch_alloc(b, &b->d_work32, need);
+    const int rc = batch_must_alloc(b, &b->d_work32, need);
     if (!rc) b->work32_doubles = need;
     return rc;
 }
@@ -889,7 +925,7 @@ static int batch_work32(bph_batch *b, size_t need) {
 int batch_reserve_converged(bph_batch *b, bool mixed, int nsteps) {
     bph_ctx *c = b->c;
     int rc;
-    if (!b->d_cnorm && (rc = batch_alloc(b, &b->d_cnorm, 2ull * b->cap * c->N))) return rc;
+    if (!b->d_cnorm && (rc = batch_must_alloc(b, &b->d_cnorm, 2ull * b->cap * c->N))) return rc;
     if (!b->h_cnorm) BPH_CUDA(cudaMallocHost((void **)&b->h_cnorm, sizeof(double) * 2 * (size_t)b->cap * c->N));
     // modal form: modal potential, residual and partial norms, and for the FP64 form the potential
     // before a cycle's last step; without room for them the other forms run
@@ -906,23 +942,15 @@ int batch_reserve_converged(bph_batch *b, bool mixed, int nsteps) {
         if (b->d_LW) b->d_mod = b->d_mnorm ? b->d_LW : nullptr;
         if (!b->d_mnorm) {  // give back what was had: the other forms need the room
             cudaGetLastError();
-            if (b->h_mnorm) cudaFreeHost(b->h_mnorm);
-            b->h_mnorm = nullptr;
-            auto give_back = [&](double *&p, size_t count) {
-                if (!p) return;
-                cudaFree(p);
-                b->bytes -= sizeof(double) * count;
-                p = nullptr;
-            };
-            give_back(b->d_mod, each);  // (nullptr where it is in the scratch)
-            if (!had_prev) give_back(b->d_prev, (size_t)b->cap * c->N * c->nplane);
+            batch_drop_modal(b);
+            if (!had_prev) batch_give_back(b, b->d_prev, (size_t)b->cap * c->N * c->nplane);
         }
     }
     if (want_modal && !mixed && b->d_mnorm && !b->d_modpre) (void)batch_alloc(b, &b->d_modpre, each);
     // FP64 on the grid-wide kernels: the previous cycle's slot arrays (the segmented kernel
     // forms the update while writing back)
     if (!mixed && !c->adi_seg && !b->d_prev &&
-        (rc = batch_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)))
+        (rc = batch_must_alloc(b, &b->d_prev, (size_t)b->cap * c->N * c->nplane)))
         return rc;
     // FP32 work arrays of the refinement: the grid-wide cycle keeps r, delta and two right-hand
     // sides per position; the warp-cooperative one the rounded residual per position

@@ -196,11 +196,13 @@ int conv_loop_device(bph_ctx *c, Schedule &s, bool mixed, double tol, int max_cy
     return BPH_OK;
 }
 
+void conv_graph_drop(ConvGraph &cg) {
+    if (cg.exec) cudaGraphExecDestroy(cg.exec);
+    cg = ConvGraph();
+}
+
 void conv_graphs_free(bph_ctx *c) {
-    for (ConvGraph &cg : c->conv) {
-        if (cg.exec) cudaGraphExecDestroy(cg.exec);
-        cg = ConvGraph();
-    }
+    for (ConvGraph &cg : c->conv) conv_graph_drop(cg);
     if (c->d_conv) cudaFree(c->d_conv);
     c->d_conv = nullptr;
 }

@@ -343,6 +343,7 @@ int adi_configure(bph_ctx *c);
 // c->d_conv.  conv_graphs_free releases the graphs and the state.
 int conv_loop_device(bph_ctx *c, Schedule &s, bool mixed, double tol, int max_cycles);
 void conv_graphs_free(bph_ctx *c);
+void conv_graph_drop(ConvGraph &cg);  // rebuilt by its next use
 // Batched solve of batch positions 0..n-1 (bph_batch.cu); instances may be
 // nullptr (position i = instance i).  With pos_status (per-position
 // BPH_OK / BPH_ERR_NONFINITE) or host arrays the call is synchronous.

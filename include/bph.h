@@ -240,8 +240,9 @@ int bph_server_create(bph_ctx_t *ctx, int max_clients, size_t mem_cap_bytes, int
  * solve (bph_batch_solve_converged with nsteps, tol, max_cycles; mixed != 0:
  * FP32 refinement on the FP64 defect; first requests of a client cold, later
  * ones from its last potential).  nsteps = 0 returns to the drop-in solve.
- * Best called before submitting; FP64 mode reserves one more slot array per
- * resident client. */
+ * Best called before submitting; it reserves up to three more slot arrays per
+ * resident client (two in mixed mode) while they fit beside what the requests
+ * themselves need, and runs a form that needs fewer where they do not. */
 int bph_server_set_converged(bph_server_t *server, int nsteps, double tol, int max_cycles, int mixed);
 /* Resident clients this server admits. */
 int bph_server_capacity(const bph_server_t *server);

@@ -142,3 +142,82 @@ def test_mixed_batches_hold_no_fp64_array(bph):
                 assert np.array_equal(a, w)
         for a, w in zip(out["mixed"]["mixed"], out["mixed"]["fp64"]):
             assert rel_l2(a, w) <= 1e-9  # tolerance 1e-11 of an update, each cycle reducing it
+
+
+def test_optional_arrays_give_way(bph):
+    """What a converged solve holds only to run in the vertical eigenbasis does not cost a later call
+    its staging arrays: with room for these only in its place the host-array calls succeed, and the
+    converged solve after them."""
+    g = (101, 75, 128, 1.0 / 97.0, 2, 8)  # batch of 16: staging 248 MB, optional arrays 3 x 115 MB
+    big = (250, 40, 512, 1.0 / 246.0, 2, 8)  # context: staging 2 x 41 MB, optional array 39 MB
+    rho, many = smooth_density(*big[:5], seed=100), [smooth_density(*g[:5], seed=101 + i) for i in range(16)]
+    out = {}
+    for scarce in (False, True):
+        s, one = bph.PotentialSolver(*g), bph.PotentialSolver(*big)
+        b = bph.Batch(s, capacity=16)
+        dev, pots = [_host(r) for r in many], [_host(r) for r in many]
+        d, pot = _host(rho), _host(rho)
+        b.solve_converged_device(dev, pots, 10, True, 1e-9, 60)
+        one.solve_converged_device(d, pot, 10, True, 1e-9, 60)
+        s.synchronize()
+        one.synchronize()
+        got = []
+        if scarce:
+            with _Filled(100 * MB):
+                got += b.solve(many, 2)
+                got += b.solve_converged(many, 10, False, 1e-11, 60)[0]
+            with _Filled(60 * MB):
+                got.append(one.potential_solver(rho, 2))
+                got.append(one.solve_converged(rho, 10, False, 1e-11, 60)[0])
+        else:
+            got += b.solve(many, 2) + b.solve_converged(many, 10, False, 1e-11, 60)[0]
+            got += [one.potential_solver(rho, 2), one.solve_converged(rho, 10, False, 1e-11, 60)[0]]
+        got += b.solve_converged(many, 10, True, 1e-11, 60)[0]
+        got.append(one.solve_converged(rho, 10, True, 1e-11, 60)[0])
+        out[scarce] = got
+        b.close()
+        s.close()
+        one.close()
+    for a, w in zip(out[True], out[False]):
+        assert rel_l2(a, w) <= 1e-12
+
+
+@pytest.mark.parametrize("room", [40, 60, 90, 130, 200])
+def test_every_form_without_room_for_the_next(oracle_mod, bph, room):
+    """Batches, schedules and converged solves created with little room left run whichever form's
+    arrays fit, and give the oracle's potential; refused calls name the reason."""
+    g = (101, 75, 128, 1.0 / 97.0, 2, 8)  # a slot array 7.6 MB; twelve steps' factors 18 MB, modal ones 8 MB more
+    o = oracle_mod.Oracle(*g)
+    rho = smooth_density(*g[:5], seed=120)
+    s = bph.PotentialSolver(*g)
+    warm = bph.PotentialSolver(*g)  # every kernel and the staging, once
+    warm.potential_solver(rho, 0)
+    warm.solve_nsteps(rho, 12, False)
+    warm.solve_converged(rho, 10, True, 1e-9, 60)
+    wb = bph.Batch(warm, capacity=2)
+    wb.solve([rho] * 2, 0)
+    wb.solve_converged([rho] * 2, 10, True, 1e-9, 60)
+    wb.close()
+    warm.close()
+    s.potential_solver(rho, 0)
+    want = o.potential_solver(rho, 0)
+    refused = 0
+    with _Filled(room * MB):
+        for call in ("steps", "converged", "batch"):
+            try:
+                if call == "steps":
+                    assert rel_l2(s.solve_nsteps(rho, 12, True), o.solve_nsteps(rho, 12, True)) <= 1e-12
+                elif call == "converged":
+                    s.solve_converged(rho, 10, True, 1e-11, 60)
+                else:
+                    b = bph.Batch(s, capacity=2)
+                    assert all(rel_l2(p, want) <= 1e-12 for p in b.solve([rho] * 2, 0))
+                    b.solve_converged([rho] * 2, 10, True, 1e-11, 60)
+                    b.close()
+            except bph.BphError as err:
+                assert err.code == bph.BPH_ERR_NOMEM
+                refused += 1
+    assert rel_l2(s.potential_solver(rho, 0), want) <= 1e-12
+    assert refused < 3 or room < 60
+    s.close()
+    o.close()
