@@ -114,6 +114,10 @@ struct ConvGraph {
     int kind = -1;
 };
 
+// Where a context's potential before a converged cycle's last step is: the grid-wide half-steps'
+// scratch d_W2, the end of d_prev's allocation, an allocation of its own.
+enum { kModpreNone = 0, kModpreScratch = 1, kModprePrev = 2, kModpreOwn = 3 };
+
 }  // namespace bph
 
 struct bph_ctx {
@@ -224,9 +228,9 @@ struct bph_ctx {
     int *d_modtab = nullptr;           // split form: signed heights of (a1, a2)
     double *d_modE = nullptr;          // packed fragments of E, then of E^T (one allocation with the arrays below)
     double *d_modlam = nullptr;        // [nz] gamma lambda_q
-    double *d_modY = nullptr;          // [N][nr][nz, even] modal residual / update
-    double *d_modpre = nullptr;        // converged form: potential before a cycle's last step (on first use; grid-wide
-                                       // half-steps: d_W2, and d_modY is d_W)
+    double *d_modY = nullptr;          // [N][nr][nz, even] modal residual / update (grid-wide half-steps: d_W)
+    double *d_modpre = nullptr;        // converged form: potential before a cycle's last step
+    int modpre_at = 0;                 // where it is: kModpre*
     double *d_modnorm = nullptr;       // [N][modal_groups][2] partial update norms of a cycle
     double *d_scf = nullptr;           // SCF-step mass partials and scale (bph_scf.cu)
     void *noalloc_scratch = nullptr;   // device address of the allocation-free contraction's scratch array

@@ -1005,7 +1005,10 @@ int modal_configure(bph_ctx *c) {
     c->d_modnorm = c->d_modlam + lams;
     c->d_modtab = reinterpret_cast<int *>(c->d_modnorm + norms);
     c->d_modY = scratch ? c->d_W : c->d_modnorm + norms + tabs;
-    if (scratch) c->d_modpre = c->d_W2;
+    if (scratch) {
+        c->d_modpre = c->d_W2;
+        c->modpre_at = kModpreScratch;
+    }
     c->bytes += sizeof(double) * all;
     pack.insert(pack.end(), lam.begin(), lam.end());
     BPH_CUDA(cudaMemcpyAsync(c->d_modE, pack.data(), sizeof(double) * pack.size(), cudaMemcpyHostToDevice, c->stream));
