@@ -74,7 +74,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 // memory (row j of X^T is column j of X; ldk = nzp + 4) and A (nzp x nzp)
 // is row-major [nzp][lda] (lda = nzp + 4).  Warp tiles of 32 rows x 16
 // columns (2 x 2 m16n8k8 tiles, three split-TF32 products each per k-step,
-// every split fragment used twice).  The column pairs are taken in blocks of
+// every split fragment used twice), or of 48 x 32.  The column pairs are taken in blocks of
 // cpb, at most kTilesPerWarp warp tiles per warp: all products of a block
 // are formed in registers, then, after a barrier, written over it.  With both
 // strides 4 modulo 32 words the fragment loads (A row g, column t; X^T row g,
@@ -92,10 +92,7 @@ __device__ __forceinline__ void tc_transform(const float *A, int lda, float *Xt,
     const int cp = nrp / 16;
     for (int cp0 = 0; cp0 < cp; cp0 += cpb) {
         const int ncp = min(cpb, cp - cp0), tiles = (nzp / 32) * ncp;
-        // Rows in units of 48 and an even number of column pairs: one 48 x 32 tile per warp, which
-        // splits 20 operand values for 36 products where three 32 x 16 tiles split 36.
-        const int half = ncp / 2;
-        if (nzp % 48 == 0 && ncp % 2 == 0 && (nzp / 48) * half <= kWarpsD) {
+        if (direct::wide_block(nzp, ncp)) {
             float acc[3][4][4];
 #pragma unroll
             for (int m = 0; m < 3; ++m)
@@ -103,8 +100,8 @@ __device__ __forceinline__ void tc_transform(const float *A, int lda, float *Xt,
                 for (int n = 0; n < 4; ++n)
 #pragma unroll
                     for (int v = 0; v < 4; ++v) acc[m][n][v] = 0.f;
-            const bool on = warp < (nzp / 48) * half;
-            const int i0 = on ? 48 * (warp / half) : 0, c0 = 16 * cp0 + 32 * (warp % half);
+            int i0, c0;
+            const bool on = direct::wide_tile(warp, nzp, cp0, ncp, i0, c0);
             if (on) {
                 for (int k0 = 0; k0 < nzp; k0 += 8) {
                     uint32_t bh[4][2], bl[4][2];
@@ -326,11 +323,11 @@ __global__ void __launch_bounds__(kDThreads, 2) k_defect_direct(DirectArgs a) {
     // the deltas of four rows are one 16-byte word of the column.
     double sd = 0.0, sp = 0.0;
     {
-        constexpr int kUpd = 12;
-        const int nchunk = (nr + 31) / 32, nband = (kWarpsD / nchunk > 1) ? kWarpsD / nchunk : 1;
-        const int band = ((nz + nband - 1) / nband + kUpd - 1) / kUpd * kUpd;
-        for (int it = warp; it < nchunk * nband; it += kWarpsD) {
-            const int j = (it % nchunk) * 32 + lane, k0 = (it / nchunk) * band, k1 = min(nz, k0 + band);
+        constexpr int kUpd = direct::kUpd;
+        for (int it = warp; it < direct::sweep_items(nr); it += kWarpsD) {
+            int jc, k0, k1;
+            direct::update_item(it, nr, nz, jc, k0, k1);
+            const int j = jc + lane;
             if (j >= nr) continue;
             const float *dcol = Xt + j * ldk;
             double *pcol = Pg + numr + 1 + j;

@@ -75,6 +75,20 @@ BPH_DIRECT_HD void warp_tile(int tile, int cp0, int ncp, int &i0, int &c0) {
     i0 = 32 * (tile / ncp);
     c0 = 16 * (cp0 + tile % ncp);
 }
+// Where the rows come in units of 48 and the block has an even number of
+// column pairs, it is cut into 48 x 32 tiles instead, at most one a warp: a
+// tile splits 20 operand values for 36 products where three 32 x 16 tiles
+// split 36.  wide_tile is false for a warp without one.
+BPH_DIRECT_HD bool wide_block(int nzp, int ncp) {
+    return nzp % 48 == 0 && ncp % 2 == 0 && (nzp / 48) * (ncp / 2) <= kWarps;
+}
+BPH_DIRECT_HD bool wide_tile(int warp, int nzp, int cp0, int ncp, int &i0, int &c0) {
+    const int half = ncp / 2;
+    const bool on = warp < (nzp / 48) * half;
+    i0 = on ? 48 * (warp / half) : 0;
+    c0 = 16 * cp0 + 32 * (warp % half);
+    return on;
+}
 // m16n8k8 fragments of lane (g = lane / 4, t = lane % 4) in the warp tile
 // (i0, c0), sub-tile (m, n), k-step k0, as word offsets:
 //   A [nzp][lda]: a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4);
@@ -101,6 +115,19 @@ BPH_DIRECT_HD void sweep_item(int it, int nr, int nz, int &jc, int &k0, int &k1)
     const int nchunk = (nr + 31) / 32;
     const int nband = (kWarps / nchunk > 1) ? kWarps / nchunk : 1;
     const int band_rows = (nz + nband - 1) / nband;
+    jc = (it % nchunk) * 32;
+    k0 = (it / nchunk) * band_rows;
+    k1 = (k0 + band_rows < nz) ? k0 + band_rows : nz;
+}
+
+// Update sweep item `it` of kWarps warps, as above with bands of whole groups
+// of kUpd rows (each group's loads before its stores; a column's deltas are
+// read as 16-byte words, four rows each).
+constexpr int kUpd = 12;
+BPH_DIRECT_HD void update_item(int it, int nr, int nz, int &jc, int &k0, int &k1) {
+    const int nchunk = (nr + 31) / 32;
+    const int nband = (kWarps / nchunk > 1) ? kWarps / nchunk : 1;
+    const int band_rows = ((nz + nband - 1) / nband + kUpd - 1) / kUpd * kUpd;
     jc = (it % nchunk) * 32;
     k0 = (it / nchunk) * band_rows;
     k1 = (k0 + band_rows < nz) ? k0 + band_rows : nz;
