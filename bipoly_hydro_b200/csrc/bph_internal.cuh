@@ -223,6 +223,7 @@ struct bph_ctx {
     int modal_min = 0;                 // steps from which a solve's schedule does, and a batch's (modal_rule)
     int modal_min_batch = 0;
     int modal_seg = 0;                 // radii per segment of a radial line
+    int modal_resident[3] = {0, 0, 0};  // resident blocks of its transforms and radial kernel on the device
     int modal_p1 = 0;                  // first factor of the split transforms (0: dense)
     int modal_beta1 = 0;               // multiplier of its angles
     int *d_modtab = nullptr;           // split form: signed heights of (a1, a2)

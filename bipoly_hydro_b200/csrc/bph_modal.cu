@@ -69,6 +69,7 @@ struct ModalArgs {
     int inst0, nslots, ntile, groups;
     int numr, numz, nr, nz, ldq, N, isym, mtiles, ksteps;
     int nsteps, source, add;
+    unsigned ahead;          // blocks of the kernel that the device holds at a time
     int lagged;              // converged form: the refinement's half-step order (nsteps counts its radial solves)
     double gamma;
     // split transforms (p1 > 0)
@@ -88,8 +89,6 @@ __device__ __forceinline__ void dmma(double *c, const double2 &a01, const double
         : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
         : "d"(a01.x), "d"(a01.y), "d"(a23.x), "d"(a23.y), "d"(b0), "d"(b1));
 }
-
-constexpr unsigned kAhead = 2 * 148;  // resident blocks of the split transforms and of short radial lines
 
 // Rows of 8 NT columns, padded to 4 modulo the 16 eight-byte banks: the four
 // rows of a B fragment then fall into different banks.
@@ -398,8 +397,8 @@ __global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
         rows[i] = (abs(a.tab[a1 * h2 + at]) - 1) * ld;
     }
     source_tile<NT>(a, ti, sx);
-    if (blockIdx.x + kAhead < gridDim.x) {
-        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + kAhead);
+    if (blockIdx.x + a.ahead < gridDim.x) {
+        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + a.ahead);
         const int jn = tn.tile * cols, count = min(cols, nr - jn);
         const long long at = tn.inst * a.N + tn.slot;
         if (a.source != kPotential) prefetch_rows(a.R + at * nr * nz + jn, nr, nz, count);
@@ -463,8 +462,8 @@ __global__ void __launch_bounds__(256, 2) k_modal_inv_split(ModalArgs a) {
             for (int q = lane; q < nz; q += 32) row[q] = 0.0;
         }
     }
-    if (blockIdx.x + kAhead < gridDim.x) {
-        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + kAhead);
+    if (blockIdx.x + a.ahead < gridDim.x) {
+        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + a.ahead);
         const int jn = tn.tile * cols;
         prefetch_rows(a.Y + (((long long)tn.row * a.N + tn.slot) * nr + jn) * a.ldq, a.ldq, min(cols, nr - jn), a.ldq);
     }
@@ -624,9 +623,8 @@ __global__ void __launch_bounds__(ROWS / SEG *kLines, ROWS == 256 ? 1 : 2) k_mod
         r[e] = (e < count && mine) ? Yq[(long long)e * a.ldq] : 0.0;
         acc[e] = 0.0;
     }
-    constexpr unsigned ahead = ROWS == 256 ? kAhead / 2 : kAhead;
-    if (blockIdx.x + ahead < gridDim.x) {
-        const TileIndex tn = tile_index(a, a.groups, blockIdx.x + ahead);
+    if (blockIdx.x + a.ahead < gridDim.x) {
+        const TileIndex tn = tile_index(a, a.groups, blockIdx.x + a.ahead);
         const int qn = tn.tile * kLines;
         prefetch_rows(a.Y + ((long long)tn.row * a.N + tn.slot) * nr * a.ldq + qn, a.ldq, nr, min(kLines, nz - qn));
     }
@@ -851,6 +849,9 @@ ModalArgs base_args(const bph_ctx *c) {
 cudaError_t launch(bph_ctx *c, const void *fn, long long blocks, int threads, size_t smem, ModalArgs &a,
                    cudaStream_t st, bool pdl) {
     ++c->launches;
+    a.ahead = (unsigned)(fn == fwd_kernel(c)   ? c->modal_resident[0]
+                         : fn == inv_kernel(c) ? c->modal_resident[1]
+                                               : c->modal_resident[2]);
     void *args[] = {&a};
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = launch_config(c, dim3((unsigned)blocks), dim3(threads), smem, attr);
@@ -1019,6 +1020,17 @@ int modal_configure(bph_ctx *c) {
     BPH_CUDA(raise_smem_limit(inv_kernel(c), (int)inv_bytes(c)));
     BPH_CUDA(raise_smem_limit(radial_kernel<false>(c), (int)radial_smem(c)));
     BPH_CUDA(raise_smem_limit(radial_kernel<true>(c), (int)radial_smem(c)));
+    // resident blocks of each (one per SM where a tall tile fills its shared memory)
+    int sms = 0;
+    BPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    const void *kernels[3] = {fwd_kernel(c), inv_kernel(c), radial_kernel<false>(c)};
+    const size_t smem[3] = {fwd_bytes(c), inv_bytes(c), radial_smem(c)};
+    for (int k = 0; k < 3; ++k) {
+        int per_sm = 0;
+        BPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[k],
+                                                               k < 2 ? tile_threads(c) : kLines * radial_nseg(c), smem[k]));
+        c->modal_resident[k] = sms * (per_sm > 1 ? per_sm : 1);
+    }
     c->modal = 1;
     return BPH_OK;
 }
