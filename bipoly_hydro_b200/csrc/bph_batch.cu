@@ -1060,11 +1060,10 @@ int batch_converged_run(bph_batch *b, int n, const int *inst, const int *d_map, 
     cv.cycles = cyc;
     if (modal) {
         BPH_CUDA(launch_modal_end(c, b->d_P, cv.mixed ? b->d_prev : b->d_modpre, n, d_map));
-        if (cv.mixed)
-            ;  // the modal potential is the result
-        else if (c->adi_seg)
+        // mixed: the modal potential is the result
+        if (!cv.mixed && c->adi_seg)
             BPH_CUDA(launch_adi_plain(c, *s, s->nsteps - 1, 1, false, b->d_P, b->d_R, n, d_map));
-        else
+        else if (!cv.mixed)
             BPH_CUDA(launch_adi_large(c, *s, s->nsteps - 1, 1, false, b->d_P, b->d_R, n, d_map, b->d_LW, b->d_LQ));
     }
     if (cv.want_resid) {

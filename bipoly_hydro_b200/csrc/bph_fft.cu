@@ -185,7 +185,8 @@ k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__re
           const double2 *__restrict__ g_tw, const double2 *__restrict__ g_tw2, const double2 *__restrict__ g_ph,
           int numr, int numz, int nr, int nz, int mmax, int fm, int isym, double four_pi,
           int *__restrict__ status, long long mstride, FftBatch bt) {
-    constexpr int kTile = tile_cols<M, true>(), NT = FftTile<M, true>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
+    constexpr int kTile = tile_cols<M, true>(), NT = FftTile<M, true>::kThreads;
+    constexpr int T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
     extern __shared__ double2 smem[];
     double2 *C = smem;  // [k1][t][column]
     double2 *tw = C + M * kTile;
@@ -333,7 +334,8 @@ __global__ void __launch_bounds__((FftTile<M, false>::kThreads), (FftShape<M, fa
 k_fft_inv(const double *__restrict__ P, double *__restrict__ pot, const double2 *__restrict__ g_tw,
           const double2 *__restrict__ g_tw2, int numr, int numz, int isym, double *__restrict__ phieff,
           const double *__restrict__ rhf, double omega, FftBatch bt) {
-    constexpr int kTile = tile_cols<M, false>(), NT = FftTile<M, false>::kThreads, T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
+    constexpr int kTile = tile_cols<M, false>(), NT = FftTile<M, false>::kThreads;
+    constexpr int T = Split<M>::T, R1 = Split<M>::R1, kOwn = Split<M>::kOwn;
     extern __shared__ double2 smem[];
     double2 *C = smem;  // [k1][t][column]
     double2 *tw = C + M * kTile;

@@ -191,7 +191,7 @@ struct bph_ctx {
     float *d_work32 = nullptr;                // global-memory refinement kernels: [4][N][np] (lazy)
     int adi_threads = 256;
     int fft_smem_fwd = 0, fft_smem_inv = 0;
-    bool fft_dense = false;      // FFT tiles compiled for eight CTAs per SM (BPH_FFT_DENSE=1)
+    bool fft_dense = false;      // single FFTs with the register budget of 768 threads per SM (set-up timing, or BPH_FFT_DENSE)
     bool have_warm = false;
     bool pdl = true;             // launch solve kernels with programmatic dependent launch
     // Overlapped solve: slots whose mode carries no boundary data (k not a
@@ -433,10 +433,12 @@ int noalloc_setup(bph_ctx *c);
 int fft_configure(bph_ctx *c);
 // ADI in the vertical eigenbasis (bph_modal.cu).  launch_modal: a whole
 // schedule on ninst instances (row r: instance inst_map[r], slots
-// slot_map[0..nslots) of each), chunk instances per pass in Y.  Converged form: begin (modal residual in Y,
-// modal potential in phi, ninst times modal_size each), cycles (partial norms
-// [ninst][N][modal_groups][2]; with *skip not 0 a cycle returns at once), end (a potential back into P: pre, the
-// caller running that step with launch_adi_plain, or phi).
+// slot_map[0..nslots) of each), chunk instances per pass in Y.  Converged
+// form: begin (modal residual in Y, modal potential in phi, ninst times
+// modal_size each), cycles (partial norms [ninst][N][modal_groups][2]; with
+// *skip not 0 a cycle returns at once; pre nullptr: the refinement's half-step
+// order), end (a potential back into P: pre, the caller running that step with
+// launch_adi_plain, or phi).
 int modal_configure(bph_ctx *c);
 void modal_free(bph_ctx *c);
 int modal_groups(const bph_ctx *c);

@@ -931,8 +931,9 @@ static void split_tables(bph_ctx *c, const std::vector<double> &wave, std::vecto
 
 // Decides whether the grid runs the modal form and prepares it.  Lines of up
 // to 256 radii fit a block; the transforms cost 4 nz FMA per zone and solve,
-// and their column tile has to fit in shared memory (nz <= 640).  BPH_ADI_WARP in the environment asks for
-// a half-step kernel by name, BPH_ADI_MODAL=0 for the half-step form.
+// and their column tile has to fit in shared memory (nz <= 640).  BPH_ADI_WARP
+// in the environment asks for a half-step kernel by name, BPH_ADI_MODAL=0 for
+// the half-step form.
 int modal_configure(bph_ctx *c) {
     c->modal = 0;
     const char *want = std::getenv("BPH_ADI_MODAL");
@@ -976,19 +977,19 @@ int modal_configure(bph_ctx *c) {
     const size_t frag = (size_t)mt * ks * 128;
     std::vector<double> pack(2 * frag);
     std::vector<int> tab;
-    if (c->modal_p1) split_tables(c, wave, pack, tab, lam);
-    else
-      for (int m = 0; m < mt; ++m)
-        for (int k = 0; k < ks; ++k)
-            for (int l = 0; l < 32; ++l) {
-                const int g = l / 4, t = l % 4;
-                for (int v = 0; v < 4; ++v) {
-                    const int row = 16 * m + g + 8 * (v & 1), col = 8 * k + t + 4 * (v >> 1);
-                    const size_t at = ((size_t)m * ks + k) * 128 + 4 * l + v;
-                    pack[at] = entry(row, col);         // E: row = mode
-                    pack[frag + at] = entry(col, row);  // E^T: row = height
-                }
-            }
+    if (c->modal_p1) {
+        split_tables(c, wave, pack, tab, lam);
+    } else {
+        for (int m = 0; m < mt; ++m)
+            for (int k = 0; k < ks; ++k)
+                for (int l = 0; l < 32; ++l)
+                    for (int v = 0; v < 4; ++v) {
+                        const int row = 16 * m + l / 4 + 8 * (v & 1), col = 8 * k + l % 4 + 4 * (v >> 1);
+                        const size_t at = ((size_t)m * ks + k) * 128 + 4 * l + v;
+                        pack[at] = entry(row, col);         // E: row = mode
+                        pack[frag + at] = entry(col, row);  // E^T: row = height
+                    }
+    }
     // One allocation: both fragment arrays, the eigenvalues, the norm partials, one instance's modal
     // array.  Slots beyond shared memory have their half-steps' scratch, which no solve needs while
     // its steps are modal (d_W >= N nr (nz + 1)): the modal array and the converged form's earlier
