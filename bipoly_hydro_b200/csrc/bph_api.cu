@@ -973,7 +973,9 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
     BPH_DEVICE_SCOPE(c);
     Schedule *s;
     if ((rc = get_schedule(c, nsteps, &s))) return rc;
-    // every array before anything of the warm state changes: a call that is refused leaves it
+    // every array before anything of the warm state changes: a call that is refused leaves it (the
+    // staging first: the optional array may give way to it)
+    if (!on_device && (rc = ensure_staging(c))) return rc;
     const bool want_modal = modal_converged(c, *s, mixed);
     if ((!mixed || want_modal) && !c->d_prev) {
         // with the FP64 form's second array in one allocation (a context's first converged solve at
@@ -995,7 +997,6 @@ static int converged_impl(bph_ctx *c, const double *rho, double *pot, int nsteps
     const double *d_rho = rho;
     double *d_pot = pot;
     if (!on_device) {
-        if ((rc = ensure_staging(c))) return rc;
         BPH_CUDA(cudaMemcpyAsync(c->d_rho_stage, rho, bytes, cudaMemcpyHostToDevice, c->stream));
         d_rho = c->d_rho_stage;
         d_pot = c->d_pot_stage;

@@ -182,6 +182,27 @@ def test_optional_arrays_give_way(bph):
         assert rel_l2(a, w) <= 1e-12
 
 
+def test_converged_host_call_whose_staging_takes_the_optional_array(bph):
+    """The FP64 converged form's optional array gives way to the staging of the very call that would
+    use it: the call runs the half-step cycles."""
+    g = (250, 40, 512, 1.0 / 246.0, 2, 8)  # staging 2 x 41 MB, optional array 39 MB with d_prev's 41
+    rho = smooth_density(*g[:5], seed=130)
+    out = []
+    for scarce in (False, True):
+        s = bph.PotentialSolver(*g)
+        d, pot = _host(rho), _host(rho)
+        s.solve_converged_device(d, pot, 10, True, 1e-11, 60)
+        s.synchronize()
+        if scarce:
+            with _Filled(60 * MB):
+                got = s.solve_converged(rho, 10, True, 1e-11, 60)
+        else:
+            got = s.solve_converged(rho, 10, True, 1e-11, 60)
+        out.append((got[0], s.solve_converged(rho, 10, True, 1e-11, 60)[0]))
+        s.close()
+    assert rel_l2(out[1][0], out[0][0]) <= 1e-12 and rel_l2(out[1][1], out[0][1]) <= 1e-12
+
+
 @pytest.mark.parametrize("room", [40, 60, 90, 130, 200])
 def test_every_form_without_room_for_the_next(oracle_mod, bph, room):
     """Batches, schedules and converged solves created with little room left run whichever form's
