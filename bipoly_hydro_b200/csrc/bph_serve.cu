@@ -53,6 +53,11 @@ struct bph_server {
     double conv_tol = 0.0;
     int conv_max_cycles = 0;
     bool conv_mixed = false;
+    // A mode change allocates, and may free, the batch's arrays: it waits for the batched calls that
+    // run, and the next ones wait for it.
+    bool busy = false;           // the worker is in its batched calls
+    int mode_changes = 0;        // waiting or at work
+    bool mode_changing = false;  // one is at work
     bool stop = false;
     std::thread worker;
 };
@@ -82,8 +87,9 @@ void serve_loop(bph_server *s) {
         bool converged = false;
         {
             std::unique_lock<std::mutex> lk(s->mu);
-            s->cv_work.wait(lk, [&] { return s->stop || !s->queue.empty(); });
+            s->cv_work.wait(lk, [&] { return (s->stop || !s->queue.empty()) && s->mode_changes == 0; });
             if (s->queue.empty()) return;  // stop requested and nothing left
+            s->busy = true;
             converged = s->conv_nsteps > 0;
             conv.nsteps = s->conv_nsteps;
             conv.tol = s->conv_tol;
@@ -144,6 +150,11 @@ void serve_loop(bph_server *s) {
             }
             s->cv_done.notify_all();
         }
+        {
+            std::lock_guard<std::mutex> lk(s->mu);
+            s->busy = false;
+        }
+        s->cv_work.notify_all();
     }
 }
 
@@ -219,17 +230,25 @@ int bph_server_set_converged(bph_server_t *s, int nsteps, double tol, int max_cy
         set_error("no mixed-precision ADI kernel is configured for this grid");
         return BPH_ERR_INVALID;
     }
-    std::lock_guard<std::mutex> lk(s->mu);
-    if (nsteps > 0) {
-        // buffers first: a batch the worker takes after the mode changes finds them
-        const int rc = batch_reserve_converged(s->batch, mixed != 0, nsteps);
-        if (rc) return rc;
+    std::unique_lock<std::mutex> lk(s->mu);
+    ++s->mode_changes;
+    s->cv_work.wait(lk, [&] { return !s->busy && !s->mode_changing; });
+    s->mode_changing = true;
+    lk.unlock();
+    // buffers first: a batch the worker takes after the mode changes finds them
+    const int rc = nsteps > 0 ? batch_reserve_converged(s->batch, mixed != 0, nsteps) : BPH_OK;
+    lk.lock();
+    if (!rc) {
+        s->conv_nsteps = nsteps;
+        s->conv_tol = tol;
+        s->conv_max_cycles = max_cycles;
+        s->conv_mixed = mixed != 0;
     }
-    s->conv_nsteps = nsteps;
-    s->conv_tol = tol;
-    s->conv_max_cycles = max_cycles;
-    s->conv_mixed = mixed != 0;
-    return BPH_OK;
+    s->mode_changing = false;
+    --s->mode_changes;
+    lk.unlock();
+    s->cv_work.notify_all();
+    return rc;
 }
 
 int bph_server_capacity(const bph_server_t *s) { return s ? s->capacity : 0; }
@@ -293,7 +312,7 @@ int bph_server_submit(bph_server_t *s, int client, const double *rho, double *po
         ++s->inflight[(size_t)client];
         *request = id;
     }
-    s->cv_work.notify_one();
+    s->cv_work.notify_all();  // mode changes wait on it too
     return BPH_OK;
 }
 
