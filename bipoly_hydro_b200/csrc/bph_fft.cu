@@ -256,9 +256,10 @@ k_fft_fwd(const double *__restrict__ src, double *__restrict__ out, double *__re
         }
         o_[so * k] = zeroed ? 0.0 : scale * F.x;
         o_[so * (M + k)] = zeroed ? 0.0 : -(scale * F.y);
-        // the boundary mode m with fm m = k
-        if (k < fm * mmax && k % fm == 0) {
-            const int m = k / fm;
+        // the boundary mode m with fm m = k (fm is 1 or 2; a division by it here took 1.0 of the 6.1 us
+        // of 66 x 66 x 64 and 2.1 of the 13.2 of 200 x 150 x 64)
+        if (k < fm * mmax && (k & (fm - 1)) == 0) {
+            const int m = k >> (fm - 1);
             const double2 ph = g_ph[m];
             mom[m * mstride + p] = ph.x * F.x - ph.y * F.y;
             mom[m * mstride + np + p] = ph.y * F.x + ph.x * F.y;
