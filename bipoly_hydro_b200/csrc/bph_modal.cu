@@ -1062,7 +1062,9 @@ cudaError_t modal_pack(bph_ctx *c, Schedule &s) {
 //   eigenbasis against 22 + 10; 66 x 66 x 64: 14 + 0.8 against 4 + 2.3): eight.
 //   The other half-step kernels: two (us for one and for two steps, half-steps
 //   against eigenbasis: 101 x 75 x 128 26 / 44 against 40 / 42, 67 x 45 x 64
-//   15 / 25 against 16 / 17, 258 x 194 x 512 424 / 790 against 485 / 526).
+//   15 / 25 against 16 / 17, 258 x 194 x 512 424 / 790 against 485 / 526);
+//   one where a slot is so small that the transforms cost no more than a step
+//   (40 x 30 x 64 13.5 against 12.5, 50 x 50 x 256 28 against 21).
 //   Tall slots, whose transforms' products are long serial chains (serial_steps
 //   of 64 clocks and more each): where the set-up's timing says, which for the
 //   five steps of a warm solve went to the half-steps at 12 x 500 x 32 (131
@@ -1095,7 +1097,7 @@ bool modal_tall(const bph_ctx *c) {
 // us[form][k]: contraction and ADI of 1 (k = 0) and 5 steps in half-steps and
 // in the eigenbasis, both linear in the steps; nullptr: untimed.
 void modal_rule(bph_ctx *c, const float (*us)[2]) {
-    c->modal_min = c->adi_warp ? 8 : 2;
+    c->modal_min = c->adi_warp ? 8 : c->nr <= 64 && c->nz <= 48 ? 1 : 2;
     c->modal_min_batch = c->modal_min;
     if (!modal_tall(c)) return;
     c->modal_min = 8;
