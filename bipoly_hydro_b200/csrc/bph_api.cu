@@ -680,6 +680,7 @@ int must_alloc(bph_ctx *c, T **p, size_t count) {
         dev_free(c->d_modpre);
     }
     c->d_modpre = nullptr;
+    c->modpre_at = kModpreNone;
     return dev_alloc(c, p, count);
 }
 

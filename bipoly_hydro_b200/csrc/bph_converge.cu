@@ -25,7 +25,7 @@ constexpr int kCheckThreads = 256;
 // skipped: an iteration of the node costs more than the two launches of a
 // skipped cycle, and most solves take three or four cycles.  (All four in the
 // body: 127 us for the one cycle of a solve that starts converged at
-// 66 x 66 x 64, 112 mixed; one ahead: 119 and 104.)
+// 66 x 66 x 64, 112 mixed; one ahead: 119, by now 110, and 104.)
 constexpr int kBodyCycles = 3;
 
 __global__ void k_conv_init(ConvState *st, double tol, int max_cycles, int mixed, double least) {

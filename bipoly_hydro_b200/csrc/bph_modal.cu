@@ -69,6 +69,7 @@ struct ModalArgs {
     int inst0, nslots, ntile, groups;
     int numr, numz, nr, nz, ldq, N, isym, mtiles, ksteps;
     int nsteps, source, add;
+    unsigned half;           // forward transform: blocks from this one on take the potential into phi
     unsigned ahead;          // blocks of the kernel that the device holds at a time
     int lagged;              // converged form: the refinement's half-step order (nsteps counts its radial solves)
     double gamma;
@@ -148,7 +149,7 @@ __device__ __forceinline__ void tile_product(const ModalArgs &a, const double *s
 // band of rows with the rows below and at hand kept in registers.  Waits for
 // the previous kernel.
 template <int NT>
-__device__ __forceinline__ void source_tile(const ModalArgs &a, const TileIndex &ti, double *sx) {
+__device__ __forceinline__ void source_tile(const ModalArgs &a, int source, const TileIndex &ti, double *sx) {
     constexpr int ld = TileShape<NT>::ld;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, numr = a.numr, j0 = ti.tile * TileShape<NT>::cols;
@@ -166,7 +167,7 @@ __device__ __forceinline__ void source_tile(const ModalArgs &a, const TileIndex 
         }
         const double al = a.alphar[j + 1], be = a.betar[j + 1], bd = a.brb[(long long)ti.slot * numr + j + 1];
         const double *p = Pg + (j + 1);
-        if (a.source == kResidual) {
+        if (source == kResidual) {
             double dn = 0.0, cur = 0.0;
             if (k0 < k1) {
                 dn = (k0 > 0 || dirichlet) ? p[(long long)k0 * numr] : 0.0;
@@ -182,7 +183,7 @@ __device__ __forceinline__ void source_tile(const ModalArgs &a, const TileIndex 
                 dn = cur;
                 cur = up;
             }
-        } else if (a.source == kColdResidual) {
+        } else if (source == kColdResidual) {
 #pragma unroll 4
             for (int k = k0; k < k1; ++k) {
                 double v = Rs[(long long)k * nr + j];
@@ -204,13 +205,14 @@ template <int NT>
 __global__ void __launch_bounds__(256) k_modal_fwd(ModalArgs a) {
     extern __shared__ double sx[];
     constexpr int ld = TileShape<NT>::ld;
-    const TileIndex ti = tile_index(a, a.ntile, blockIdx.x);
+    const bool second = blockIdx.x >= a.half;
+    const TileIndex ti = tile_index(a, a.ntile, second ? blockIdx.x - a.half : blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, j0 = ti.tile * TileShape<NT>::cols;
     for (int e = threadIdx.x; e < (8 * a.ksteps - nz) * ld; e += blockDim.x) sx[nz * ld + e] = 0.0;
-    source_tile<NT>(a, ti, sx);
+    source_tile<NT>(a, second ? kPotential : a.source, ti, sx);
     __syncthreads();
-    double *Yb = a.Y + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
+    double *Yb = (second ? a.phi : a.Y) + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
     const int g = lane >> 2, t = lane & 3;
     for (int mt = warp; mt < a.mtiles; mt += nwarps) {
         double acc[NT][4];
@@ -383,7 +385,8 @@ template <int NT, int P1>
 __global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
     extern __shared__ double sx[];
     constexpr int ld = TileShape<NT>::ld, cols = TileShape<NT>::cols, h = (P1 - 1) / 2;
-    const TileIndex ti = tile_index(a, a.ntile, blockIdx.x);
+    const bool second = blockIdx.x >= a.half;
+    const TileIndex ti = tile_index(a, a.ntile, second ? blockIdx.x - a.half : blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int nr = a.nr, nz = a.nz, h2 = a.h2, k2 = 8 * a.ks2, j0 = ti.tile * cols;
     int *tab = reinterpret_cast<int *>(sx + nz * ld);  // [P1][h2]
@@ -396,13 +399,15 @@ __global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
         const int at = (grp <= h && a2 == 0) ? 1 : a2;
         rows[i] = (abs(a.tab[a1 * h2 + at]) - 1) * ld;
     }
-    source_tile<NT>(a, ti, sx);
+    source_tile<NT>(a, second ? kPotential : a.source, ti, sx);
     if (blockIdx.x + a.ahead < gridDim.x) {
-        const TileIndex tn = tile_index(a, a.ntile, blockIdx.x + a.ahead);
+        const unsigned next = blockIdx.x + a.ahead;
+        const int source = next >= a.half ? kPotential : a.source;
+        const TileIndex tn = tile_index(a, a.ntile, next >= a.half ? next - a.half : next);
         const int jn = tn.tile * cols, count = min(cols, nr - jn);
         const long long at = tn.inst * a.N + tn.slot;
-        if (a.source != kPotential) prefetch_rows(a.R + at * nr * nz + jn, nr, nz, count);
-        if (a.source != kColdResidual)
+        if (source != kPotential) prefetch_rows(a.R + at * nr * nz + jn, nr, nz, count);
+        if (source != kColdResidual)
             prefetch_rows(a.P + at * a.numr * a.numz + a.numr + jn + 1, a.numr, nz, count);
     }
     __syncthreads();
@@ -416,7 +421,7 @@ __global__ void __launch_bounds__(256, 2) k_modal_fwd_split(ModalArgs a) {
             });
     }
     __syncthreads();
-    double *Yb = a.Y + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
+    double *Yb = (second ? a.phi : a.Y) + ((long long)ti.row * a.N + ti.slot) * nr * a.ldq;
     const int g = lane >> 2, t = lane & 3;
     for (int u = warp; u < (h + 1) * a.mt2; u += nwarps) {
         const int b1 = u / a.mt2, mt = u % a.mt2;
@@ -812,6 +817,7 @@ int tile_threads(const bph_ctx *c) {
 
 ModalArgs base_args(const bph_ctx *c) {
     ModalArgs a = {};
+    a.half = ~0u;
     a.brb = c->d_brb;
     a.alphar = c->d_alphar;
     a.betar = c->d_betar;
@@ -1178,12 +1184,16 @@ cudaError_t launch_modal_begin(bph_ctx *c, bool cold, double *P, const double *R
     a.E = c->d_modE;
     a.source = cold ? kColdResidual : kResidual;
     const long long blocks = (long long)ninst * c->N * a.ntile;
-    cudaError_t e = launch(c, fwd_kernel(c), blocks, tile_threads(c), fwd_bytes(c), a, c->stream, c->pdl);
-    if (e != cudaSuccess) return e;
-    if (cold) return cudaMemsetAsync(phi, 0, sizeof(double) * (size_t)ninst * modal_size(c), c->stream);
-    a.Y = phi;
-    a.source = kPotential;
-    return launch(c, fwd_kernel(c), blocks, tile_threads(c), fwd_bytes(c), a, c->stream, c->pdl);
+    // warm: both transforms in one launch, side by side where one alone leaves SMs idle (us of a solve
+    // of one cycle: 66 x 66 x 64 119 -> 110, 40 x 400 x 64 540 -> 400, 12 x 500 x 32 390 -> 297)
+    if (!cold) {
+        a.phi = phi;
+        a.half = (unsigned)blocks;
+    }
+    const cudaError_t e =
+        launch(c, fwd_kernel(c), cold ? blocks : 2 * blocks, tile_threads(c), fwd_bytes(c), a, c->stream, c->pdl);
+    if (e != cudaSuccess || !cold) return e;
+    return cudaMemsetAsync(phi, 0, sizeof(double) * (size_t)ninst * modal_size(c), c->stream);
 }
 
 cudaError_t launch_modal_cycle(bph_ctx *c, const Schedule &s, double *Y, double *phi, double *pre, int ninst,
