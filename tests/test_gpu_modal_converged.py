@@ -91,3 +91,31 @@ def test_device_loop_ends_after_any_cycle(bph, monkeypatch, kind):
     for n, (a, b) in enumerate(zip(out["1"], out["0"]), 1):
         assert a[1].cycles == b[1].cycles and (a[1].cycles == n or kind != "fp64")
         assert np.array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("nsteps", [1, 2, 8, 15])
+def test_cycle_lengths(bph, monkeypatch, nsteps):
+    """Four cycles of any length are the half-steps' iterate: FP64 to rounding (1e-12, the drop-in's
+    bar), the refinement's order to the FP32 cycles' rounding (2^-23 of an update, a few times over)
+    where they reduce the error: cycles of one and two steps do not (they amplify FP32 rounding to
+    1e-4 and 1e-6 of the potential, and the order's algebra is exact there as elsewhere)."""
+    g = (50, 37, 32, 1.0 / 46.0, 2, 8)
+    rhos = [np.asfortranarray(smooth_density(*g[:5], seed=150 + i)) for i in range(2)]
+    out = {}
+    for form in ("modal", "half"):
+        if form == "half":
+            monkeypatch.setenv("BPH_ADI_MODAL", "0")
+        s = bph.PotentialSolver(*g)
+        s.set_mixed_adi(MIXED_ADI_GLOBAL)
+        b = bph.Batch(s, capacity=2)
+        full = [s.solve_converged(rhos[0], nsteps, True, 0.0, 4)[0], s.solve_converged(rhos[1], nsteps, False, 0.0, 4)[0]]
+        full += b.solve_converged(rhos, nsteps, True, 0.0, 4)[0]
+        mixed = s.solve_converged_mixed(rhos[0], nsteps, True, 0.0, 4)
+        out[form] = full, mixed
+        b.close()
+        s.close()
+    for a, h in zip(out["modal"][0], out["half"][0]):
+        assert rel_l2(a, h) <= 1e-12
+    (a, ia), (h, ih) = out["modal"][1], out["half"][1]
+    assert ia.cycles == ih.cycles
+    assert nsteps <= 2 or rel_l2(a, h) <= 8 * 2.0 ** -23
